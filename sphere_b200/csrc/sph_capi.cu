@@ -23,8 +23,8 @@ int count_live_slots(const StepArgs &A, cudaStream_t st, unsigned long long *d_c
                      uint64_t *launches);
 int launch_step_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
                       uint64_t *launches, Prof *prof);
-int relax_sweep(const StepArgs &A, cudaStream_t st, double alpha, double z_top,
-                unsigned long long *d_max, uint64_t *launches);
+int relax_sweeps(const StepArgs &A, cudaStream_t st, uint32_t sweeps, double alpha, double z_top,
+                 unsigned long long *d_max, uint64_t *launches);
 int porosity_profile(const double4 *x, uint32_t p0, uint32_t np, double h_slice, double V_slice,
                      uint32_t nslices, double *z_pos, double *por, cudaStream_t st);
 int find_overlaps(OverlapArgs O, uint32_t ncells, uint32_t *scan_tmp, cudaStream_t st, int stage);
@@ -2453,8 +2453,8 @@ int sph_relax(SphHandle *h, uint32_t sweeps, double alpha, double z_top, double 
         invalidate_pair(h);   // the sweeps move the spheres in the FP64 arrays
     }
     uint64_t nl = 0;
-    for (uint32_t k = 0; k < sweeps; ++k) {
-        int st = sph::relax_sweep(h->A, h->stream, alpha, z_top, h->d_count, &nl);
+    {
+        int st = sph::relax_sweeps(h->A, h->stream, sweeps, alpha, z_top, h->d_count, &nl);
         if (st != SPH_OK) return fail(h, st, "relax sweep launch failed");
     }
     h->launches += nl;
