@@ -25,6 +25,7 @@ int launch_step_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
                       uint64_t *launches, Prof *prof);
 int relax_sweeps(const StepArgs &A, cudaStream_t st, uint32_t sweeps, double alpha, double z_top,
                  unsigned long long *d_max, uint64_t *launches);
+int sort_from_ids(const StepArgs &A, cudaStream_t st);
 int porosity_profile(const double4 *x, uint32_t p0, uint32_t np, double h_slice, double V_slice,
                      uint32_t nslices, double *z_pos, double *por, cudaStream_t st);
 int find_overlaps(OverlapArgs O, uint32_t ncells, uint32_t *scan_tmp, cudaStream_t st, int stage);
@@ -95,6 +96,11 @@ struct SphHandle {
     // of A are behind them (brought up to date by sync_public)
     sph::PairArgs P{};
     bool pair_alloc = false, pair_valid = false, pair_ahead = false;
+    // which steps the neighbour lists (and the cells of the lazily sorted
+    // split step) belong to: prepare_steps asks for a rebuild when that
+    // changes
+    enum ListUse { LISTS_NONE, LISTS_CHAIN, LISTS_LAZY, LISTS_PAIR };
+    ListUse list_use = LISTS_NONE;
     // steps launched kernel by kernel instead of as captured graphs
     // (SPHERE_B200_EAGER=1 at sph_create): for profilers that cannot see
     // into graphs with conditional nodes; the list step then reads its
@@ -228,6 +234,29 @@ static void invalidate_pair(SphHandle *h)
     h->pair_ahead = false;
 }
 
+// The launch settings of a step: the split step sorts lazily unless some
+// box's grid is adaptive or some populated box cannot have neighbour lists.
+static StepConfig step_config(const SphHandle *h)
+{
+    StepConfig cfg = h->cfg;
+    cfg.lazy_sort = h->uploaded && !pair_active(h) && sph::split_active(h->A, cfg);
+    for (uint32_t k = 0; k < h->nbox; ++k)
+        if (h->boxes[k].grid.adaptive || (h->dbox[k].np > 0 && h->dbox[k].vrange < 1))
+            cfg.lazy_sort = false;
+    return cfg;
+}
+
+// The next steps use the lists as `use` says: the list step keeps lists of
+// its own but shares the reference positions, and only the lazily sorted
+// split step keeps the spheres' cells current at the end of a step, so the
+// steps after a change rebuild.
+static int claim_lists(SphHandle *h, SphHandle::ListUse use)
+{
+    if (h->list_use != use) CUDA_TRY(h, cudaMemsetAsync(h->A.vflag, 1, 1, h->stream));
+    h->list_use = use;
+    return SPH_OK;
+}
+
 // Before steps of the active launch variant are queued: the list step
 // loads its compact state when that is stale; every other variant needs
 // the FP64 arrays current, and leaves the compact state stale.
@@ -242,12 +271,12 @@ static int prepare_steps(SphHandle *h)
             h->pair_valid = true;
         }
         h->pair_ahead = true;
-        return SPH_OK;
+        return claim_lists(h, SphHandle::LISTS_PAIR);
     }
     int st = sync_public(h);
     if (st != SPH_OK) return st;
     h->pair_valid = false;
-    return SPH_OK;
+    return claim_lists(h, step_config(h).lazy_sort ? SphHandle::LISTS_LAZY : SphHandle::LISTS_CHAIN);
 }
 
 // src/sphere.cpp:145-345 checkValues, parts that do not need particle data.
@@ -506,7 +535,7 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
         (st = dalloc(h, &bcsr_off, n + 1)) || (st = dalloc(h, &bcsr_ent, 2 * nb)) ||
         (st = dalloc(h, &A.err, 1)) || (st = dalloc(h, &h->d_count, 1)) ||
         (st = dalloc(h, &A.vlist, n * sph::VL_MAX)) || (st = dalloc(h, &A.vcount, n)) ||
-        (st = dalloc(h, &A.vflag, 2)) || (st = dalloc(h, &A.xref, n)) ||
+        (st = dalloc(h, &A.vflag, 3)) || (st = dalloc(h, &A.sort_bar, 2)) || (st = dalloc(h, &A.xref, n)) ||
         (st = dalloc(h, &A.cellc, n))) {
         fprintf(stderr, "sphere_b200: %s\n", h->err.c_str());
         return bail(st);
@@ -866,7 +895,8 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
     CUDA_TRY(h, cudaMemcpyAsync(A.boxes, h->dbox.data(), sizeof(DevBox) * h->nbox,
                                 cudaMemcpyHostToDevice, cs));
     CUDA_TRY(h, cudaMemsetAsync(A.err, 0, sizeof(uint32_t), cs));
-    CUDA_TRY(h, cudaMemsetAsync(A.vflag, 0, 2 * sizeof(uint32_t), cs));
+    CUDA_TRY(h, cudaMemsetAsync(A.sort_bar, 0, 2 * sizeof(uint32_t), cs));
+    CUDA_TRY(h, cudaMemsetAsync(A.vflag, 0, 3 * sizeof(uint32_t), cs));
     CUDA_TRY(h, cudaMemsetAsync(A.vflag, 1, 1, cs));   // build the lists in the first step
     // the caller's buffers are read only during the call
     CUDA_TRY(h, cudaStreamSynchronize(cs));
@@ -883,15 +913,11 @@ static int capture_step(SphHandle *h, sph::Prof *prof, cudaGraph_t *g, cudaGraph
     // an error left by an earlier failed call (already returned to its
     // caller) must not be taken for a launch error of this capture
     (void)cudaGetLastError();
-    StepConfig cfg = h->cfg;
+    StepConfig cfg = step_config(h);
     cfg.phase = phase;
-    cfg.side = h->side;
-    cfg.fork = h->ev_fork;
-    cfg.join = h->ev_join;
     const bool pair = pair_active(h);
-    if ((pair || h->darcy_on) && !h->side) {
-        // the list step captures its rebuild body, the Darcy coupling its
-        // Jacobi loop's body, on the side stream
+    if (h->darcy_on && !h->side) {
+        // the Darcy coupling captures its Jacobi loop's body on the side stream
         CUDA_TRY(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
         CUDA_TRY(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
         CUDA_TRY(h, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
@@ -902,7 +928,6 @@ static int capture_step(SphHandle *h, sph::Prof *prof, cudaGraph_t *g, cudaGraph
     if (pair) {
         int st = ensure_pair(h);
         if (st != SPH_OK) return st;
-        cfg.side = h->side;
     }
     CUDA_TRY(h, cudaStreamBeginCapture(h->own, cudaStreamCaptureModeThreadLocal));
     int st = pair ? sph::launch_step_pair(h->A, h->P, cfg, h->own, nl, prof)
@@ -990,6 +1015,9 @@ static int collect_errors(SphHandle *h)
     CUDA_TRY(h, cudaMemcpy(&bits, h->A.err, sizeof bits, cudaMemcpyDeviceToHost));
     CUDA_TRY(h, cudaMemset(h->A.err, 0, sizeof(uint32_t)));
     if (!bits) return SPH_OK;
+    // a rebuild that gave up left its barrier half counted
+    if (bits & (1u << SPH_ERR_TIMEOUT))
+        CUDA_TRY(h, cudaMemset(h->A.sort_bar, 0, 2 * sizeof(uint32_t)));
     static const int order[] = {SPH_ERR_TIMEOUT, SPH_ERR_NAN, SPH_ERR_OUT_OF_GRID, SPH_ERR_INPUT,
                                 SPH_ERR_NC_OVERFLOW};
     for (int code : order)
@@ -1066,7 +1094,7 @@ static int queue_steps_now(SphHandle *h, uint64_t nsteps, uint8_t *states)
         // kernel by kernel on the handle's stream (no graphs)
         if ((st = prepare_steps(h)) != SPH_OK) return st;
         const size_t bytes = sizeof(DevBox) * h->nbox;
-        StepConfig cfg = h->cfg;
+        const StepConfig cfg = step_config(h);
         for (uint64_t s = 0; s < nsteps; ++s) {
             uint64_t nl = 0;
             st = pair_active(h) ? sph::launch_step_pair(h->A, h->P, cfg, h->stream, &nl, nullptr)
@@ -1722,6 +1750,13 @@ int sph_get_sort(SphHandle *h, uint32_t *cell_id, uint32_t *perm, uint32_t *cell
     cudaSetDevice(h->device);
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     const uint64_t n = h->ntot, nc = h->ncells;
+    // the lazily sorted split step keeps each step's cell ids; the order
+    // that follows from them is made here
+    if (h->list_use == SphHandle::LISTS_LAZY && n && (perm || cell_start || cell_end)) {
+        int st = sph::sort_from_ids(h->A, h->stream);
+        if (st != SPH_OK) return fail(h, st, "cell sort failed");
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    }
     if (cell_id && n) CUDA_TRY(h, cudaMemcpy(cell_id, h->A.cell_id, 4 * n, cudaMemcpyDeviceToHost));
     if (perm && n) CUDA_TRY(h, cudaMemcpy(perm, h->A.perm, 4 * n, cudaMemcpyDeviceToHost));
     if (cell_start || cell_end) {
@@ -1859,7 +1894,7 @@ int sph_adjoint_forward(SphHandle *h, uint64_t nsteps, uint32_t ckpt, double *fo
                     "kappa = 0, no bonds, no dynamic walls, fixed grid, gamma_wt = 0");
     cudaSetDevice(h->device);
     int st;
-    if ((st = build_graph(h)) != SPH_OK) return st;
+    if ((st = build_graph(h)) != SPH_OK || (st = prepare_steps(h)) != SPH_OK) return st;
     free_adjoint(h);
     const uint64_t nseg = (nsteps + ckpt - 1) / ckpt;
     const size_t sb = state_bytes(h);
@@ -1977,7 +2012,7 @@ int sph_adjoint_backward(SphHandle *h, const double *dx_final, double *grad_para
                 Ar.tape_rows_post = Ar.tape_rows_pre + (size_t)n * sph::NC;
                 Ar.tape_hist = (double4 *)(Ar.tape_rows_post + (size_t)n * sph::NC);
                 uint64_t nl = 0;
-                rst = sph::launch_step(Ar, h->cfg, h->own, &nl);
+                rst = sph::launch_step(Ar, step_config(h), h->own, &nl);
             }
         } else {
             const bool first = (kind >> 1) != 0;

@@ -48,10 +48,15 @@ struct StepArgs {
     // sphere uses the cell search), xref = position at the list build; cellc = packed cell
     // coordinates of the current step (k_hash); vflag[0] != 0 requests a
     // rebuild before the next contact search, vflag[1] counts rebuilds
+    // vflag[2] != 0: some sphere had no list at the last build
     uint32_t *vlist, *vcount, *vflag;
+    uint32_t *sort_bar;        // grid-barrier words of the one-launch rebuilds
     float4 *xref;
     uint64_t *cellc;
     uint32_t vcap;             // list capacity in use (<= VL_MAX)
+    // the split step without a sort per step: k_search checks its sphere's
+    // position and stores its cell id, k_finish the cell of its new position
+    uint32_t lazy_sort;
     // split step (k_search / k_contacts / k_finish): per warp of 32
     // original indexes, a region of 32 * NC entries holding the warp's live
     // contacts from its start, sphere after sphere, each in slot order
@@ -210,11 +215,21 @@ struct StepConfig {
     int variant = 1;  // interact launch variant (sph_autotune)
     int pair_shape = 0;   // register budget of the list-step kernel (sph_autotune)
     bool all_cm23 = false;   // every box uses contact model 2 or 3
+    // the split step sorts only when its lists are rebuilt (k_resort); not
+    // with an adaptive grid, whose cells change at every step
+    bool lazy_sort = false;
     int phase = STEP_WHOLE;
     cudaStream_t side = nullptr;                       // STEP_OVERLAP only
     cudaEvent_t fork = nullptr, join = nullptr;        // STEP_OVERLAP only
     const DarcyArgs *darcy = nullptr;                  // the Darcy coupling, null: off
 };
+
+// Whether a step with these settings runs as the split step.
+inline bool split_active(const StepArgs &A, const StepConfig &cfg)
+{
+    return cfg.variant == SPLIT_VARIANT && !cfg.unfused && cfg.all_cm23 && A.vlist && A.csum &&
+           A.ntot > 0;
+}
 
 // Per-kernel timing of an un-graphed step (the counterpart of the
 // reference's PROFILING breakdown, src/device.cu:947-987 and 2711-2808):
@@ -287,12 +302,6 @@ int pair_count_live(const StepArgs &A, const PairArgs &P, cudaStream_t st,
 int barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds,
                   unsigned long long limit_ns, uint32_t *d_words, uint32_t *d_err,
                   cudaStream_t st);
-// Sort and neighbour lists for a rebuild of the list step's lists
-// (sph_kernels.cu): the positions of the current state (xr[*pp]) into A.x,
-// the cell sort, and the lists into the buffers not in use
-// (ids / cnt [*lsel ^ 1]).
-void launch_pair_sort_build(const StepArgs &A, const PairArgs &P, cudaStream_t st);
-
 // Ray-traced image of one box (sph_render): tiles of the screen, entries of
 // the tile lists, kernels launched.
 struct RenderStats {

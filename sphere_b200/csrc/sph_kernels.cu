@@ -27,6 +27,7 @@
 
 #include "sph_device.cuh"
 #include "sph_internal.h"
+#include "sph_sort.cuh"
 #include "sph_step.cuh"
 
 namespace sph {
@@ -35,41 +36,6 @@ static inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n
 
 // ------------------------------------------------------------------ sorting
 
-// sorting.cuh:7-51 calcParticleCellID + device.cu:241-276 position checks
-// for sphere i at x, by whole warps (valid: the lane holds a sphere).
-__device__ __forceinline__ void hash_sphere(const StepArgs &A, const DevBox &B, uint32_t i,
-                                            double4 x, bool valid)
-{
-    const double xv[3] = {x.x, x.y, x.z};
-    uint32_t c[3];
-    bool nonfinite = !isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z);
-    bool outside = false;
-    for (int d = 0; d < 3; ++d) {
-        double f = floor((xv[d] - B.origo[d]) / (B.L[d] / B.num[d]));
-        if (!(f >= 0.0)) { outside = true; f = 0.0; }
-        if (f >= (double)B.num[d]) { outside = true; f = (double)(B.num[d] - 1); }
-        c[d] = (uint32_t)f;
-    }
-    if (valid) {
-        if (nonfinite) raise_flag(A.err, SPH_ERR_NAN);
-        else if (outside || x.x > B.L[0] || x.y > B.L[1] || x.z > B.L[2])
-            raise_flag(A.err, SPH_ERR_OUT_OF_GRID);
-    }
-    const uint32_t cell = B.cell_base + (c[2] * B.num[1]) * B.num[0] + c[1] * B.num[0] + c[0];
-    // lanes of the warp in the same cell take consecutive slots with one
-    // atomic (the slot order within a cell is free: k_place orders by index)
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t peers = __match_any_sync(0xffffffffu, valid ? cell : 0xffffffffu);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (valid && (int)lane == leader) base = atomicAdd(&A.cell_count[cell], (uint32_t)__popc(peers));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (!valid) return;
-    A.cell_id[i] = cell;
-    if (A.cellc) A.cellc[i] = pack_cell(c[0], c[1], c[2]);
-    A.local_off[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-}
-
 __global__ void k_hash(StepArgs A)
 {
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -77,42 +43,6 @@ __global__ void k_hash(StepArgs A)
     const uint32_t i = valid ? i0 : 0u;
     const DevBox &B = A.boxes[A.nboxes == 1 ? 0u : A.box_of[i]];
     hash_sphere(A, B, i, A.x[i], valid);
-}
-
-// Exclusive scan of n uint32 (3 launches): per-block totals, a one-block
-// scan of the totals, then per-block scans with the block offset.
-constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_ITEMS = 4;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *smem,
-                                                         uint32_t *total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) smem[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < (int)(blockDim.x >> 5) ? smem[lane] : 0u;
-        uint32_t wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += y;
-        }
-        smem[lane] = wi - w;
-        if (lane == 31) smem[32] = wi;
-    }
-    __syncthreads();
-    const uint32_t r = smem[warp] + incl - v;
-    *total = smem[32];
-    __syncthreads();
-    return r;
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *in, uint64_t n,
@@ -185,107 +115,21 @@ __global__ void k_scatter(StepArgs A)
     A.unsorted[A.cell_off[A.cell_id[i]] + A.local_off[i]] = i;
 }
 
-// The stable sort by cell id and the sorted copies (sorting.cuh:118-130)
-// in one pass over the particles in original order: particle i goes to
-// cell_off[c] + (the number of particles of its cell with a smaller index),
-// so each cell is ordered by original index.  rank = inverse of perm.
-// ALL = false for the split step, which reads velocities and partners in
-// original order and needs only the sorted positions and rank (the
-// neighbour-list build and the cell-search fallback).
+// place_sphere for every sphere; ALL: the sorted velocities too (the fused
+// kernels; the split step reads velocities and partners in original order).
 template <bool ALL>
 __global__ void k_place(StepArgs A)
 {
     grid_dependency_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.ntot) return;
-    const uint32_t c = A.cell_id[i];
-    const uint32_t s = A.cell_off[c], e = A.cell_off[c + 1];
-    uint32_t j = s;
-    for (uint32_t k = s; k < e; ++k) j += A.unsorted[k] < i ? 1u : 0u;
-    A.perm[j] = i;
-    const double4 x = A.x[i];
-    A.xs[j] = x;
-    A.xf[j] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
-    A.rank[i] = j;
-    if (ALL) {
-        A.vs[j] = A.vel[i];
-        A.ws[j] = A.angvel[i];
-    }
+    if (i < A.ntot) place_sphere<ALL>(A, i);
 }
 
 // --------------------------------------------------------- neighbour lists
 
-constexpr int VLIST_THREADS = 128;
-
-// Neighbour lists for the contact search of contact models 2 and 3: for the
-// sphere at sorted position a, the ids of all spheres within
-// ra + rb + vskin among the +-vrange cells around it (FP32 test widened by
-// the prefilter margin, so the list may hold a few more), ascending and
-// without repeats.  A sphere that moves less than vskin / 2 (checked in the
-// integration against xref) keeps every sphere it can touch in its list.
-// Runs only when vflag[0] is set; a list that overflows vcap (<= VL_MAX) is
-// marked VL_MAX + 1 and that sphere uses the cell search.  Entry k of
-// sphere i goes to vlist[i * row_stride + k * k_stride] (rows of VL_MAX for
-// the FP64 form's lists, entry-major for the list step's).
-__device__ __forceinline__ void vlist_build_one(const StepArgs &A, uint32_t a, uint32_t *lst,
-                                                uint32_t *vlist, uint32_t *vcount, uint32_t cap,
-                                                uint32_t row_stride, uint32_t k_stride)
-{
-    const int RS = VLIST_THREADS;
-    const uint32_t i = A.perm[a];
-    const DevBox &B = A.boxes[A.box_of[i]];
-    const float4 xaf = A.xf[a];
-    A.xref[i] = xaf;
-    const int R = B.vrange;
-    const uint32_t cm = B.P.contactmodel;
-    if (R < 1 || (cm != 2 && cm != 3)) {
-        vcount[i] = VL_MAX + 1;
-        return;
-    }
-    int g0, g1, g2;
-    unpack_cell(A.cellc[i], g0, g1, g2);
-    const int nx = (int)B.num[0], ny = (int)B.num[1];
-    const float reach = B.pre_margin + B.vskin;
-    const float Lf0 = (float)B.L[0], Lf1 = (float)B.L[1];
-    int n = 0;
-    bool over = false;
-    for (int dz = -R; dz <= R && !over; ++dz)
-        for (int dy = -R; dy <= R && !over; ++dy)
-            for (int dx = -R; dx <= R && !over; ++dx) {
-                int tx = g0 + dx, ty = g1 + dy, sx, sy;
-                const int tz = g2 + dz;
-                if (!image_cell(B, tx, ty, tz, sx, sy)) continue;
-                const float fsx = sx == 0 ? 0.f : (sx > 0 ? Lf0 : -Lf0);
-                const float fsy = sy == 0 ? 0.f : (sy > 0 ? Lf1 : -Lf1);
-                const uint32_t cell = B.cell_base + (uint32_t)(tx + ty * nx + (nx * ny) * tz);
-                const uint32_t start = A.cell_off[cell], end = A.cell_off[cell + 1];
-                for (uint32_t b = start; b < end; ++b) {
-                    if (b == a) continue;
-                    if (!maybe_touching(xaf, A.xf[b], fsx, fsy, reach)) continue;
-                    const uint32_t bo = A.perm[b];
-                    int q = n;
-                    while (q > 0 && lst[(q - 1) * RS] > bo) --q;
-                    if (q > 0 && lst[(q - 1) * RS] == bo) continue;   // another image
-                    if (n == (int)cap) {
-                        over = true;
-                        break;
-                    }
-                    for (int k = n; k > q; --k) lst[k * RS] = lst[(k - 1) * RS];
-                    lst[q * RS] = bo;
-                    ++n;
-                }
-            }
-    if (over) {
-        vcount[i] = VL_MAX + 1;
-        return;
-    }
-    uint32_t *out = vlist + (size_t)i * row_stride;
-    for (int k = 0; k < n; ++k) out[(size_t)k * k_stride] = lst[k * RS];
-    vcount[i] = (uint32_t)n;
-}
-
 // A grid of a few blocks per SM that strides over the spheres, so that the
 // launch costs little on the steps that build nothing.
+constexpr int VLIST_THREADS = 128;
 constexpr unsigned VLIST_BLOCKS = 148u * 8u;
 
 __global__ void __launch_bounds__(VLIST_THREADS) k_vlist_build(StepArgs A)
@@ -295,24 +139,40 @@ __global__ void __launch_bounds__(VLIST_THREADS) k_vlist_build(StepArgs A)
     __shared__ uint32_t s_list[VL_MAX * VLIST_THREADS];
     for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < A.ntot;
          a += gridDim.x * blockDim.x)
-        vlist_build_one(A, a, s_list + threadIdx.x, A.vlist, A.vcount, A.vcap, VL_MAX, 1u);
+        vlist_build_one(A, a, s_list + threadIdx.x, A.vlist, A.vcount, A.vcap, VL_MAX, 1u,
+                        VLIST_THREADS);
 }
 
-// The list step's rebuild (sph_pair.cu): its current positions into A.x for
-// the cell sort, and its lists built at full capacity into the buffers not
-// in use.
-__global__ void k_pair_sync_x(StepArgs A, PairArgs P)
+// The sort and the list build of the split step, when they are needed: the
+// step's other kernels read the sorted order and the lists only, and those
+// hold until a sphere has moved half the skin (vflag[0], raised by the
+// integration) -- unless some sphere has no list (vflag[2]) and goes
+// through the cells at every step, which takes this step's sort.  Most
+// steps find neither and end at once: one launch of 1-2 us in the place of
+// the chain k_hash .. k_vlist_done of eight, which took 57 us of a step at
+// 1e6 spheres and 16 us of 33 at 1e4.
+__global__ void __launch_bounds__(RESORT_THREADS) k_resort(StepArgs A, GridSync G)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < A.ntot) A.x[i] = P.xr[*P.pp][i];
-}
-
-__global__ void __launch_bounds__(VLIST_THREADS) k_pair_vlist(StepArgs A, PairArgs P)
-{
-    __shared__ uint32_t s_list[VL_MAX * VLIST_THREADS];
-    const uint32_t alt = *P.lsel ^ 1u;
-    const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < A.ntot) vlist_build_one(A, a, s_list + threadIdx.x, P.ids[alt], P.cnt[alt], VL_MAX, 1u, P.nrow);
+    extern __shared__ uint32_t s_mem[];
+    uint32_t *s_scan = s_mem + VL_MAX * RESORT_THREADS;
+    const uint32_t rebuild = A.vflag[0];
+    if ((rebuild | A.vflag[2]) == 0u) return;
+    // (sort_all's barriers lie between these reads and the writes below)
+    if (!sort_all<false>(A, G, s_scan, [&](uint32_t i) { return A.x[i]; })) return;
+    if (rebuild == 0u) return;
+    uint32_t none = 0;
+    for (uint32_t a = blockIdx.x * RESORT_THREADS + threadIdx.x; a < A.ntot;
+         a += gridDim.x * RESORT_THREADS)
+        if (!vlist_build_one(A, a, s_mem + threadIdx.x, A.vlist, A.vcount, A.vcap, VL_MAX, 1u,
+                             RESORT_THREADS))
+            none = 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.vflag[2] = 0u;
+    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    if (none) A.vflag[2] = 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.vflag[0] = 0u;
+        A.vflag[1] += 1u;
+    }
 }
 
 // After the (possible) build: clear the request, count builds.
@@ -535,9 +395,7 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
 // FP32 on the 16-byte copy (maybe_touching: never false for an overlapping
 // pair), RELAX_BATCH loads in flight; the FP64 test, square root and
 // division run for the few that pass, in the cells' visit order, so the
-// sums are those of the plain loop (a sweep of 1e6 spheres: 1.26 -> 0.70 ms
-// with the positions' update and the next sweep's cells in the same kernel
-// and one atomic per block).  The cells of a row (dx = -1, 0, 1) are
+// sums are those of the plain loop.  The cells of a row (dx = -1, 0, 1) are
 // neighbours in the cell order, so away from the grid's x edges a row is
 // one range of candidates.
 constexpr int RELAX_THREADS = 128;
@@ -937,18 +795,26 @@ static void contacts_fp64(const StepArgs &A, cudaStream_t st, unsigned grid, int
     launch_contacts<false>(A, st, grid, lm, pdl);
 }
 
-void launch_pair_sort_build(const StepArgs &A, const PairArgs &P, cudaStream_t st)
+// The cell counts and each sphere's place in its cell from the cell ids.
+__global__ void k_recount(StepArgs A)
 {
-    k_pair_sync_x<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A, P);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.ntot) A.local_off[i] = atomicAdd(&A.cell_count[A.cell_id[i]], 1u);
+}
+
+// The sorted order (cell_off, perm, rank) of the cell ids in A.cell_id; the
+// sorted copies get the current positions.
+int sort_from_ids(const StepArgs &A, cudaStream_t st)
+{
     cudaMemsetAsync(A.cell_count, 0, sizeof(uint32_t) * A.ncells, st);
-    k_hash<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
+    k_recount<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
     const uint32_t nb = blocks_for(A.ncells, SCAN_TILE);
     k_scan_reduce<<<nb, SCAN_THREADS, 0, st>>>(A.cell_count, A.ncells, A.scan_tmp);
     k_scan_top<<<1, SCAN_THREADS, 0, st>>>(A.scan_tmp, nb);
     k_scan_down<<<nb, SCAN_THREADS, 0, st>>>(A.cell_count, A.ncells, A.scan_tmp, nb, A.cell_off);
     k_scatter<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
     k_place<false><<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
-    k_pair_vlist<<<blocks_for(A.ntot, VLIST_THREADS), VLIST_THREADS, 0, st>>>(A, P);
+    return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 
 int launch_step(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, uint64_t *launches,
@@ -957,10 +823,12 @@ int launch_step(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, uint6
     return launch_step_with(A, cfg, st, launches, prof, interact_fp64, contacts_fp64);
 }
 
-int launch_step_with(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
+int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t st,
                      uint64_t *launches, Prof *prof, InteractLauncher interact,
                      ContactLauncher contact)
 {
+    StepArgs A = args;
+    A.lazy_sort = cfg.lazy_sort && split_active(A, cfg) ? 1u : 0u;
     uint64_t nl = 0;
     // programmatic dependent launches along the step's chain of kernels,
     // except where events are recorded between them (profiling)
@@ -994,30 +862,35 @@ int launch_step_with(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
         cudaEventRecord(cfg.join, cfg.side);
     }
     if (A.ntot > 0) {
-        cudaMemsetAsync(A.cell_count, 0, sizeof(uint32_t) * A.ncells, st);
-        k_hash<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
-        mark(prof, st, "k_hash");
-        const uint32_t nb = blocks_for(A.ncells, SCAN_TILE);
-        launch_k(pdl, k_scan_reduce, nb, SCAN_THREADS, st, (const uint32_t *)A.cell_count,
-                 A.ncells, A.scan_tmp);
-        launch_k(pdl, k_scan_top, 1, SCAN_THREADS, st, A.scan_tmp, nb);
-        launch_k(pdl, k_scan_down, nb, SCAN_THREADS, st, (const uint32_t *)A.cell_count, A.ncells,
-                 (const uint32_t *)A.scan_tmp, nb, A.cell_off);
-        mark(prof, st, "k_scan(3)");
-        launch_k(pdl, k_scatter, blocks_for(A.ntot, 256), 256, st, A);
-        mark(prof, st, "k_scatter");
-        const bool split = cfg.variant == SPLIT_VARIANT && !cfg.unfused && cfg.all_cm23 &&
-                           A.vlist && A.csum;
-        if (split) launch_k(pdl, k_place<false>, blocks_for(A.ntot, 256), 256, st, A);
-        else launch_k(pdl, k_place<true>, blocks_for(A.ntot, 256), 256, st, A);
-        mark(prof, st, "k_place");
-        nl += 7;
-        if (A.vlist) {
-            const unsigned gv = blocks_for(A.ntot, VLIST_THREADS);
-            launch_k(pdl, k_vlist_build, gv < VLIST_BLOCKS ? gv : VLIST_BLOCKS, VLIST_THREADS, st, A);
-            launch_k(pdl, k_vlist_done, 1, 1, st, A);
-            mark(prof, st, "k_vlist");
-            nl += 2;
+        const bool split = split_active(A, cfg);
+        if (A.lazy_sort) {
+            launch_resort(k_resort, A.ntot, st, A, resort_sync(A));
+            mark(prof, st, "k_resort");
+            nl += 1;
+        } else {
+            cudaMemsetAsync(A.cell_count, 0, sizeof(uint32_t) * A.ncells, st);
+            k_hash<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
+            mark(prof, st, "k_hash");
+            const uint32_t nb = blocks_for(A.ncells, SCAN_TILE);
+            launch_k(pdl, k_scan_reduce, nb, SCAN_THREADS, st, (const uint32_t *)A.cell_count,
+                     A.ncells, A.scan_tmp);
+            launch_k(pdl, k_scan_top, 1, SCAN_THREADS, st, A.scan_tmp, nb);
+            launch_k(pdl, k_scan_down, nb, SCAN_THREADS, st, (const uint32_t *)A.cell_count, A.ncells,
+                     (const uint32_t *)A.scan_tmp, nb, A.cell_off);
+            mark(prof, st, "k_scan(3)");
+            launch_k(pdl, k_scatter, blocks_for(A.ntot, 256), 256, st, A);
+            mark(prof, st, "k_scatter");
+            if (split) launch_k(pdl, k_place<false>, blocks_for(A.ntot, 256), 256, st, A);
+            else launch_k(pdl, k_place<true>, blocks_for(A.ntot, 256), 256, st, A);
+            mark(prof, st, "k_place");
+            nl += 7;
+            if (A.vlist) {
+                const unsigned gv = blocks_for(A.ntot, VLIST_THREADS);
+                launch_k(pdl, k_vlist_build, gv < VLIST_BLOCKS ? gv : VLIST_BLOCKS, VLIST_THREADS, st, A);
+                launch_k(pdl, k_vlist_done, 1, 1, st, A);
+                mark(prof, st, "k_vlist");
+                nl += 2;
+            }
         }
         if (A.nbonds) {
             if (cfg.lenmode == SPH_LEN_FP64) k_bonds<SPH_LEN_FP64><<<blocks_for(A.nbonds, 128), 128, 0, st>>>(A);

@@ -49,6 +49,7 @@
 #include "sph_device.cuh"
 #include "sph_internal.h"
 #include "sph_mixed_laws.cuh"
+#include "sph_sort.cuh"
 #include "sph_step.cuh"
 #include "sph_sync.cuh"
 
@@ -657,20 +658,13 @@ __global__ void k_barrier_check(GridSync G, uint32_t expected, uint32_t rounds, 
         if (!grid_barrier(G, expected, err)) return;
 }
 
-// Rebuild request -> the condition of the rebuild node.
-__global__ void k_pair_cond(cudaGraphConditionalHandle hc, const uint32_t *vflag)
-{
-    cudaGraphSetConditional(hc, vflag[0] != 0u ? 1u : 0u);
-}
-
 // After a list build into the buffers not in use: each sphere's touching
 // entries (and their histories) carried over to the new list -- from the
 // old list, or, after pair_load, from the FP64 contact rows.
-__global__ void k_pair_remap(StepArgs A, PairArgs P)
+__device__ __forceinline__ void remap_sphere(const StepArgs &A, const PairArgs &P, uint32_t i,
+                                             uint32_t ls)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.ntot) return;
-    const uint32_t ls = *P.lsel, nw = ls ^ 1u;
+    const uint32_t nw = ls ^ 1u;
     const ListRow NL(P, nw, i);
     uint32_t nn = P.cnt[nw][i];
     if (nn > (uint32_t)VL_MAX) nn = 0;   // overflowed: raised by the step kernel
@@ -709,14 +703,14 @@ __global__ void k_pair_remap(StepArgs A, PairArgs P)
     P.live[nw][i] = live;
 }
 
-// The threads' order over the new lists (P.order[*lsel ^ 1]): within each
-// group of PAIR_ORDER_GROUP spheres, ascending list length, ties by index
-// (a stable rank), spheres past the end last.  One block per group.
-__global__ void __launch_bounds__(PAIR_ORDER_GROUP) k_pair_order(StepArgs A, PairArgs P)
+// The threads' order over the new lists (P.order[nw]) for one group of
+// PAIR_ORDER_GROUP spheres: ascending list length, ties by index (a stable
+// rank), spheres past the end last.  Thread t of the group, whose threads
+// run this together; s_key: the group's words of shared memory.
+__device__ __forceinline__ void order_sphere(const StepArgs &A, const PairArgs &P, uint32_t nw,
+                                             uint32_t base, uint32_t t, uint32_t *s_key)
 {
-    __shared__ uint32_t s_key[PAIR_ORDER_GROUP];
-    const uint32_t nw = *P.lsel ^ 1u;
-    const uint32_t base = blockIdx.x * PAIR_ORDER_GROUP, t = threadIdx.x, i = base + t;
+    const uint32_t i = base + t;
     uint32_t key = 0xffffffffu;
     if (i < A.ntot) key = min(P.cnt[nw][i], (uint32_t)VL_MAX + 1u);
     s_key[t] = key;
@@ -727,14 +721,42 @@ __global__ void __launch_bounds__(PAIR_ORDER_GROUP) k_pair_order(StepArgs A, Pai
         rank += (k < key || (k == key && u < t)) ? 1u : 0u;
     }
     if (i < A.ntot) P.order[nw][base + rank] = i;
+    __syncthreads();
 }
 
-__global__ void k_pair_done(StepArgs A, PairArgs P)
+// The list rebuild, when the integration of the step before asked for it
+// (or the state was just loaded): the current positions into A.x and the
+// cell sort, the lists into the buffers not in use, each sphere's touching
+// entries and histories carried over, the threads' order, and the hand-over.
+// One cooperative launch that ends at once on the other steps (1-2 us; the
+// same kernels behind a conditional graph node held every step up by about
+// 10 us, a quarter of a step of 20,000 spheres).
+__global__ void __launch_bounds__(RESORT_THREADS) k_pair_resort(StepArgs A, PairArgs P, GridSync G)
 {
-    *P.lsel ^= 1u;
-    *P.from_rows = 0u;
-    A.vflag[0] = 0u;
-    A.vflag[1] += 1u;
+    extern __shared__ uint32_t s_mem[];
+    if (A.vflag[0] == 0u) return;
+    const uint32_t ls = *P.lsel, nw = ls ^ 1u;
+    const double4 *xr = P.xr[*P.pp];
+    if (!sort_all<true>(A, G, s_mem + VL_MAX * RESORT_THREADS, [&](uint32_t i) { return xr[i]; }))
+        return;
+    const uint32_t nt = gridDim.x * RESORT_THREADS, t0 = blockIdx.x * RESORT_THREADS + threadIdx.x;
+    for (uint32_t a = t0; a < A.ntot; a += nt)
+        vlist_build_one(A, a, s_mem + threadIdx.x, P.ids[nw], P.cnt[nw], VL_MAX, 1u, P.nrow,
+                        RESORT_THREADS);
+    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    for (uint32_t i = t0; i < A.ntot; i += nt) remap_sphere(A, P, i, ls);
+    // RESORT_THREADS is a multiple of the group; the loop is uniform in a block
+    for (uint32_t base = blockIdx.x * RESORT_THREADS; base < A.ntot; base += nt) {
+        const uint32_t g = threadIdx.x / PAIR_ORDER_GROUP * PAIR_ORDER_GROUP;
+        order_sphere(A, P, nw, base + g, threadIdx.x - g, s_mem + g);
+    }
+    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *P.lsel = nw;
+        *P.from_rows = 0u;
+        A.vflag[0] = 0u;
+        A.vflag[1] += 1u;
+    }
 }
 
 // The FP64 arrays -> the compact state (into the [*pp] half); the next step
@@ -922,69 +944,19 @@ void launch_pair_kernel(const StepArgs &A, const PairArgs &P, const StepConfig &
     else launch_pair_lm<SPH_LEN_REFERENCE>(A, P, cfg.pair_shape, st);
 }
 
-void launch_rebuild_body(const StepArgs &A, const PairArgs &P, cudaStream_t st)
-{
-    launch_pair_sort_build(A, P, st);
-    k_pair_remap<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A, P);
-    k_pair_order<<<blocks_for(A.ntot, PAIR_ORDER_GROUP), PAIR_ORDER_GROUP, 0, st>>>(A, P);
-    k_pair_done<<<1, 1, 0, st>>>(A, P);
-}
-
 }  // namespace
 
-// One step of the list form on st.  Under stream capture the list rebuild
-// is a conditional node (run when the integration of the step before asked
-// for it); outside a capture the request is read on the host.  cfg.side:
-// a second stream, on which the conditional node's body is captured.
+// One step of the list form on st.
 int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg, cudaStream_t st,
                      uint64_t *launches, Prof *prof)
 {
-    uint64_t nl = 0;
+    uint64_t nl = 1;
     if (prof) {
         prof->n = 0;
         record(prof->ev[0], st);
     }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) return SPH_ERR_CUDA;
-    if (cs == cudaStreamCaptureStatusActive) {
-        if (!cfg.side) return SPH_ERR_CUDA;
-        cudaGraph_t g = nullptr;
-        const cudaGraphNode_t *deps = nullptr;
-        size_t nd = 0;
-        if (cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd) != cudaSuccess)
-            return SPH_ERR_CUDA;
-        cudaGraphConditionalHandle hc;
-        if (cudaGraphConditionalHandleCreate(&hc, g, 0u, cudaGraphCondAssignDefault) != cudaSuccess)
-            return SPH_ERR_CUDA;
-        k_pair_cond<<<1, 1, 0, st>>>(hc, A.vflag);
-        if (cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd) != cudaSuccess)
-            return SPH_ERR_CUDA;
-        cudaGraphNodeParams np = {};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = hc;
-        np.conditional.type = cudaGraphCondTypeIf;
-        np.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, g, deps, nd, &np) != cudaSuccess) return SPH_ERR_CUDA;
-        if (cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies) !=
-            cudaSuccess)
-            return SPH_ERR_CUDA;
-        cudaGraph_t body = np.conditional.phGraph_out[0];
-        if (cudaStreamBeginCaptureToGraph(cfg.side, body, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-            return SPH_ERR_CUDA;
-        launch_rebuild_body(A, P, cfg.side);
-        cudaGraph_t done = nullptr;
-        if (cudaStreamEndCapture(cfg.side, &done) != cudaSuccess) return SPH_ERR_CUDA;
-        nl += 1;
-    } else {
-        uint32_t flag = 0;
-        if (cudaMemcpyAsync(&flag, A.vflag, sizeof flag, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return SPH_ERR_CUDA;
-        if (flag) launch_rebuild_body(A, P, st);
-    }
-    mark(prof, st, "k_pair_cond");
+    launch_resort(k_pair_resort, A.ntot, st, A, P, resort_sync(A));
+    mark(prof, st, "k_pair_resort");
     launch_pair_kernel(A, P, cfg, st);
     if (pair_shape_persistent(cfg.pair_shape)) {
         // the persistent shapes do the wall stage themselves

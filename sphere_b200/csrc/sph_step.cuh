@@ -32,6 +32,33 @@ __device__ __forceinline__ uint32_t box_index(const StepArgs &A, uint32_t i)
     return A.nboxes == 1 ? 0u : A.box_of[i];
 }
 
+// floor((x - o) / (L / num)), the cell coordinate of sorting.cuh:7-20,
+// from a product with num / L: that differs from the quotient by a few units
+// in the last place, so away from an integer (by 1e-6, with |t| < 1e9) the
+// floors are equal; else (and for NaN) the quotient itself.
+__device__ __forceinline__ double cell_floor(double x, double o, double L, uint32_t num)
+{
+    const double d = x - o;
+    const double t = d * ((double)num / L);
+    const double f = floor(t);
+    if (fabs(t) < 1e9 && fabs((t - f) - 0.5) < 0.5 - 1e-6) return f;
+    return floor(d / (L / num));
+}
+
+// Clamped cell coordinates of a position, as the sort stores them, from its
+// cell_floor values; false when some coordinate lies outside the grid.
+__device__ __forceinline__ bool clamp_cell(const DevBox &B, const double f[3], uint32_t c[3])
+{
+    bool inside = true;
+    for (int d = 0; d < 3; ++d) {
+        double v = f[d];
+        if (!(v >= 0.0)) { inside = false; v = 0.0; }
+        if (v >= (double)B.num[d]) { inside = false; v = (double)(B.num[d] - 1); }
+        c[d] = (uint32_t)v;
+    }
+    return inside;
+}
+
 // ---------------------------------------------------------------- integrate
 
 // integration.cuh:14-305 integrate (TY3) for one particle.
@@ -130,6 +157,15 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
             else if (ey < -0.5f * ly) ey += ly;
         }
         if (!(ex * ex + ey * ey + ez * ez <= B.vdisp2)) A.vflag[0] = 1u;
+    }
+    if (A.lazy_sort) {
+        // the next step's contact search reads the spheres' cells
+        double f[3];
+        uint32_t c[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) f[d] = cell_floor(xn[d], B.origo[d], B.L[d], B.num[d]);
+        (void)clamp_cell(B, f, c);
+        A.cellc[i] = pack_cell(c[0], c[1], c[2]);
     }
     if (vel.w > 5.0 && vel.w < 10.0) {
         if (B.change_velocity_state == 1) vn[0] *= 10.0;
@@ -728,10 +764,20 @@ __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i,
 #pragma unroll
         for (int q = 0; q < NC / 4; ++q) tp[q] = grow[q];
     }
-    int g[3];
-    g[0] = (int)floor((xa.x - B.origo[0]) / (B.L[0] / B.num[0]));
-    g[1] = (int)floor((xa.y - B.origo[1]) / (B.L[1] / B.num[1]));
-    g[2] = (int)floor((xa.z - B.origo[2]) / (B.L[2] / B.num[2]));
+    double gf[3];
+    gf[0] = cell_floor(xa.x, B.origo[0], B.L[0], B.num[0]);
+    gf[1] = cell_floor(xa.y, B.origo[1], B.L[1], B.num[1]);
+    gf[2] = cell_floor(xa.z, B.origo[2], B.L[2], B.num[2]);
+    const int g[3] = {(int)gf[0], (int)gf[1], (int)gf[2]};
+    if (A.lazy_sort) {
+        // no k_hash in this step: its checks and its cell id
+        uint32_t c[3];
+        const bool inside = clamp_cell(B, gf, c);
+        if (!isfinite(xa.x) || !isfinite(xa.y) || !isfinite(xa.z)) raise_flag(A.err, SPH_ERR_NAN);
+        else if (!inside || xa.x > B.L[0] || xa.y > B.L[1] || xa.z > B.L[2])
+            raise_flag(A.err, SPH_ERR_OUT_OF_GRID);
+        A.cell_id[i] = B.cell_base + (c[2] * B.num[1]) * B.num[0] + c[1] * B.num[0] + c[0];
+    }
     const uint32_t *lst = A.vlist ? A.vlist + (size_t)i * VL_MAX : nullptr;
     const uint32_t vc = lst ? A.vcount[i] : (uint32_t)VL_MAX + 1u;
     // the first entries are read together with the count (the list row
