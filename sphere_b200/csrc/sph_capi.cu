@@ -175,7 +175,17 @@ static int ensure_pair(SphHandle *h)
         const uint32_t nch = (h->dbox[k].np + (1u << sph::PAIR_CHUNK_LOG2) - 1) >> sph::PAIR_CHUNK_LOG2;
         for (uint32_t c = 0; c < nch; ++c) cbox.push_back(k);
     }
-    uint32_t *chunk_box = nullptr, *box_chunk0 = nullptr, *words = nullptr;
+    // the keys of the compact numbering: 512 per 8 x 8 x 8-cell tile
+    std::vector<uint32_t> kb(h->nbox);
+    uint64_t nkeys = 0;
+    for (uint32_t k = 0; k < h->nbox; ++k) {
+        const uint32_t *num = h->dbox[k].num;
+        kb[k] = (uint32_t)nkeys;
+        nkeys += 512ull * ((num[0] + 7ull) / 8) * ((num[1] + 7ull) / 8) * ((num[2] + 7ull) / 8);
+        if (nkeys > sph::SCAN_MAX) break;
+    }
+    if (nkeys > sph::SCAN_MAX) nkeys = 0;
+    uint32_t *chunk_box = nullptr, *box_chunk0 = nullptr, *words = nullptr, *key_base = nullptr;
     int st;
     if ((st = dalloc(h, &P.xr[0], n)) || (st = dalloc(h, &P.xr[1], n)) ||
         (st = dalloc(h, &P.vw[0], 2 * n)) || (st = dalloc(h, &P.vw[1], 2 * n)) ||
@@ -191,8 +201,14 @@ static int ensure_pair(SphHandle *h)
         (st = dalloc(h, &P.hist[0], 3 * n * sph::VL_MAX)) ||
         (st = dalloc(h, &P.hist[1], 3 * n * sph::VL_MAX)) || (st = dalloc(h, &words, 5)) ||
         (st = dalloc(h, &P.chunk_part, cbox.size())) || (st = dalloc(h, &chunk_box, cbox.size())) ||
-        (st = dalloc(h, &box_chunk0, h->nbox)))
+        (st = dalloc(h, &box_chunk0, h->nbox)) || (st = dalloc(h, &key_base, h->nbox)) ||
+        (st = dalloc(h, &P.src, n)) || (st = dalloc(h, &P.dst, n)) ||
+        (st = dalloc(h, &P.key_count, nkeys)) || (st = dalloc(h, &P.key_off, nkeys + 1)) ||
+        (st = dalloc(h, &P.key_scan, nkeys / 4096 + 2)))
         return st;
+    P.key_base = key_base;
+    P.nkeys = (uint32_t)nkeys;
+    CUDA_TRY(h, cudaMemcpy(key_base, kb.data(), 4 * kb.size(), cudaMemcpyHostToDevice));
     P.pp = words;
     P.lsel = words + 1;
     P.from_rows = words + 2;
@@ -1090,6 +1106,7 @@ static int queue_steps(SphHandle *h, uint64_t nsteps, uint8_t *states)
 static int queue_steps_now(SphHandle *h, uint64_t nsteps, uint8_t *states)
 {
     int st;
+    if (nsteps == 0) return SPH_OK;
     if (h->eager) {
         // kernel by kernel on the handle's stream (no graphs)
         if ((st = prepare_steps(h)) != SPH_OK) return st;
@@ -1752,12 +1769,25 @@ int sph_get_sort(SphHandle *h, uint32_t *cell_id, uint32_t *perm, uint32_t *cell
     const uint64_t n = h->ntot, nc = h->ncells;
     // the lazily sorted split step keeps each step's cell ids; the order
     // that follows from them is made here
-    if (h->list_use == SphHandle::LISTS_LAZY && n && (perm || cell_start || cell_end)) {
-        int st = sph::sort_from_ids(h->A, h->stream);
+    // (of the last rebuild after list steps, from that step's numbering)
+    uint32_t *ids = nullptr;
+    if (n && (h->list_use == SphHandle::LISTS_LAZY || h->list_use == SphHandle::LISTS_PAIR)) {
+        StepArgs T = h->A;
+        int st = SPH_OK;
+        if (h->list_use == SphHandle::LISTS_PAIR) {
+            CUDA_TRY(h, cudaMalloc((void **)&ids, 4 * n));
+            st = sph::pair_public_ids(h->A, h->P, ids, h->stream);
+            T.cell_id = ids;
+        }
+        if (st == SPH_OK) st = sph::sort_from_ids(T, h->stream);
+        cudaError_t e = cudaStreamSynchronize(h->stream);
+        if (e == cudaSuccess && cell_id) e = cudaMemcpy(cell_id, T.cell_id, 4 * n, cudaMemcpyDeviceToHost);
+        cudaFree(ids);
         if (st != SPH_OK) return fail(h, st, "cell sort failed");
-        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        CUDA_TRY(h, e);
+    } else if (cell_id && n) {
+        CUDA_TRY(h, cudaMemcpy(cell_id, h->A.cell_id, 4 * n, cudaMemcpyDeviceToHost));
     }
-    if (cell_id && n) CUDA_TRY(h, cudaMemcpy(cell_id, h->A.cell_id, 4 * n, cudaMemcpyDeviceToHost));
     if (perm && n) CUDA_TRY(h, cudaMemcpy(perm, h->A.perm, 4 * n, cudaMemcpyDeviceToHost));
     if (cell_start || cell_end) {
         std::vector<uint32_t> off(nc + 1);

@@ -80,7 +80,8 @@ constexpr int PAIR_VARIANT = 4;        // the list step of the FP32-mixed form (
 constexpr uint32_t SPLIT_ID_MASK = 0x07ffffffu;   // sphere index bits of a live entry
 
 // The list step of the FP32-mixed form (launch variant 4, sph_pair.cu).
-// Its state lives in compact arrays of its own while it steps; the FP64
+// Its state lives in compact arrays of its own while it steps, in a
+// numbering of their own that follows the spheres' places (src, dst); the FP64
 // arrays of StepArgs are brought up to date from them (pair_flush) before
 // anything else reads them, and the compact arrays are loaded from them
 // (pair_load) before the first list step after anything wrote them.
@@ -119,6 +120,13 @@ struct PairArgs {
     // each group of PAIR_ORDER_GROUP consecutive spheres, by list length
     // (built with each list), so that a warp's lists are of similar length
     uint32_t *order[2];
+    // the numbering: src[j] = original index of compact sphere j, dst its
+    // inverse (a box's spheres keep the box's range), and the counting sort
+    // that makes it (k_pair_key; key_base: first key of each box)
+    uint32_t *src, *dst;
+    uint32_t *key_count, *key_off, *key_scan;
+    const uint32_t *key_base;
+    uint32_t nkeys;
     uint32_t *pp, *lsel;
     uint32_t *from_rows;       // != 0: the next rebuild takes histories from A.slots / A.hist
     uint32_t *bar;             // grid-barrier words of the persistent shapes: count, generation
@@ -297,6 +305,11 @@ int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st);
 int pair_flush(const StepArgs &A, const PairArgs &P, cudaStream_t st);
 int pair_count_live(const StepArgs &A, const PairArgs &P, cudaStream_t st,
                     unsigned long long *d_count);
+// The cell ids of the list step's last rebuild in the original numbering.
+int pair_public_ids(const StepArgs &A, const PairArgs &P, uint32_t *ids, cudaStream_t st);
+// Exclusive scan of n counts into off[0 .. n] (tmp: n / 4096 + 2 words).
+constexpr uint64_t SCAN_MAX = 4096ull * 4096ull;
+void scan_counts(const uint32_t *in, uint64_t n, uint32_t *tmp, uint32_t *off, cudaStream_t st);
 // Self-check of the grid barrier (sph_barrier_check): `rounds` barriers of
 // `expected` arrivals among `blocks` resident blocks; error bits in *err.
 int barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds,

@@ -802,16 +802,21 @@ __global__ void k_recount(StepArgs A)
     if (i < A.ntot) A.local_off[i] = atomicAdd(&A.cell_count[A.cell_id[i]], 1u);
 }
 
+void scan_counts(const uint32_t *in, uint64_t n, uint32_t *tmp, uint32_t *off, cudaStream_t st)
+{
+    const uint32_t nb = blocks_for(n, SCAN_TILE);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, st>>>(in, n, tmp);
+    k_scan_top<<<1, SCAN_THREADS, 0, st>>>(tmp, nb);
+    k_scan_down<<<nb, SCAN_THREADS, 0, st>>>(in, n, tmp, nb, off);
+}
+
 // The sorted order (cell_off, perm, rank) of the cell ids in A.cell_id; the
 // sorted copies get the current positions.
 int sort_from_ids(const StepArgs &A, cudaStream_t st)
 {
     cudaMemsetAsync(A.cell_count, 0, sizeof(uint32_t) * A.ncells, st);
     k_recount<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
-    const uint32_t nb = blocks_for(A.ncells, SCAN_TILE);
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, st>>>(A.cell_count, A.ncells, A.scan_tmp);
-    k_scan_top<<<1, SCAN_THREADS, 0, st>>>(A.scan_tmp, nb);
-    k_scan_down<<<nb, SCAN_THREADS, 0, st>>>(A.cell_count, A.ncells, A.scan_tmp, nb, A.cell_off);
+    scan_counts(A.cell_count, A.ncells, A.scan_tmp, A.cell_off, st);
     k_scatter<<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
     k_place<false><<<blocks_for(A.ntot, 256), 256, 0, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
