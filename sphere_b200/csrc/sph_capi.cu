@@ -73,6 +73,7 @@ struct SphHandle {
     int pnext = 0;
     uint64_t pcount = 0;
     bool uploaded = false;
+    bool variant_set = false;   // cfg.variant was chosen by the caller or the tuner
     std::string err;
     std::vector<void *> allocs;
     unsigned long long *d_count = nullptr;
@@ -95,6 +96,9 @@ struct SphHandle {
     // compact arrays hold the current state; pair_ahead: the FP64 arrays
     // of A are behind them (brought up to date by sync_public)
     sph::PairArgs P{};
+    // free slots may hold a history (sph_set_contacts): the next flush of the
+    // list step clears all of them
+    bool free_hist = false;
     bool pair_alloc = false, pair_valid = false, pair_ahead = false;
     // which steps the neighbour lists (and the cells of the lazily sorted
     // split step) belong to: prepare_steps asks for a rebuild when that
@@ -235,7 +239,8 @@ static int ensure_pair(SphHandle *h)
 static int sync_public(SphHandle *h)
 {
     if (!h->pair_ahead) return SPH_OK;
-    int st = sph::pair_flush(h->A, h->P, h->stream);
+    int st = sph::pair_flush(h->A, h->P, h->free_hist, h->stream);
+    h->free_hist = false;
     if (st != SPH_OK) return fail(h, st, "list-step state flush failed");
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     h->pair_ahead = false;
@@ -256,9 +261,17 @@ static StepConfig step_config(const SphHandle *h)
 {
     StepConfig cfg = h->cfg;
     cfg.lazy_sort = h->uploaded && !pair_active(h) && sph::split_active(h->A, cfg);
-    for (uint32_t k = 0; k < h->nbox; ++k)
-        if (h->boxes[k].grid.adaptive || (h->dbox[k].np > 0 && h->dbox[k].vrange < 1))
-            cfg.lazy_sort = false;
+    cfg.touch = true;
+    for (uint32_t k = 0; k < h->nbox; ++k) {
+        const DevBox &d = h->dbox[k];
+        if (h->boxes[k].grid.adaptive || (d.np > 0 && d.vrange < 1)) cfg.lazy_sort = false;
+        // a touching pair's distance, as the reference rounds it to FP32,
+        // may exceed 2 r_max by 6e-8 of itself
+        for (int c = 0; c < 3; ++c)
+            if (d.np > 0 && h->uploaded && !(d.L[c] / d.num[c] > 2.0 * h->rmax_box[k] * (1.0 + 1e-6)))
+                cfg.touch = false;
+    }
+    cfg.touch = cfg.touch && cfg.lazy_sort;
     return cfg;
 }
 
@@ -771,6 +784,9 @@ static int put1(SphHandle *h, double *dst, const double *src, uint64_t n, cudaSt
     return SPH_OK;
 }
 
+static int ensure_split(SphHandle *h);
+static int drop_graphs(SphHandle *h);
+
 int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
 {
     if (!h || !p) return SPH_ERR_INPUT;
@@ -917,6 +933,17 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
     // the caller's buffers are read only during the call
     CUDA_TRY(h, cudaStreamSynchronize(cs));
     h->uploaded = true;
+    // Unless a variant was chosen: the split step wherever it can run.  It
+    // gives the fused kernel's bits at every size and is faster at every
+    // size measured, since no thread walks a sphere's contacts one after the
+    // other (us a step, fused / split, shear pack, FP64: 500 spheres 66 / 45,
+    // 10,000 125 / 56, 60,000 181 / 80, 200,000 361 / 167; without contacts,
+    // 10,000 settling: 33 / 22).
+    if (!h->variant_set && n > 0 && h->cfg.all_cm23 && !h->cfg.unfused && A.vlist &&
+        h->cfg.variant != sph::SPLIT_VARIANT && ensure_split(h) == SPH_OK) {
+        h->cfg.variant = sph::SPLIT_VARIANT;
+        return drop_graphs(h);
+    }
     return SPH_OK;
 }
 
@@ -1596,7 +1623,8 @@ int sph_snapshot(SphHandle *h)
     }
     if (h->pair_ahead) {
         // the compact state into the FP64 arrays, on the stream, before the copies
-        int st = sph::pair_flush(h->A, h->P, h->stream);
+        int st = sph::pair_flush(h->A, h->P, h->free_hist, h->stream);
+        h->free_hist = false;
         if (st != SPH_OK) return fail(h, st, "list-step state flush failed");
         h->pair_ahead = false;
     }
@@ -1734,6 +1762,8 @@ int sph_set_contacts(SphHandle *h, const uint32_t *contacts, const double *delta
     k_image_codes<<<(unsigned)((ns + 255) / 256), 256, 0, h->stream>>>(h->A, ns);
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    CUDA_TRY(h, cudaMemset(h->A.vflag, 1, 1));   // k_touch's record of the rows is stale
+    h->free_hist = true;
     invalidate_pair(h);
     return SPH_OK;
 }
@@ -2181,7 +2211,7 @@ static int ensure_split(SphHandle *h)
     sph::Acc *csum = nullptr;
     int st;
     if ((st = dalloc(h, &lent, n * sph::NC)) || (st = dalloc(h, &nlive, n)) ||
-        (st = dalloc(h, &csum, n)))
+        (st = dalloc(h, &csum, n)) || (st = dalloc(h, &h->A.lmask, n)) || (st = dalloc(h, &h->A.occ, n)))
         return st;
     h->A.lent = lent;
     h->A.nlive = nlive;
@@ -2209,6 +2239,7 @@ int sph_set_variant(SphHandle *h, int variant)
         if (st != SPH_OK) return st;
     }
     h->cfg.variant = variant;
+    h->variant_set = true;
     return drop_graphs(h);
 }
 
@@ -2322,6 +2353,7 @@ int sph_autotune(SphHandle *h, uint32_t steps, double *ms_per_step, int *chosen)
     h->launches = launches_saved;
     cudaMemset(h->A.err, 0, sizeof(uint32_t));
     h->cfg.variant = best;
+    h->variant_set = true;
     h->cfg.pair_shape = best_shape;
     const int st2 = drop_graphs(h);
     if (st != SPH_OK) return fail(h, st, "autotune step failed");

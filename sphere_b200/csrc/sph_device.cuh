@@ -96,6 +96,18 @@ __device__ __forceinline__ double vlen(d3 v)
     if (LM == SPH_LEN_FP64) return sqrt(d);
     return (double)__fsqrt_rn(__double2float_rn(d));
 }
+// vlen<LM> with the dot product rounded operation by operation, also where
+// the file is compiled with contraction (the overlap tests of the contact
+// search, whose outcome is the same in both forms).
+template <int LM>
+__device__ __forceinline__ double len_rn(d3 v)
+{
+    const double d = __dadd_rn(__dadd_rn(__dmul_rn(v.x, v.x), __dmul_rn(v.y, v.y)),
+                               __dmul_rn(v.z, v.z));
+    if (LM == SPH_LEN_FP64) return __dsqrt_rn(d);
+    return (double)__fsqrt_rn(__double2float_rn(d));
+}
+
 __device__ __forceinline__ double fsqrtf_d(double d)
 {
     return (double)__fsqrt_rn(__double2float_rn(d));

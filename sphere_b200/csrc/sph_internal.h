@@ -57,6 +57,12 @@ struct StepArgs {
     // the split step without a sort per step: k_search checks its sphere's
     // position and stores its cell id, k_finish the cell of its new position
     uint32_t lazy_sort;
+    // k_touch in the place of k_search and k_contacts: per sphere the list
+    // entries whose partners are in its row (LMASK_VALID: known) and the
+    // occupied slots
+    uint32_t touch;
+    unsigned long long *lmask;
+    uint32_t *occ;
     // split step (k_search / k_contacts / k_finish): per warp of 32
     // original indexes, a region of 32 * NC entries holding the warp's live
     // contacts from its start, sphere after sphere, each in slot order
@@ -226,6 +232,9 @@ struct StepConfig {
     // the split step sorts only when its lists are rebuilt (k_resort); not
     // with an adaptive grid, whose cells change at every step
     bool lazy_sort = false;
+    // ... and searches in the contact kernel (k_touch): every cell wider
+    // than the largest diameter
+    bool touch = false;
     int phase = STEP_WHOLE;
     cudaStream_t side = nullptr;                       // STEP_OVERLAP only
     cudaEvent_t fork = nullptr, join = nullptr;        // STEP_OVERLAP only
@@ -302,7 +311,8 @@ int launch_step_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
 int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg, cudaStream_t st,
                      uint64_t *launches, Prof *prof);
 int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st);
-int pair_flush(const StepArgs &A, const PairArgs &P, cudaStream_t st);
+// (all: clear the history of every free slot)
+int pair_flush(const StepArgs &A, const PairArgs &P, bool all, cudaStream_t st);
 int pair_count_live(const StepArgs &A, const PairArgs &P, cudaStream_t st,
                     unsigned long long *d_count);
 // The cell ids of the list step's last rebuild in the original numbering.

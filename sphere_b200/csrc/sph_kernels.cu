@@ -163,9 +163,12 @@ __global__ void __launch_bounds__(RESORT_THREADS) k_resort(StepArgs A, GridSync 
     uint32_t none = 0;
     for (uint32_t a = blockIdx.x * RESORT_THREADS + threadIdx.x; a < A.ntot;
          a += gridDim.x * RESORT_THREADS)
+    {
         if (!vlist_build_one(A, a, s_mem + threadIdx.x, A.vlist, A.vcount, A.vcap, VL_MAX, 1u,
                              RESORT_THREADS))
             none = 1u;
+        A.lmask[A.perm[a]] = 0ull;   // new lists: k_touch goes through the row
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) A.vflag[2] = 0u;
     if (!grid_barrier(G, gridDim.x, A.err)) return;
     if (none) A.vflag[2] = 1u;
@@ -834,6 +837,7 @@ int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t s
 {
     StepArgs A = args;
     A.lazy_sort = cfg.lazy_sort && split_active(A, cfg) ? 1u : 0u;
+    A.touch = A.lazy_sort && cfg.touch ? 1u : 0u;
     uint64_t nl = 0;
     // programmatic dependent launches along the step's chain of kernels,
     // except where events are recorded between them (profiling)
@@ -908,20 +912,23 @@ int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t s
             const unsigned gs = blocks_for(A.ntot, SEARCH_THREADS);
             // after k_bonds (when there are bonds) an ordinary launch
             const bool pdl_s = pdl && !A.nbonds;
-            if (cfg.lenmode == SPH_LEN_FP64)
-                launch_k(pdl_s, k_search<SPH_LEN_FP64>, gs, SEARCH_THREADS, st, A);
-            else
-                launch_k(pdl_s, k_search<SPH_LEN_REFERENCE>, gs, SEARCH_THREADS, st, A);
-            mark(prof, st, "k_search");
-            contact(A, st, blocks_for(A.ntot, CONTACT_THREADS), cfg.lenmode, pdl);
-            mark(prof, st, "k_contacts");
+            if (!A.touch) {
+                if (cfg.lenmode == SPH_LEN_FP64)
+                    launch_k(pdl_s, k_search<SPH_LEN_FP64>, gs, SEARCH_THREADS, st, A);
+                else
+                    launch_k(pdl_s, k_search<SPH_LEN_REFERENCE>, gs, SEARCH_THREADS, st, A);
+                mark(prof, st, "k_search");
+                nl += 1;
+            }
+            contact(A, st, blocks_for(A.ntot, CONTACT_THREADS), cfg.lenmode, A.touch ? pdl_s : pdl);
+            mark(prof, st, A.touch ? "k_touch" : "k_contacts");
             if (overlap) cudaStreamWaitEvent(st, cfg.join, 0);
             if (cfg.lenmode == SPH_LEN_FP64)
                 k_finish<SPH_LEN_FP64><<<blocks_for(A.ntot, FINISH_THREADS), FINISH_THREADS, 0, st>>>(A);
             else
                 k_finish<SPH_LEN_REFERENCE><<<blocks_for(A.ntot, FINISH_THREADS), FINISH_THREADS, 0, st>>>(A);
             mark(prof, st, "k_finish");
-            nl += 3;
+            nl += 2;
         } else if (!cfg.unfused) {
             if (overlap) cudaStreamWaitEvent(st, cfg.join, 0);
             interact(A, st, gi, true, cfg.lenmode,

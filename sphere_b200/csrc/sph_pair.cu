@@ -82,16 +82,6 @@ __device__ __forceinline__ d3 centre_line(const DevBox &B, const double4 &xa, co
     return mk(dx, dy, dz);
 }
 
-// vlen<LM> with the dot product rounded operation by operation.
-template <int LM>
-__device__ __forceinline__ double len_rn(d3 v)
-{
-    const double d = __dadd_rn(__dadd_rn(__dmul_rn(v.x, v.x), __dmul_rn(v.y, v.y)),
-                               __dmul_rn(v.z, v.z));
-    if (LM == SPH_LEN_FP64) return __dsqrt_rn(d);
-    return (double)__fsqrt_rn(__double2float_rn(d));
-}
-
 // Sphere i's list and history in their entry-major layout (PairArgs):
 // entry k's id at ids[k * nrow], history component c at
 // hist[(3 k + c) * nrow], from the sphere's own column.
@@ -861,9 +851,9 @@ __global__ void k_pair_load(StepArgs A, PairArgs P)
 // list -> the sphere's contact row (by ascending partner, slots 0, 1, ...)
 // with their histories and image codes.  A free slot's history is zero by
 // construction (upload, ended contacts), so only the slots that the row
-// held and no longer holds are cleared: 1 KB per sphere less to write (885
+// held and no longer holds are cleared (all: every free slot): 1 KB per sphere less to write (885
 // -> 190 us at 1e6 spheres).
-__global__ void k_pair_flush(StepArgs A, PairArgs P)
+__global__ void k_pair_flush(StepArgs A, PairArgs P, bool all)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= A.ntot) return;
@@ -916,7 +906,7 @@ __global__ void k_pair_flush(StepArgs A, PairArgs P)
         ++s;
     }
     for (; s < NC; ++s) {
-        if (row[s] == EMPTY) continue;
+        if (row[s] == EMPTY && !all) continue;
         row[s] = EMPTY;
         hist[s] = make_double4(0.0, 0.0, 0.0, 0.0);
     }
@@ -1125,9 +1115,9 @@ int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 
-int pair_flush(const StepArgs &A, const PairArgs &P, cudaStream_t st)
+int pair_flush(const StepArgs &A, const PairArgs &P, bool all, cudaStream_t st)
 {
-    if (A.ntot) k_pair_flush<<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P);
+    if (A.ntot) k_pair_flush<<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P, all);
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 

@@ -241,7 +241,7 @@ __device__ __forceinline__ uint16_t list_key(const StepArgs &A, const DevBox &B,
     const d3 dm = shift_vec(B, sx, sy);
     d3 x_ab = mk(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z);
     x_ab = vadd(x_ab, dm);
-    const double len = vlen<LM>(x_ab);
+    const double len = len_rn<LM>(x_ab);
     if (!(len - (xa.w + xb.w) < 0.0)) return NO_KEY;
     const int ord = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
     return (uint16_t)((ord << 10) | (shift_code(sx, sy) << 6) | (int)k);
@@ -290,7 +290,7 @@ __device__ __forceinline__ void list_keys_batch(const StepArgs &A, const DevBox 
         const d3 dm = shift_vec(B, sx, sy);
         d3 x_ab = mk(xa.x - xb[j].x, xa.y - xb[j].y, xa.z - xb[j].z);
         x_ab = vadd(x_ab, dm);
-        const double len = vlen<LM>(x_ab);
+        const double len = len_rn<LM>(x_ab);
         if (!(len - (xa.w + xb[j].w) < 0.0)) continue;
         const int ord = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
         out[j] = (uint16_t)((ord << 10) | (shift_code(sx, sy) << 6) | (int)(k0 + j));
@@ -387,7 +387,7 @@ __device__ __forceinline__ bool search_cells(const StepArgs &A, const DevBox &B,
                     const double4 xb = A.xs[b];
                     d3 x_ab = mk(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z);
                     x_ab = vadd(x_ab, dm);
-                    const double len = vlen<LM>(x_ab);
+                    const double len = len_rn<LM>(x_ab);
                     const double delta = len - (radius_a + xb.w);
                     if (delta < 0.0) {
                         const uint32_t b_orig = A.perm[b];
@@ -718,7 +718,8 @@ __global__ void __launch_bounds__(INTERACT_THREADS, MINB) k_interact(StepArgs A)
 // ------------------------------------------------------------ split step
 //
 // The step of k_interact for contact models 2 and 3 with fused integration,
-// in three launches that keep more memory requests in flight:
+// in three launches that keep more memory requests in flight (two where
+// k_touch takes the place of the first two):
 //   k_search   one thread per sphere: contact search on the slot row (kept
 //              with a bitmask of the slots in use), the list of live slots
 //              (ascending);
@@ -736,10 +737,42 @@ constexpr int SEARCH_THREADS = 128;
 constexpr int CONTACT_THREADS = 128;
 constexpr int FINISH_THREADS = 128;
 
+// In a step without k_hash: its checks of the sphere's position and its cell
+// id.
+__device__ __forceinline__ void position_check(const StepArgs &A, const DevBox &B, uint32_t i,
+                                               double4 x)
+{
+    const double f[3] = {cell_floor(x.x, B.origo[0], B.L[0], B.num[0]),
+                         cell_floor(x.y, B.origo[1], B.L[1], B.num[1]),
+                         cell_floor(x.z, B.origo[2], B.L[2], B.num[2])};
+    uint32_t c[3];
+    const bool inside = clamp_cell(B, f, c);
+    if (!isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z)) raise_flag(A.err, SPH_ERR_NAN);
+    else if (!inside || x.x > B.L[0] || x.y > B.L[1] || x.z > B.L[2])
+        raise_flag(A.err, SPH_ERR_OUT_OF_GRID);
+    A.cell_id[i] = B.cell_base + (c[2] * B.num[1]) * B.num[0] + c[1] * B.num[0] + c[0];
+}
+
+// The image shift that brings b nearest to a along the periodic axes.
+__device__ __forceinline__ void nearest_image(const DevBox &B, const double4 &xa, const double4 &xb,
+                                              int &sx, int &sy)
+{
+    sx = sy = 0;
+    if (B.periodic == 1 || B.periodic == 2) {
+        const double d = xa.x - xb.x;
+        sx = d > 0.5 * B.L[0] ? -1 : (d < -0.5 * B.L[0] ? 1 : 0);
+    }
+    if (B.periodic == 1) {
+        const double d = xa.y - xb.y;
+        sy = d > 0.5 * B.L[1] ? -1 : (d < -0.5 * B.L[1] ? 1 : 0);
+    }
+}
+
 // Contact search of sphere i (original index: its row, list and state are
 // read without a permutation lookup) on its slot row, staged in shared
-// memory (row[s * RS]); returns the bitmask of occupied slots.
-template <int LM>
+// memory (row[s * RS]), or, IN_PLACE, in the row itself; returns the bitmask
+// of occupied slots.
+template <int LM, bool IN_PLACE>
 __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i, uint32_t *row,
                                                   uint16_t *keys, int RS)
 {
@@ -750,10 +783,12 @@ __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i,
 #pragma unroll
     for (int q = 0; q < NC / 4; ++q) {
         const uint4 w = grow[q];
-        row[(4 * q + 0) * RS] = w.x;
-        row[(4 * q + 1) * RS] = w.y;
-        row[(4 * q + 2) * RS] = w.z;
-        row[(4 * q + 3) * RS] = w.w;
+        if (!IN_PLACE) {
+            row[(4 * q + 0) * RS] = w.x;
+            row[(4 * q + 1) * RS] = w.y;
+            row[(4 * q + 2) * RS] = w.z;
+            row[(4 * q + 3) * RS] = w.w;
+        }
         occ |= (w.x != EMPTY ? 1u : 0u) << (4 * q);
         occ |= (w.y != EMPTY ? 1u : 0u) << (4 * q + 1);
         occ |= (w.z != EMPTY ? 1u : 0u) << (4 * q + 2);
@@ -769,15 +804,7 @@ __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i,
     gf[1] = cell_floor(xa.y, B.origo[1], B.L[1], B.num[1]);
     gf[2] = cell_floor(xa.z, B.origo[2], B.L[2], B.num[2]);
     const int g[3] = {(int)gf[0], (int)gf[1], (int)gf[2]};
-    if (A.lazy_sort) {
-        // no k_hash in this step: its checks and its cell id
-        uint32_t c[3];
-        const bool inside = clamp_cell(B, gf, c);
-        if (!isfinite(xa.x) || !isfinite(xa.y) || !isfinite(xa.z)) raise_flag(A.err, SPH_ERR_NAN);
-        else if (!inside || xa.x > B.L[0] || xa.y > B.L[1] || xa.z > B.L[2])
-            raise_flag(A.err, SPH_ERR_OUT_OF_GRID);
-        A.cell_id[i] = B.cell_base + (c[2] * B.num[1]) * B.num[0] + c[1] * B.num[0] + c[0];
-    }
+    if (!IN_PLACE && A.lazy_sort) position_check(A, B, i, xa);
     const uint32_t *lst = A.vlist ? A.vlist + (size_t)i * VL_MAX : nullptr;
     const uint32_t vc = lst ? A.vcount[i] : (uint32_t)VL_MAX + 1u;
     // the first entries are read together with the count (the list row
@@ -867,7 +894,7 @@ __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i,
             if (w != EMPTY) A.tape_hist[(size_t)i * NC + s] = hist[s];
         }
     }
-    if (dirty) {
+    if (!IN_PLACE && dirty) {
         uint4 *wrow = reinterpret_cast<uint4 *>(A.slots + (size_t)i * NC);
 #pragma unroll
         for (int q = 0; q < NC / 4; ++q)
@@ -888,7 +915,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_search(StepArgs A)
     const int RS = SEARCH_THREADS;
     uint32_t *row = s_row + threadIdx.x;
     const uint32_t occ =
-        i < A.ntot ? search_sphere<LM>(A, i, row, s_keys + threadIdx.x, RS) : 0u;
+        i < A.ntot ? search_sphere<LM, false>(A, i, row, s_keys + threadIdx.x, RS) : 0u;
     // the warp's live contacts, sphere after sphere, each in slot order,
     // written contiguously from the start of the warp's region
     const uint32_t nl = __popc(occ);
@@ -946,6 +973,121 @@ __device__ __forceinline__ ContactRec get_rec(const RecSlab &S, int t)
     return r;
 }
 
+// The contact of slot s (word w) of sphere i: the law with its additions
+// recorded in r and the new history written, or the slot freed when the
+// pair no longer touches (r.nev < 0 then); returns whether it touches.
+// NEAREST: the image is the nearest one (see k_touch) and the slot's code is
+// brought up to date; else the slot's code says it.
+template <int LM, bool MIXED, bool NEAREST>
+__device__ __forceinline__ bool slot_contact(const StepArgs &A, uint32_t i, int s, uint32_t w,
+                                             ContactRec &r)
+{
+    const DevBox &B = A.boxes[box_index(A, i)];
+    const SphParams &P = B.P;
+    const double dt = B.dt;
+    const uint32_t cm = P.contactmodel;
+    // the sphere's own data in original order (the step's start
+    // state until k_finish), like its partner's
+    const double4 xa = A.x[i];
+    const double radius_a = xa.w;
+    const d3 vel_a = xyz(A.vel[i]);
+    const d3 angvel_a = xyz(A.angvel[i]);
+    uint32_t *slots = A.slots + (size_t)i * NC;
+    double4 *hist = A.hist + (size_t)i * NC;
+    const uint32_t bo = w & ID_MASK;   // partner's original id
+    // the partner's data (original order: A.x, A.vel, A.angvel hold
+    // the step's start state until k_finish) and the history are
+    // loaded together
+    const double4 xb = A.x[bo];
+    const double4 vb4 = A.vel[bo];
+    const double4 wb4 = A.angvel[bo];
+    const double4 h4 = hist[s];
+    int sx, sy;
+    if (NEAREST) nearest_image(B, xa, xb, sx, sy);
+    else decode_shift(w >> CODE_SHIFT, sx, sy);
+    const d3 dm = shift_vec(B, sx, sy);
+    const d3 x_ab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
+    const double x_ab_length = vlen<LM>(x_ab);
+    const double delta_n = x_ab_length - (radius_a + xb.w);
+    if (!(delta_n < 0.0)) {
+        slots[s] = EMPTY;
+        hist[s] = make_double4(0.0, 0.0, 0.0, 0.0);
+        return false;
+    }
+    if (NEAREST) {
+        const uint32_t v = bo | (shift_code(sx, sy) << CODE_SHIFT);
+        if (v != w) {
+            slots[s] = v;
+            if (A.tape_rows_post) A.tape_rows_post[(size_t)i * NC + s] = v;
+        }
+    }
+    r.nev = 0;
+    const d3 vel_b = xyz(vb4);
+    const d3 h0 = xyz(h4);
+    d3 nd;
+    if (MIXED) {
+        const MixedPair mp = mixed_pair(x_ab, x_ab_length, delta_n, vel_a, vel_b,
+                                        tof(angvel_a), xyzf(wb4), radius_a, xb.w);
+        if (cm == 2) nd = contact_linear_mixed(P, dt, r, mp, h0);
+        else nd = contact_hertz_mixed(P, dt, r, mp, h0);
+    } else {
+        const d3 angvel_b = xyz(wb4);
+        if (cm == 2)
+            nd = contact_linear<LM>(P, dt, r, vel_a, vel_b, angvel_a, angvel_b,
+                                    radius_a, xb.w, x_ab, x_ab_length, delta_n, h0);
+        else
+            nd = contact_hertz<LM>(P, dt, r, vel_a, vel_b, angvel_a, angvel_b,
+                                   radius_a, xb.w, x_ab, x_ab_length, delta_n, h0);
+    }
+    hist[s] = make_double4(nd.x, nd.y, nd.z, 0.0);
+    return true;
+}
+
+__device__ __forceinline__ Acc zero_acc()
+{
+    Acc acc;
+    acc.F = mk(0.0, 0.0, 0.0);
+    acc.T = mk(0.0, 0.0, 0.0);
+    acc.es_dot = 0.0;
+    acc.ev_dot = 0.0;
+    acc.p = 0.0;
+    return acc;
+}
+
+__device__ __forceinline__ ContactRec no_rec()
+{
+    ContactRec r;
+    r.F = mk(0.0, 0.0, 0.0);
+    r.T = mk(0.0, 0.0, 0.0);
+    r.ev0 = r.ev1 = r.es = r.p = 0.0;
+    r.nev = -1;   // nothing to add unless a live contact is computed
+    r.nes = 0;
+    return r;
+}
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, uint32_t lane)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += u;
+    }
+    return v;
+}
+
+// The records of one warp round (S, from the warp's word wbase) that belong
+// to the lane's sphere -- contacts [excl, incl) of the warp -- added in slot
+// order.
+__device__ __forceinline__ void replay_round(Acc &acc, const RecSlab &S, int wbase, uint32_t base,
+                                             uint32_t excl, uint32_t incl)
+{
+    const uint32_t lo = max(excl, base), hi = min(incl, base + 32u);
+    for (uint32_t e = lo; e < hi; ++e) {
+        const ContactRec o = get_rec(S, wbase + (int)(e - base));
+        if (o.nev >= 0) replay(acc, o);
+    }
+}
+
 // One warp per 32 consecutive spheres (original indexes), its lanes dealt
 // the warp's live contacts in order: round r computes contacts 32r .. 32r +
 // 31 of the warp's list (the spheres' live lists one after the other), so a
@@ -962,94 +1104,195 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_contacts(StepArgs A)
     const uint32_t i0 = i_own - lane;
     const bool valid = i_own < A.ntot;
     const uint32_t nl_own = valid ? A.nlive[i_own] : 0u;
-    // inclusive prefix sum of the live counts over the warp
-    uint32_t incl = nl_own;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += v;
-    }
+    const uint32_t incl = warp_inclusive(nl_own, lane);
     const uint32_t excl = incl - nl_own;
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    Acc acc;
-    acc.F = mk(0.0, 0.0, 0.0);
-    acc.T = mk(0.0, 0.0, 0.0);
-    acc.es_dot = 0.0;
-    acc.ev_dot = 0.0;
-    acc.p = 0.0;
+    Acc acc = zero_acc();
     const uint2 *ent = A.lent + (size_t)i0 * NC;
     for (uint32_t base = 0; base < total; base += 32) {
         const uint32_t f = base + lane;
-        ContactRec r;
-        r.F = mk(0.0, 0.0, 0.0);
-        r.T = mk(0.0, 0.0, 0.0);
-        r.ev0 = r.ev1 = r.es = r.p = 0.0;
-        r.nev = -1;   // nothing to add unless a live contact is computed
-        r.nes = 0;
+        ContactRec r = no_rec();
         if (f < total) {
             const uint2 e = ent[f];
-            const uint32_t i = e.y & SPLIT_ID_MASK;
-            const int s = (int)(e.y >> 27);
-            const uint32_t w = e.x;
-            const DevBox &B = A.boxes[box_index(A, i)];
-            const SphParams &P = B.P;
-            const double dt = B.dt;
-            const uint32_t cm = P.contactmodel;
-            // the sphere's own data in original order (the step's start
-            // state until k_finish), like its partner's
-            const double4 xa = A.x[i];
-            const double radius_a = xa.w;
-            const d3 vel_a = xyz(A.vel[i]);
-            const d3 angvel_a = xyz(A.angvel[i]);
-            uint32_t *slots = A.slots + (size_t)i * NC;
-            double4 *hist = A.hist + (size_t)i * NC;
-            const uint32_t bo = w & ID_MASK;   // partner's original id
+            (void)slot_contact<LM, MIXED, false>(A, e.y & SPLIT_ID_MASK, (int)(e.y >> 27), e.x, r);
+        }
+        put_rec(S, (int)threadIdx.x, r);
+        __syncwarp();
+        replay_round(acc, S, wbase, base, excl, incl);
+        __syncwarp();
+    }
+    if (valid) A.csum[i_own] = acc;
+}
+
+// Search and contacts in one kernel, for the lazily sorted split step on
+// grids whose cells are wider than the largest diameter (cfg.touch).
+//
+// The search's work hardly changes from step to step: the row keeps its
+// contacts, and an entry of the neighbour list that is not in the row seldom
+// starts to touch.  So the entries that are in the row are remembered (a bit
+// per list entry, A.lmask, with LMASK_VALID while it holds; the occupied
+// slots in A.occ), and a step tests only the others.  One that touches takes
+// the highest free slot, as the reference's rule has it; only when several
+// do, or the lists are new, does the sphere go through search_sphere, on its
+// row in memory.  At 1e6 spheres in contact with 4.3
+// others of 5.7 listed that leaves 1.4 position gathers per sphere of the
+// row, the list and 5.7 cell gathers.
+//
+// The image of a pair is the nearest one.  A touching pair's centres are
+// less than a cell apart along each axis, so their cells are neighbours, and
+// with at least three cells along a periodic axis the image under which the
+// cell search visits the partner is the nearest; a pair that touches under
+// neither is no contact under both.
+//
+// Contacts are then dealt to the warp's lanes as in k_contacts, contact f of
+// the warp found from the lanes' counts and occupied slots.
+constexpr unsigned long long LMASK_VALID = 1ull << 63;
+
+// The search of sphere i on its row in memory; which entries of its list are
+// in the row is found anew.  (Rare: not inlined, for the registers.)
+template <int LM>
+__device__ __noinline__ uint32_t touch_row(const StepArgs &A, uint32_t i)
+{
+    uint32_t *row = A.slots + (size_t)i * NC;
+    const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
+    const uint32_t vc = A.vcount[i];
+    uint16_t keys[VL_MAX];
+    const uint32_t occ = search_sphere<LM, true>(A, i, row, keys, 1);
+    A.occ[i] = occ;
+    // the list entries that are in the row
+    unsigned long long in = 0ull;
+    if (vc <= (uint32_t)VL_MAX) {
+        for (uint32_t m2 = occ; m2; m2 &= m2 - 1u) {
+            const uint32_t b = row[__ffs(m2) - 1] & ID_MASK;
+            for (uint32_t k = 0; k < vc; ++k)
+                if (lst[k] == b) in |= 1ull << k;
+        }
+        in |= LMASK_VALID;
+    }
+    A.lmask[i] = in;
+    return occ;
+}
+
+template <int LM>
+__device__ __forceinline__ uint32_t touch_search(const StepArgs &A, uint32_t i)
+{
+    const DevBox &B = A.boxes[box_index(A, i)];
+    const unsigned long long m = A.lmask[i];
+    const uint32_t vc = A.vcount[i];
+    uint32_t occ = A.occ[i];
+    const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
+    const double4 xa = A.x[i];
+    position_check(A, B, i, xa);
+    if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return touch_row<LM>(A, i);
+    // the first entry that is not in the row and touches, and its slot word
+    uint32_t found = 0, kf = 0, wf = 0;
+    for (unsigned long long todo = ((1ull << vc) - 1ull) & ~m; todo;) {
+        // the next KB entries' gathers in flight together
+        uint32_t bo[KB], ke[KB];
+        double4 xb[KB];
+        int nb = 0;
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+            if (todo) {
+                ke[j] = (uint32_t)(__ffsll((long long)todo) - 1);
+                bo[j] = lst[ke[j]];
+                todo &= todo - 1ull;
+                ++nb;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < KB; ++j)
+            if (j < nb) xb[j] = A.x[bo[j]];
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+            if (j >= nb) continue;
             int sx, sy;
-            decode_shift(w >> CODE_SHIFT, sx, sy);
+            nearest_image(B, xa, xb[j], sx, sy);
             const d3 dm = shift_vec(B, sx, sy);
-            // the partner's data (original order: A.x, A.vel, A.angvel hold
-            // the step's start state until k_finish) and the history are
-            // loaded together
-            const double4 xb = A.x[bo];
-            const double4 vb4 = A.vel[bo];
-            const double4 wb4 = A.angvel[bo];
-            const double4 h4 = hist[s];
-            const d3 x_ab = mk(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
-            const double x_ab_length = vlen<LM>(x_ab);
-            const double delta_n = x_ab_length - (radius_a + xb.w);
-            if (delta_n < 0.0) {
-                r.nev = 0;
-                const d3 vel_b = xyz(vb4);
-                const d3 h0 = xyz(h4);
-                d3 nd;
-                if (MIXED) {
-                    const MixedPair mp = mixed_pair(x_ab, x_ab_length, delta_n, vel_a, vel_b,
-                                                    tof(angvel_a), xyzf(wb4), radius_a, xb.w);
-                    if (cm == 2) nd = contact_linear_mixed(P, dt, r, mp, h0);
-                    else nd = contact_hertz_mixed(P, dt, r, mp, h0);
-                } else {
-                    const d3 angvel_b = xyz(wb4);
-                    if (cm == 2)
-                        nd = contact_linear<LM>(P, dt, r, vel_a, vel_b, angvel_a, angvel_b,
-                                                radius_a, xb.w, x_ab, x_ab_length, delta_n, h0);
-                    else
-                        nd = contact_hertz<LM>(P, dt, r, vel_a, vel_b, angvel_a, angvel_b,
-                                               radius_a, xb.w, x_ab, x_ab_length, delta_n, h0);
+            d3 x_ab = mk(xa.x - xb[j].x, xa.y - xb[j].y, xa.z - xb[j].z);
+            x_ab = vadd(x_ab, dm);
+            if (len_rn<LM>(x_ab) - (xa.w + xb[j].w) < 0.0) {
+                if (found++ == 0u) {
+                    kf = ke[j];
+                    wf = bo[j] | (shift_code(sx, sy) << CODE_SHIFT);
                 }
-                hist[s] = make_double4(nd.x, nd.y, nd.z, 0.0);
-            } else {
-                slots[s] = EMPTY;
-                hist[s] = make_double4(0.0, 0.0, 0.0, 0.0);
+            }
+        }
+    }
+    // several new contacts take their slots in the cells' visit order
+    if (found > 1u || (found == 1u && occ == 0xffffffffu)) return touch_row<LM>(A, i);
+    uint32_t *row = A.slots + (size_t)i * NC;
+    if (A.tape_rows_pre)
+        for (int s = 0; s < NC; ++s) A.tape_rows_pre[(size_t)i * NC + s] = row[s];
+    if (found) {
+        // one: the highest free slot
+        const int s = 31 - __clz((int)~occ);
+        row[s] = wf;
+        occ |= 1u << s;
+        A.occ[i] = occ;
+        A.lmask[i] = m | (1ull << kf);
+    }
+    if (A.tape_rows_post) {
+        const double4 *hist = A.hist + (size_t)i * NC;
+        for (int s = 0; s < NC; ++s) {
+            const uint32_t w = row[s];
+            A.tape_rows_post[(size_t)i * NC + s] = w;
+            if (w != EMPTY) A.tape_hist[(size_t)i * NC + s] = hist[s];
+        }
+    }
+    return occ;
+}
+
+template <int LM, bool MIXED>
+__global__ void __launch_bounds__(CONTACT_THREADS, 6) k_touch(const __grid_constant__ StepArgs A)
+{
+    __shared__ RecSlab S;
+    grid_dependency_wait();
+    const uint32_t lane = threadIdx.x & 31u;
+    const int wbase = (int)(threadIdx.x & ~31u);
+    const uint32_t i_own = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i0 = i_own - lane;
+    const bool valid = i_own < A.ntot;
+    const uint32_t occ_own = valid ? touch_search<LM>(A, i_own) : 0u;
+    const uint32_t nl_own = (uint32_t)__popc(occ_own);
+    const uint32_t incl = warp_inclusive(nl_own, lane);
+    const uint32_t excl = incl - nl_own;
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    Acc acc = zero_acc();
+    __syncwarp();   // the rows and tape rows written above are read and patched below
+    for (uint32_t base = 0; base < total; base += 32) {
+        const uint32_t f = base + lane;
+        // the sphere of contact f: the first lane whose inclusive count
+        // exceeds f
+        uint32_t o = 0;
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1) {
+            const uint32_t v = __shfl_sync(0xffffffffu, incl, (int)(o + (uint32_t)st - 1u));
+            if (v <= f) o += (uint32_t)st;
+        }
+        o = min(o, 31u);
+        uint32_t m = __shfl_sync(0xffffffffu, occ_own, (int)o);
+        const uint32_t e0 = __shfl_sync(0xffffffffu, excl, (int)o);
+        ContactRec r = no_rec();
+        if (f < total) {
+            for (uint32_t q = f - e0; q; --q) m &= m - 1u;
+            const int s = __ffs(m) - 1;
+            const uint32_t i = i0 + o;
+            const uint32_t w = A.slots[(size_t)i * NC + s];
+            if (!slot_contact<LM, MIXED, true>(A, i, s, w, r)) {
+                // the contact ended: its entry is no longer in the row
+                const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
+                const uint32_t vc = A.vcount[i];
+                uint32_t k = 0;
+                if (vc <= (uint32_t)VL_MAX)
+                    while (k < vc && lst[k] != (w & ID_MASK)) ++k;
+                if (k < vc && vc <= (uint32_t)VL_MAX) atomicAnd(&A.lmask[i], ~(1ull << k));
+                atomicAnd(&A.occ[i], ~(1u << s));
             }
         }
         put_rec(S, (int)threadIdx.x, r);
         __syncwarp();
-        // this lane's sphere: its entries of this round, in slot order
-        const uint32_t lo = max(excl, base), hi = min(incl, base + 32u);
-        for (uint32_t e = lo; e < hi; ++e) {
-            const ContactRec o = get_rec(S, wbase + (int)(e - base));
-            if (o.nev >= 0) replay(acc, o);
-        }
+        replay_round(acc, S, wbase, base, excl, incl);
         __syncwarp();
     }
     if (valid) A.csum[i_own] = acc;
@@ -1095,6 +1338,11 @@ inline void launch_interact_lm(const StepArgs &A, cudaStream_t st, unsigned grid
 template <bool MIXED>
 inline void launch_contacts(const StepArgs &A, cudaStream_t st, unsigned grid, int lm, bool pdl)
 {
+    if (A.touch) {
+        if (lm == SPH_LEN_FP64) launch_k(pdl, k_touch<SPH_LEN_FP64, MIXED>, grid, CONTACT_THREADS, st, A);
+        else launch_k(pdl, k_touch<SPH_LEN_REFERENCE, MIXED>, grid, CONTACT_THREADS, st, A);
+        return;
+    }
     if (lm == SPH_LEN_FP64) launch_k(pdl, k_contacts<SPH_LEN_FP64, MIXED>, grid, CONTACT_THREADS, st, A);
     else launch_k(pdl, k_contacts<SPH_LEN_REFERENCE, MIXED>, grid, CONTACT_THREADS, st, A);
 }
