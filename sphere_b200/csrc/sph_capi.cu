@@ -2447,10 +2447,11 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
     O.count = (uint32_t *)get(4 * (ncells + 1));
     O.coff = (uint32_t *)get(4 * (ncells + 1));
     O.items = (uint32_t *)get(4 * n);
+    O.xs = (double4 *)get(sizeof(double4) * n);
     O.npair = (uint32_t *)get(4 * (n + 1));
     O.poff = (uint32_t *)get(4 * (n + 1));
     uint32_t *scan_tmp = (uint32_t *)get(4 * (ncells / 4096 + n / 4096 + 2));
-    if (!O.cell_of || !O.slot || !O.count || !O.coff || !O.items || !O.npair || !O.poff ||
+    if (!O.cell_of || !O.slot || !O.count || !O.coff || !O.items || !O.xs || !O.npair || !O.poff ||
         !scan_tmp) {
         release();
         return fail(h, SPH_ERR_NOMEM, "overlap-search buffers");

@@ -167,6 +167,7 @@ struct OverlapArgs {
     double origo[3], cw[3];
     int num[3], R;
     uint32_t *cell_of, *slot, *count, *coff, *items, *npair, *poff;
+    double4 *xs;      // positions in cell order
     uint32_t *pairs;
     double *delta;
 };

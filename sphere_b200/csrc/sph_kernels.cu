@@ -554,87 +554,132 @@ int relax_sweeps(const StepArgs &A, cudaStream_t st, uint32_t sweeps, double alp
 
 // ---------------------------------------------------------------- analysis
 
-// src/sphere.cpp:487-606 DEM::porosity, one thread per slab: the slab
-// volume less the spheres' volumes inside it (with the reference's cap
-// terms), spheres in index order, so that every slab's sum is the
-// reference's, operation for operation.  All threads of a warp read the
-// same sphere at a time (broadcast).
-// One block per slab.  The slab's void volume is the reference's sequential
-// subtraction over the spheres in index order (one or two subtractions per
-// sphere that reaches into the slab, none otherwise); the threads compute
-// the terms of 256 spheres at a time and thread 0 applies them in index
-// order, skipping the spheres without a term (src/sphere.cpp:520-587).
-constexpr int POR_THREADS = 256;
+// src/sphere.cpp:487-606 DEM::porosity, one block per slab.  The slab's
+// void volume is the reference's sequential subtraction over the spheres in
+// index order (one or two subtractions per sphere that reaches into the
+// slab, none otherwise, src/sphere.cpp:520-587), so that the profile is the
+// reference's, operation for operation.  That chain of dependent
+// subtractions is the bound, and nothing else should lie on it: the producer
+// warps compute the terms of POR_TILE spheres at a time and pack them, in
+// index order, into one half of a shared buffer while one thread of the
+// consumer warp subtracts the other half from the sum.
+constexpr int POR_PRODUCERS = 512;
+constexpr int POR_TILE = 2 * POR_PRODUCERS;      // two consecutive spheres per producer
+constexpr int POR_THREADS = POR_PRODUCERS + 32;
+
+// The terms of a sphere at height zc with radius r in [z_low, z_high]; their
+// number (0 to 2).
+__device__ __forceinline__ int porosity_terms(double zc, double r, double z_low, double z_high,
+                                              double &t0, double &t1)
+{
+    const double zl = zc - r, zh = zc + r;
+    // every term below needs a bound of the slab in [zl, zh], or the sphere
+    // between the bounds
+    if (zh < z_low || zl > z_high) return 0;
+    const double V_s = 4.0 / 3.0 * M_PI * r * r * r;
+    if (z_low <= zl && zh <= z_high) {
+        t0 = V_s;
+        return 1;
+    }
+    int n = 0;
+    if (z_low >= zc && z_low <= zh) {
+        const double h = zh - z_low;
+        t0 = M_PI * h * h / 3.0 * (3.0 * r - h);
+        n = 1;
+    } else if (z_low < zc && z_low > zl) {
+        const double h = z_low - zl;
+        t0 = V_s + M_PI * h * h / 3.0 * (3.0 * r - h);
+        n = 1;
+    }
+    double tb = 0.0;
+    bool hb = false;
+    if (z_high <= zc && z_high >= zl) {
+        const double h = z_high - zl;
+        tb = M_PI * h * h / 3.0 * (3.0 * r - h);
+        hb = true;
+    } else if (z_high > zc && z_high < zh) {
+        const double h = zh - z_high;
+        tb = V_s + M_PI * h * h / 3.0 * (3.0 * r - h);
+        hb = true;
+    }
+    if (hb) {
+        if (n == 0) t0 = tb;
+        else t1 = tb;
+        ++n;
+    }
+    return n;
+}
 
 __global__ void __launch_bounds__(POR_THREADS) k_porosity(const double4 *x, uint32_t p0,
                                                           uint32_t np, double h_slice,
                                                           double V_slice, uint32_t nslices,
                                                           double *z_pos, double *por)
 {
-    __shared__ double s_t[2][POR_THREADS];
-    __shared__ int s_n[POR_THREADS];
-    __shared__ uint32_t s_mask[POR_THREADS / 32];
+    __shared__ double s_t[2][2 * POR_TILE];
+    __shared__ int s_n[2], s_warp[POR_PRODUCERS / 32];
     const uint32_t iz = blockIdx.x;
     const double z_low = (double)iz * h_slice;
     const double z_high = z_low + h_slice;
+    const uint32_t tiles = (np + POR_TILE - 1) / POR_TILE;
+    const bool producer = threadIdx.x < POR_PRODUCERS;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     double V_void = V_slice;
-    for (uint32_t base = 0; base < np; base += POR_THREADS) {
-        const uint32_t i = base + threadIdx.x;
-        int n = 0;
-        double t0 = 0.0, t1 = 0.0;
-        if (i < np) {
-            const double4 p = x[p0 + i];
-            const double zc = p.z, r = p.w;
-            const double zl = zc - r, zh = zc + r;
-            const double V_s = 4.0 / 3.0 * M_PI * r * r * r;
-            if (z_low <= zl && zh <= z_high) {
-                t0 = V_s;
-                n = 1;
-            } else {
-                if (z_low >= zc && z_low <= zh) {
-                    const double h = zh - z_low;
-                    t0 = M_PI * h * h / 3.0 * (3.0 * r - h);
-                    n = 1;
-                } else if (z_low < zc && z_low > zl) {
-                    const double h = z_low - zl;
-                    t0 = V_s + M_PI * h * h / 3.0 * (3.0 * r - h);
-                    n = 1;
-                }
-                double tb = 0.0;
-                bool hb = false;
-                if (z_high <= zc && z_high >= zl) {
-                    const double h = z_high - zl;
-                    tb = M_PI * h * h / 3.0 * (3.0 * r - h);
-                    hb = true;
-                } else if (z_high > zc && z_high < zh) {
-                    const double h = zh - z_high;
-                    tb = V_s + M_PI * h * h / 3.0 * (3.0 * r - h);
-                    hb = true;
-                }
-                if (hb) {
-                    if (n == 0) t0 = tb;
-                    else t1 = tb;
-                    ++n;
-                }
+    // height and radius of the producer's two spheres of the next tile,
+    // loaded one tile ahead
+    double2 q[2];
+    auto load = [&](uint32_t tile) {
+        const uint32_t i = tile * POR_TILE + 2u * threadIdx.x;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            q[j] = i + j < np ? reinterpret_cast<const double2 *>(x + p0 + i + j)[1] : make_double2(0.0, 0.0);
+    };
+    if (producer && tiles) load(0);
+    for (uint32_t tile = 0; tile <= tiles; ++tile) {
+        if (producer && tile < tiles) {
+            const uint32_t i = tile * POR_TILE + 2u * threadIdx.x;
+            double t[4];
+            int n0 = 0, n1 = 0;
+            if (i < np) n0 = porosity_terms(q[0].x, q[0].y, z_low, z_high, t[0], t[1]);
+            if (i + 1 < np) n1 = porosity_terms(q[1].x, q[1].y, z_low, z_high, t[2], t[3]);
+            if (tile + 1 < tiles) load(tile + 1);
+            int incl = n0 + n1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += v;
             }
+            if (lane == 31) s_warp[warp] = incl;
+            asm volatile("bar.sync 1, %0;" ::"n"(POR_PRODUCERS) : "memory");
+            int at = incl - n0 - n1, total = 0;
+#pragma unroll
+            for (int w = 0; w < POR_PRODUCERS / 32; ++w) {
+                const int v = s_warp[w];
+                if (w < (int)warp) at += v;
+                total += v;
+            }
+            double *out = s_t[tile & 1u];
+            if (n0 > 0) out[at++] = t[0];
+            if (n0 > 1) out[at++] = t[1];
+            if (n1 > 0) out[at++] = t[2];
+            if (n1 > 1) out[at++] = t[3];
+            if (threadIdx.x == 0) s_n[tile & 1u] = total;
         }
-        s_t[0][threadIdx.x] = t0;
-        s_t[1][threadIdx.x] = t1;
-        s_n[threadIdx.x] = n;
-        const uint32_t m = __ballot_sync(0xffffffffu, n > 0);
-        if ((threadIdx.x & 31) == 0) s_mask[threadIdx.x >> 5] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 0; w < POR_THREADS / 32; ++w)
-                for (uint32_t b = s_mask[w]; b; b &= b - 1u) {
-                    const int t = w * 32 + __ffs(b) - 1;
-                    V_void -= s_t[0][t];
-                    if (s_n[t] > 1) V_void -= s_t[1][t];
-                }
+        if (threadIdx.x == POR_PRODUCERS && tile > 0) {
+            const double *in = s_t[(tile - 1) & 1u];
+            const int n = s_n[(tile - 1) & 1u];
+            int k = 0;
+            for (; k + 16 <= n; k += 16) {
+                double v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = in[k + j];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) V_void -= v[j];
+            }
+            for (; k < n; ++k) V_void -= in[k];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0 && iz < nslices) {
+    if (threadIdx.x == POR_PRODUCERS && iz < nslices) {
         z_pos[iz] = z_low + 0.5 * h_slice;
         por[iz] = V_void / V_slice;
     }
@@ -679,55 +724,65 @@ __global__ void k_ov_scatter(OverlapArgs O)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= O.np) return;
-    O.items[O.coff[O.cell_of[i]] + O.slot[i]] = i;
+    const uint32_t q = O.coff[O.cell_of[i]] + O.slot[i];
+    O.items[q] = i;
+    O.xs[q] = O.x[O.p0 + i];
 }
 
-// WRITE = false: count the pairs of sphere i; true: write them sorted by j.
+// One thread per sphere in cell order (its candidates are then its warp's
+// too); WRITE = false: count the pairs of sphere i; true: write them sorted
+// by j.  The cells of a row are neighbours in the cell order, so each row of
+// the search block is one range.  Most candidates are far apart: the squared
+// distance against a bound just above (ri + rj)^2 drops those before the
+// square root, and never drops an overlapping pair (the root and the sum
+// each round by less than 2^-52).
 template <bool WRITE>
 __global__ void k_ov_pairs(OverlapArgs O)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= O.np) return;
-    const double4 xi = O.x[O.p0 + i];
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= O.np) return;
+    const uint32_t i = O.items[p];
+    const double4 xi = O.xs[p];
+    const uint32_t cnt = WRITE ? O.npair[i] : 0u;
+    if (WRITE && cnt == 0u) return;
     const bool free_i = O.vel[O.p0 + i].w == 0.0;
     int c[3];
     ov_cell(O, xi, c);
     uint32_t n = 0;
     const uint32_t base = WRITE ? O.poff[i] : 0u;
-    const uint32_t cnt = WRITE ? O.npair[i] : 0u;
-    for (int dz = -O.R; dz <= O.R; ++dz)
-        for (int dy = -O.R; dy <= O.R; ++dy)
-            for (int dx = -O.R; dx <= O.R; ++dx) {
-                const int tx = c[0] + dx, ty = c[1] + dy, tz = c[2] + dz;
-                if (tx < 0 || ty < 0 || tz < 0 || tx >= O.num[0] || ty >= O.num[1] ||
-                    tz >= O.num[2])
-                    continue;
-                const uint32_t cell = (uint32_t)((tz * O.num[1] + ty) * O.num[0] + tx);
-                for (uint32_t q = O.coff[cell]; q < O.coff[cell + 1]; ++q) {
-                    const uint32_t j = O.items[q];
-                    if (j <= i) continue;
-                    const double4 xj = O.x[O.p0 + j];
-                    const double ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
-                    const double len = sqrt(ddx * ddx + ddy * ddy + ddz * ddz);
-                    const double d = len - (xi.w + xj.w);
-                    if (!(d < 0.0 && free_i && O.vel[O.p0 + j].w == 0.0)) continue;
-                    if (WRITE && n < cnt) {
-                        // insertion by j into this sphere's part of the list
-                        uint32_t k = n;
-                        while (k > 0 && O.pairs[2 * (size_t)(base + k - 1) + 1] > j) {
-                            O.pairs[2 * (size_t)(base + k)] = O.pairs[2 * (size_t)(base + k - 1)];
-                            O.pairs[2 * (size_t)(base + k) + 1] =
-                                O.pairs[2 * (size_t)(base + k - 1) + 1];
-                            O.delta[base + k] = O.delta[base + k - 1];
-                            --k;
-                        }
-                        O.pairs[2 * (size_t)(base + k)] = i;
-                        O.pairs[2 * (size_t)(base + k) + 1] = j;
-                        O.delta[base + k] = d;
+    const int x0 = max(c[0] - O.R, 0), x1 = min(c[0] + O.R, O.num[0] - 1);
+    for (int dz = -O.R; dz <= O.R && free_i; ++dz)
+        for (int dy = -O.R; dy <= O.R; ++dy) {
+            const int ty = c[1] + dy, tz = c[2] + dz;
+            if (ty < 0 || tz < 0 || ty >= O.num[1] || tz >= O.num[2]) continue;
+            const uint32_t row = (uint32_t)((tz * O.num[1] + ty) * O.num[0]);
+            const uint32_t q1 = O.coff[row + (uint32_t)x1 + 1u];
+            for (uint32_t q = O.coff[row + (uint32_t)x0]; q < q1; ++q) {
+                const double4 xj = O.xs[q];
+                const double ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
+                const double d2 = ddx * ddx + ddy * ddy + ddz * ddz, rr = xi.w + xj.w;
+                if (d2 > rr * rr * (1.0 + 1e-12)) continue;
+                const uint32_t j = O.items[q];
+                if (j <= i) continue;
+                const double len = sqrt(d2);
+                const double d = len - rr;
+                if (!(d < 0.0 && O.vel[O.p0 + j].w == 0.0)) continue;
+                if (WRITE && n < cnt) {
+                    // insertion by j into this sphere's part of the list
+                    uint32_t k = n;
+                    while (k > 0 && O.pairs[2 * (size_t)(base + k - 1) + 1] > j) {
+                        O.pairs[2 * (size_t)(base + k)] = O.pairs[2 * (size_t)(base + k - 1)];
+                        O.pairs[2 * (size_t)(base + k) + 1] = O.pairs[2 * (size_t)(base + k - 1) + 1];
+                        O.delta[base + k] = O.delta[base + k - 1];
+                        --k;
                     }
-                    ++n;
+                    O.pairs[2 * (size_t)(base + k)] = i;
+                    O.pairs[2 * (size_t)(base + k) + 1] = j;
+                    O.delta[base + k] = d;
                 }
+                ++n;
             }
+        }
     if (!WRITE) O.npair[i] = n;
 }
 
