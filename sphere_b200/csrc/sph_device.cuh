@@ -78,7 +78,39 @@ __device__ __forceinline__ d3 vsub(d3 a, d3 b) { return mk(a.x - b.x, a.y - b.y,
 __device__ __forceinline__ d3 vadds(d3 a, double b) { return mk(a.x + b, a.y + b, a.z + b); }
 __device__ __forceinline__ d3 smul(double s, d3 a) { return mk(s * a.x, s * a.y, s * a.z); }
 __device__ __forceinline__ d3 muls(d3 a, double s) { return mk(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ d3 divs(d3 a, double s) { return mk(a.x / s, a.y / s, a.z / s); }
+
+// Several correctly rounded quotients by one divisor b, by Markstein's
+// correction (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990) from
+// r = RN(1 / b): q0 = RN(a r) lies within one ulp of a / b, the remainder
+// a - b q0 is exact (one FMA), and RN(q0 + r * remainder) is the quotient,
+// while a, r and q0 lie away from the ends of the range.  A zero a with a
+// finite r gives q0 = +-0, the quotient with its sign; every other operand
+// takes the division itself.  A multiply and two FMAs for each quotient
+// after the first division, instead of a division sequence (about ten FP64
+// instructions and a branch).
+struct Divisor {
+    double b, r;
+    bool ok;
+    __device__ __forceinline__ explicit Divisor(double b_) : b(b_), r(1.0 / b_)
+    {
+        ok = fabs(r) > 0x1p-1000 && fabs(r) < 0x1p+1000;
+    }
+    __device__ __forceinline__ double div(double a) const
+    {
+        const double q0 = __dmul_rn(a, r);
+        const double aq = fabs(q0);
+        if (ok && aq > 0x1p-900 && aq < 0x1p+1000 && fabs(a) > 0x1p-900)
+            return __fma_rn(__fma_rn(-q0, b, a), r, q0);
+        if (ok && a == 0.0) return q0;
+        return a / b;
+    }
+};
+__device__ __forceinline__ d3 divs(d3 a, double s)
+{
+    const Divisor q(s);
+    return mk(q.div(a.x), q.div(a.y), q.div(a.z));
+}
 __device__ __forceinline__ d3 vneg(d3 a) { return mk(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ double dot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ d3 cross(d3 a, d3 b)

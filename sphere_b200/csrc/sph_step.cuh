@@ -84,12 +84,14 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     const double radius = x.w;
     const double m = 4.0 / 3.0 * PI * radius * radius * radius * P.rho;
     double acc[3], angacc[3];
-    acc[0] = F.x / m + P.g[0];
-    acc[1] = F.y / m + P.g[1];
-    acc[2] = F.z / m + P.g[2];
-    angacc[0] = T.x * 1.0 / (2.0 / 5.0 * m * radius * radius);
-    angacc[1] = T.y * 1.0 / (2.0 / 5.0 * m * radius * radius);
-    angacc[2] = T.z * 1.0 / (2.0 / 5.0 * m * radius * radius);
+    // (twelve quotients by three divisors)
+    const Divisor by_m(m), by_i(2.0 / 5.0 * m * radius * radius), by_dt(dt);
+    acc[0] = by_m.div(F.x) + P.g[0];
+    acc[1] = by_m.div(F.y) + P.g[1];
+    acc[2] = by_m.div(F.z) + P.g[2];
+    angacc[0] = by_i.div(T.x * 1.0);
+    angacc[1] = by_i.div(T.y * 1.0);
+    angacc[2] = by_i.div(T.z * 1.0);
     double angacc_w = 0.0;
     if (wall0mode == 3 && vel.w > 0.0001 && x.z > B.L[2] * 0.5) {
         const double f_tau_x = (B.tau_x + B.tau_eff_x) * B.L[0] * B.L[1];
@@ -123,8 +125,8 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     double xn[3], vn[3], pn[3], wn[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double dacc = (acc[d] - a0[d]) / dt;
-        const double dangacc = (angacc[d] - w0[d]) / dt;
+        const double dacc = by_dt.div(acc[d] - a0[d]);
+        const double dangacc = by_dt.div(angacc[d] - w0[d]);
         xn[d] = xv[d] + vv[d] * dt + 0.5 * acc[d] * dt * dt + 1.0 / 6.0 * dacc * dt * dt * dt;
         vn[d] = vv[d] + acc[d] * dt + 0.5 * dacc * dt * dt;
         pn[d] = pv[d] + wv[d] * dt + 0.5 * angacc[d] * dt * dt + 1.0 / 6.0 * dangacc * dt * dt * dt;
