@@ -260,6 +260,7 @@ static void invalidate_pair(SphHandle *h)
 static StepConfig step_config(const SphHandle *h)
 {
     StepConfig cfg = h->cfg;
+    cfg.box0 = h->nbox == 1 ? &h->dbox[0] : nullptr;
     cfg.lazy_sort = h->uploaded && !pair_active(h) && sph::split_active(h->A, cfg);
     cfg.touch = true;
     for (uint32_t k = 0; k < h->nbox; ++k) {

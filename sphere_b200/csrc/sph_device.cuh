@@ -68,6 +68,36 @@ struct DevBox {
     int32_t change_velocity_state;
 };
 
+// What a run never changes of a box (L[2] of an adaptive grid excepted: it is
+// read from the box).  Kernels of one-box handles take it as an argument, in
+// the constant bank, where an instruction reads it as an operand; from the
+// box table in memory every use after a store is a load of its own, since the
+// store might have changed it.
+struct BoxConst {
+    SphParams P;
+    double origo[3], L[3];
+    double dt;
+    uint32_t num[3];
+    int32_t periodic;
+    uint32_t nw;
+    uint32_t cell_base;
+};
+inline BoxConst box_const(const DevBox &B)
+{
+    BoxConst c;
+    c.P = B.P;
+    for (int k = 0; k < 3; ++k) {
+        c.origo[k] = B.origo[k];
+        c.L[k] = B.L[k];
+        c.num[k] = B.num[k];
+    }
+    c.dt = B.dt;
+    c.periodic = B.periodic;
+    c.nw = B.nw;
+    c.cell_base = B.cell_base;
+    return c;
+}
+
 struct d3 {
     double x, y, z;
 };
@@ -261,7 +291,8 @@ __device__ __forceinline__ bool relative_cell(const DevBox &B, const int g[3], i
 }
 
 // Image shift vector exactly as findDistMod accumulates it from zero.
-__device__ __forceinline__ d3 shift_vec(const DevBox &B, int sx, int sy)
+template <class BX>
+__device__ __forceinline__ d3 shift_vec(const BX &B, int sx, int sy)
 {
     const double dx = sx == 0 ? 0.0 : (sx > 0 ? B.L[0] : -B.L[0]);
     const double dy = sy == 0 ? 0.0 : (sy > 0 ? B.L[1] : -B.L[1]);

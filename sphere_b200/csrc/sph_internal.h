@@ -240,6 +240,10 @@ struct StepConfig {
     cudaStream_t side = nullptr;                       // STEP_OVERLAP only
     cudaEvent_t fork = nullptr, join = nullptr;        // STEP_OVERLAP only
     const DarcyArgs *darcy = nullptr;                  // the Darcy coupling, null: off
+    // the box of a one-box handle as uploaded: the kernels of the list and
+    // split step then take what never changes in it (parameters, grid,
+    // time step) from their arguments (BoxConst)
+    const DevBox *box0 = nullptr;
 };
 
 // Whether a step with these settings runs as the split step.
@@ -274,8 +278,8 @@ typedef void (*InteractLauncher)(const StepArgs &A, cudaStream_t st, unsigned gr
                                  int lenmode, int variant);
 int launch_step(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, uint64_t *launches,
                 Prof *prof = nullptr);
-typedef void (*ContactLauncher)(const StepArgs &A, cudaStream_t st, unsigned grid, int lenmode,
-                                bool pdl);
+typedef void (*ContactLauncher)(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
+                                unsigned grid, bool pdl);
 
 // Launch kern<<<grid, block, 0, st>>>(args...); with pdl, as a programmatic
 // dependent launch: the grid may be scheduled while the kernel before it

@@ -266,7 +266,7 @@ __global__ void k_integrate(StepArgs A)
     const uint32_t i = A.perm[a];
     const DevBox &B = A.boxes[A.box_of[i]];
     const double4 f = A.force[i], t = A.torque[i];
-    integrate_particle(A, B, i, A.xs[a], A.vs[a], A.ws[a], xyz(f), xyz(t));
+    integrate_particle(A, B, B, i, A.xs[a], A.vs[a], A.ws[a], xyz(f), xyz(t));
 }
 
 // integration.cuh:457-484 findShearStressOnFixedMovingParticles
@@ -406,10 +406,14 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
 // neighbours in the cell order, so away from the grid's x edges a row is
 // one range of candidates.
 constexpr int RELAX_THREADS = 128;
-constexpr int RELAX_BATCH = 8;
+#ifndef RB
+#define RB 8
+#define RM 4
+#endif
+constexpr int RELAX_BATCH = RB;
 constexpr int RELAX_NOTES = 24;
 
-__global__ void __launch_bounds__(RELAX_THREADS, 4) k_relax(StepArgs A, double alpha, double z_top,
+__global__ void __launch_bounds__(RELAX_THREADS, RM) k_relax(StepArgs A, double alpha, double z_top,
                                                             unsigned long long *max_ov, bool next)
 {
     __shared__ unsigned long long s_max[RELAX_THREADS / 32];
@@ -432,6 +436,7 @@ __global__ void __launch_bounds__(RELAX_THREADS, 4) k_relax(StepArgs A, double a
             const uint32_t w = s_note[k][threadIdx.x];
             int sx, sy;
             decode_shift(w >> CODE_SHIFT, sx, sy);
+            if ((w & ID_MASK) == a) continue;   // the sphere itself
             const d3 dm = shift_vec(B, sx, sy);
             const double4 xb = A.xs[w & ID_MASK];
             const double rx = xa.x - xb.x + dm.x, ry = xa.y - xb.y + dm.y, rz = xa.z - xb.z + dm.z;
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(RELAX_THREADS, 4) k_relax(StepArgs A, double a
             if (noted + RELAX_BATCH > RELAX_NOTES) push_apart();
 #pragma unroll
             for (int j = 0; j < RELAX_BATCH; ++j)
-                if (b + j < b1 && b + j != a && maybe_touching(xaf, xf[j], fsx, fsy, margin))
+                if (b + j < b1 && maybe_touching(xaf, xf[j], fsx, fsy, margin))
                     s_note[noted++][threadIdx.x] = (b + j) | code;
         }
     };
@@ -857,9 +862,10 @@ static void interact_fp64(const StepArgs &A, cudaStream_t st, unsigned grid, boo
     launch_interact<false>(A, st, grid, fused, lm, variant);
 }
 
-static void contacts_fp64(const StepArgs &A, cudaStream_t st, unsigned grid, int lm, bool pdl)
+static void contacts_fp64(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, unsigned grid,
+                          bool pdl)
 {
-    launch_contacts<false>(A, st, grid, lm, pdl);
+    launch_contacts<false>(A, cfg, st, grid, pdl);
 }
 
 // The cell counts and each sphere's place in its cell from the cell ids.
@@ -984,13 +990,19 @@ int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t s
                 mark(prof, st, "k_search");
                 nl += 1;
             }
-            contact(A, st, blocks_for(A.ntot, CONTACT_THREADS), cfg.lenmode, A.touch ? pdl_s : pdl);
+            contact(A, cfg, st, blocks_for(A.ntot, CONTACT_THREADS), A.touch ? pdl_s : pdl);
             mark(prof, st, A.touch ? "k_touch" : "k_contacts");
             if (overlap) cudaStreamWaitEvent(st, cfg.join, 0);
-            if (cfg.lenmode == SPH_LEN_FP64)
-                k_finish<SPH_LEN_FP64><<<blocks_for(A.ntot, FINISH_THREADS), FINISH_THREADS, 0, st>>>(A);
-            else
-                k_finish<SPH_LEN_REFERENCE><<<blocks_for(A.ntot, FINISH_THREADS), FINISH_THREADS, 0, st>>>(A);
+            const unsigned gf = blocks_for(A.ntot, FINISH_THREADS);
+            const bool lm64 = cfg.lenmode == SPH_LEN_FP64;
+            if (cfg.box0) {
+                const BoxConst C = box_const(*cfg.box0);
+                if (lm64) k_finish1<SPH_LEN_FP64><<<gf, FINISH_THREADS, 0, st>>>(A, C);
+                else k_finish1<SPH_LEN_REFERENCE><<<gf, FINISH_THREADS, 0, st>>>(A, C);
+            } else {
+                if (lm64) k_finish<SPH_LEN_FP64><<<gf, FINISH_THREADS, 0, st>>>(A);
+                else k_finish<SPH_LEN_REFERENCE><<<gf, FINISH_THREADS, 0, st>>>(A);
+            }
             mark(prof, st, "k_finish");
             nl += 2;
         } else if (!cfg.unfused) {

@@ -16,9 +16,10 @@ static void interact_mixed(const StepArgs &A, cudaStream_t st, unsigned grid, bo
     launch_interact<true>(A, st, grid, fused, lm, variant);
 }
 
-static void contacts_mixed(const StepArgs &A, cudaStream_t st, unsigned grid, int lm, bool pdl)
+static void contacts_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, unsigned grid,
+                           bool pdl)
 {
-    launch_contacts<true>(A, st, grid, lm, pdl);
+    launch_contacts<true>(A, cfg, st, grid, pdl);
 }
 
 int launch_step_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,

@@ -85,9 +85,33 @@ __device__ __forceinline__ void mixed_stiffness(const SphParams &P, float ra, fl
     }
 }
 
+// The contact parameters rounded to FP32 once, under the names of SphParams
+// (the laws round them where they use them, to the same values).
+struct MixedParams {
+    float k_n, k_t, E, gamma_n, gamma_t, gamma_r, mu_s, mu_d, mu_r, kappa;
+    int32_t use_E;          // E > .001 in FP64
+    uint32_t contactmodel;
+};
+inline MixedParams mixed_params(const SphParams &P)
+{
+    return MixedParams{(float)P.k_n,     (float)P.k_t,  (float)P.E,    (float)P.gamma_n,
+                       (float)P.gamma_t, (float)P.gamma_r, (float)P.mu_s, (float)P.mu_d,
+                       (float)P.mu_r,    (float)P.kappa, P.E > .001 ? 1 : 0, P.contactmodel};
+}
+__device__ __forceinline__ void mixed_stiffness(const MixedParams &P, float ra, float rb, float &k_n,
+                                                float &k_t)
+{
+    k_n = P.k_n;
+    k_t = P.k_t;
+    if (P.use_E) {
+        k_n = 3.141592654f / 2.0f * P.E * (ra + rb) / 2.f;
+        k_t = k_n;
+    }
+}
+
 // contactLinear (contact model 2), contactmodels.cuh:244-411
-template <class AccT>
-__device__ __forceinline__ d3 contact_linear_mixed(const SphParams &P, double dt, AccT &a,
+template <class PT, class AccT>
+__device__ __forceinline__ d3 contact_linear_mixed(const PT &P, double dt, AccT &a,
                                                    const MixedPair &q, d3 delta_t0_uncor)
 {
     const f3 n = q.n;
@@ -134,8 +158,8 @@ __device__ __forceinline__ d3 contact_linear_mixed(const SphParams &P, double dt
 
 // contactHertz (contact model 3) with the overlap-magnitude powers of the
 // FP64 form, contactmodels.cuh:417-600
-template <class AccT>
-__device__ __forceinline__ d3 contact_hertz_mixed(const SphParams &P, double dt, AccT &a,
+template <class PT, class AccT>
+__device__ __forceinline__ d3 contact_hertz_mixed(const PT &P, double dt, AccT &a,
                                                   const MixedPair &q, d3 delta_t0_uncor)
 {
     const f3 n = q.n;

@@ -64,7 +64,8 @@ inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 
 // uses (the nearest one: along a periodic axis a difference over half the
 // box is shifted by -+L), rounded as the FP64 form's (xa - xb) + shift;
 // code: the image code of a slot word (shift_code).
-__device__ __forceinline__ d3 centre_line(const DevBox &B, const double4 &xa, const double4 &xb,
+template <class BX>
+__device__ __forceinline__ d3 centre_line(const BX &B, const double4 &xa, const double4 &xb,
                                           uint32_t *code)
 {
     double dx = __dsub_rn(xa.x, xb.x), dy = __dsub_rn(xa.y, xb.y);
@@ -141,13 +142,13 @@ __device__ __forceinline__ MixedPair mixed_pair_f(d3 x_ab, double x_length, doub
 // of the list step: wall w is the box's wall w when w < nw, else the
 // default plane (top at L[2], sides at 0 and L); the normal force on wall 0
 // is returned.  Reads each wall from the box table where it is used.
-template <int LM>
-__device__ __forceinline__ double walls_pair(const DevBox &B, double4 xa, d3 vel_a, d3 angvel_a,
+template <int LM, class BX>
+__device__ __forceinline__ double walls_pair(const DevBox &B, const BX &C, double4 xa, d3 vel_a, d3 angvel_a,
                                              MixedAcc &acc)
 {
-    const SphParams &Pm = B.P;
-    const double dt = B.dt, r = xa.w;
-    const uint32_t nw = B.nw;
+    const SphParams &Pm = C.P;
+    const double dt = C.dt, r = xa.w;
+    const uint32_t nw = C.nw;
     auto plane = [&](uint32_t w, double dx, double dy, double dz, double dpos, d3 &n, double &pos,
                      double &vel) {
         if (w < nw) {
@@ -165,19 +166,19 @@ __device__ __forceinline__ double walls_pair(const DevBox &B, double4 xa, d3 vel
     plane(0, 0.0, 0.0, -1.0, B.L[2], n, pos, wv);
     double delta_w = pos - (xa.z + r);
     if (delta_w < 0.0) w0_force = contact_linear_wall<LM>(Pm, dt, acc, vel_a, angvel_a, r, n, delta_w, wv);
-    delta_w = xa.z - r - B.origo[2];
+    delta_w = xa.z - r - C.origo[2];
     if (delta_w < 0.0)
         (void)contact_linear_wall<LM>(Pm, dt, acc, vel_a, angvel_a, r, mk(0.0, 0.0, 1.0), delta_w, 0.0);
-    if (B.periodic == 0) {
-        plane(1, -1.0, 0.0, 0.0, B.L[0], n, pos, wv);
+    if (C.periodic == 0) {
+        plane(1, -1.0, 0.0, 0.0, C.L[0], n, pos, wv);
         delta_w = pos - (xa.x + r);
         if (delta_w < 0.0) (void)contact_linear_wall<LM>(Pm, dt, acc, vel_a, angvel_a, r, n, delta_w, wv);
         plane(2, 1.0, 0.0, 0.0, 0.0, n, pos, wv);
         delta_w = xa.x - r - pos;
         if (delta_w < 0.0) (void)contact_linear_wall<LM>(Pm, dt, acc, vel_a, angvel_a, r, n, delta_w, wv);
     }
-    if (B.periodic == 0 || B.periodic == 2) {
-        plane(3, 0.0, -1.0, 0.0, B.L[1], n, pos, wv);
+    if (C.periodic == 0 || C.periodic == 2) {
+        plane(3, 0.0, -1.0, 0.0, C.L[1], n, pos, wv);
         delta_w = pos - (xa.y + r);
         if (delta_w < 0.0) (void)contact_linear_wall<LM>(Pm, dt, acc, vel_a, angvel_a, r, n, delta_w, wv);
         plane(4, 0.0, 1.0, 0.0, 0.0, n, pos, wv);
@@ -190,12 +191,13 @@ __device__ __forceinline__ double walls_pair(const DevBox &B, double4 xa, d3 vel
 // integration.cuh:14-305 (TY3) for one sphere of the list step: FP64
 // arithmetic on the compact state; the new state goes to the [nxt] half of
 // the ping-pong arrays and to the sphere's own arrays.
+template <class BX>
 __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs &P,
-                                               const DevBox &B, uint32_t i, uint32_t nxt,
+                                               const DevBox &B, const BX &C, uint32_t i, uint32_t nxt,
                                                double4 x, double4 vel, float4 wf, d3 F, d3 T)
 {
-    const SphParams &Pm = B.P;
-    const double dt = B.dt;
+    const SphParams &Pm = C.P;
+    const double dt = C.dt;
     const float4 apf = P.angpos[i];
     double4 xyzsum = P.xyzsum[i];
     double a0[3] = {0.0, 0.0, 0.0}, w0[3] = {0.0, 0.0, 0.0};
@@ -248,14 +250,14 @@ __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs
         wn[d] = wv[d] + angacc[d] * dt + 0.5 * dangacc * dt * dt;
         sv[d] += dx;
     }
-    if (B.periodic == 1) {
-        if (xn[0] < B.origo[0]) xn[0] += B.L[0];
-        if (xn[0] > B.L[0]) xn[0] -= B.L[0];
-        if (xn[1] < B.origo[1]) xn[1] += B.L[1];
-        if (xn[1] > B.L[1]) xn[1] -= B.L[1];
-    } else if (B.periodic == 2) {
-        if (xn[0] < B.origo[0]) xn[0] += B.L[0];
-        if (xn[0] > B.L[0]) xn[0] -= B.L[0];
+    if (C.periodic == 1) {
+        if (xn[0] < C.origo[0]) xn[0] += C.L[0];
+        if (xn[0] > C.L[0]) xn[0] -= C.L[0];
+        if (xn[1] < C.origo[1]) xn[1] += C.L[1];
+        if (xn[1] > C.L[1]) xn[1] -= C.L[1];
+    } else if (C.periodic == 2) {
+        if (xn[0] < C.origo[0]) xn[0] += C.L[0];
+        if (xn[0] > C.L[0]) xn[0] -= C.L[0];
     }
     {
         // neighbour-list validity: displacement since the list build
@@ -263,13 +265,13 @@ __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs
         const float4 r = A.xref[i];
         float ex = (float)xn[0] - r.x, ey = (float)xn[1] - r.y;
         const float ez = (float)xn[2] - r.z;
-        if (B.periodic == 1 || B.periodic == 2) {
-            const float lx = (float)B.L[0];
+        if (C.periodic == 1 || C.periodic == 2) {
+            const float lx = (float)C.L[0];
             if (ex > 0.5f * lx) ex -= lx;
             else if (ex < -0.5f * lx) ex += lx;
         }
-        if (B.periodic == 1) {
-            const float ly = (float)B.L[1];
+        if (C.periodic == 1) {
+            const float ly = (float)C.L[1];
             if (ey > 0.5f * ly) ey -= ly;
             else if (ey < -0.5f * ly) ey += ly;
         }
@@ -290,25 +292,25 @@ __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs
 }
 
 // After a sphere's contacts: its touching bits, walls, sums and integration.
-template <int LM>
+template <int LM, class BX>
 __device__ __forceinline__ void finish_sphere(const StepArgs &A, const PairArgs &P,
-                                              const DevBox &B, uint32_t i, uint32_t nxt,
+                                              const DevBox &B, const BX &C, uint32_t i, uint32_t nxt,
                                               uint32_t ls, double4 xa, float4 wa, MixedAcc &acc,
                                               unsigned long long live_old,
                                               unsigned long long live_new)
 {
-    const double dt = B.dt;
+    const double dt = C.dt;
     if (__popcll(live_new) > NC) raise_flag(A.err, SPH_ERR_NC_OVERFLOW);
     if (live_new != live_old) P.live[ls][i] = live_new;
     const double4 vel = P.vel[i];
-    const double w0_force = walls_pair<LM>(B, xa, xyz(vel), mk(wa.x, wa.y, wa.z), acc);
+    const double w0_force = walls_pair<LM>(B, C, xa, xyz(vel), mk(wa.x, wa.y, wa.z), acc);
     P.force[i] = make_float4((float)acc.F.x, (float)acc.F.y, (float)acc.F.z, 0.f);
     P.torque[i] = make_float4((float)acc.T.x, (float)acc.T.y, (float)acc.T.z, 0.f);
     P.epp[i] = make_float4(acc.es_dot, acc.ev_dot, acc.p, 0.f);
     const double2 e0 = P.eacc[i];
     P.eacc[i] = make_double2(e0.x + (double)acc.es_dot * dt, e0.y + (double)acc.ev_dot * dt);
-    if (B.nw > 0) A.wf_pp[i] = w0_force;
-    integrate_pair(A, P, B, i, nxt, xa, vel, wa, acc.F, acc.T);
+    if (C.nw > 0) A.wf_pp[i] = w0_force;
+    integrate_pair(A, P, B, C, i, nxt, xa, vel, wa, acc.F, acc.T);
 }
 
 // One sphere of the list step (thread slot t of the ordering): its list
@@ -319,14 +321,15 @@ __device__ __forceinline__ void finish_sphere(const StepArgs &A, const PairArgs 
 // the current entry is computed (more loads in flight per thread, about 20
 // more registers); without it each entry is loaded at its turn and the
 // latency is hidden by more resident warps.  Both give the same bits.
-template <int LM, bool AHEAD = true>
-__device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P, uint32_t t,
-                                            uint32_t cur, uint32_t nxt, uint32_t ls)
+// C, M: the box's constants and its contact parameters (the box itself and
+// its P, or those of a one-box launch's arguments).
+template <int LM, bool AHEAD, class BX, class PT>
+__device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P, const DevBox &B,
+                                            const BX &C, const PT &M, uint32_t i, uint32_t cur,
+                                            uint32_t nxt, uint32_t ls)
 {
-    const uint32_t i = P.order[ls][t];
     const double4 *__restrict__ xr = P.xr[cur];
     const float4 *__restrict__ vw = P.vw[cur];
-    const DevBox &B = A.boxes[box_index(A, i)];
     uint32_t n = P.cnt[ls][i];
     if (n > (uint32_t)VL_MAX) {   // the list overflowed at its build
         raise_flag(A.err, SPH_ERR_NC_OVERFLOW);
@@ -337,7 +340,7 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
     const ListRow L(P, ls, i);
     const double4 xa = xr[i];
     const float4 va = vw[2 * i], wa = vw[2 * i + 1];
-    const double dt = B.dt;
+    const double dt = C.dt;
 
     MixedAcc acc;
     acc.F = mk(0.0, 0.0, 0.0);
@@ -365,7 +368,7 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
                 wb = vw[2 * b + 1];
                 hb = L.hist3(k);
             }
-            const d3 x_ab = centre_line(B, xa, xb, nullptr);
+            const d3 x_ab = centre_line(C, xa, xb, nullptr);
             const double x_ab_length = len_rn<LM>(x_ab);
             const double delta_n = __dsub_rn(x_ab_length, __dadd_rn(xa.w, xb.w));
             if (delta_n < 0.0) {
@@ -374,13 +377,13 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
                     wb = vw[2 * b + 1];
                 }
                 const MixedPair q = mixed_pair_f(x_ab, x_ab_length, delta_n, va, vb, wa, wb, xa.w, xb.w);
-                const d3 nd = B.P.contactmodel == 2 ? contact_linear_mixed(B.P, dt, acc, q, hb)
-                                                    : contact_hertz_mixed(B.P, dt, acc, q, hb);
+                const d3 nd = M.contactmodel == 2 ? contact_linear_mixed(M, dt, acc, q, hb)
+                                                    : contact_hertz_mixed(M, dt, acc, q, hb);
                 L.put3(k, nd);
                 live_new |= 1ull << k;
             }
         }
-        finish_sphere<LM>(A, P, B, i, nxt, ls, xa, wa, acc, live_old, live_new);
+        finish_sphere<LM>(A, P, B, C, i, nxt, ls, xa, wa, acc, live_old, live_new);
         return;
     }
     // entry k's partner state and history are loaded during entry k - 1,
@@ -410,13 +413,13 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
             if ((live_old >> (k + 1)) & 1ull)
                 hq = L.hist3(k + 1);
         }
-        const d3 x_ab = centre_line(B, xa, xb, nullptr);
+        const d3 x_ab = centre_line(C, xa, xb, nullptr);
         const double x_ab_length = len_rn<LM>(x_ab);
         const double delta_n = __dsub_rn(x_ab_length, __dadd_rn(xa.w, xb.w));
         if (delta_n < 0.0) {
             const MixedPair q = mixed_pair_f(x_ab, x_ab_length, delta_n, va, vb, wa, wb, xa.w, xb.w);
-            const d3 nd = B.P.contactmodel == 2 ? contact_linear_mixed(B.P, dt, acc, q, hb)
-                                                : contact_hertz_mixed(B.P, dt, acc, q, hb);
+            const d3 nd = M.contactmodel == 2 ? contact_linear_mixed(M, dt, acc, q, hb)
+                                                : contact_hertz_mixed(M, dt, acc, q, hb);
             L.put3(k, nd);
             live_new |= 1ull << k;
         }
@@ -425,16 +428,31 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
         wb = wq;
         hb = hq;
     }
-    finish_sphere<LM>(A, P, B, i, nxt, ls, xa, wa, acc, live_old, live_new);
+    finish_sphere<LM>(A, P, B, C, i, nxt, ls, xa, wa, acc, live_old, live_new);
 }
 
 template <int LM, int NT, int MINB, bool AHEAD = true>
-__global__ void __launch_bounds__(NT, MINB) k_pair_step(StepArgs A, PairArgs P)
+__global__ void __launch_bounds__(NT, MINB) k_pair_step(const __grid_constant__ StepArgs A,
+                                                        const __grid_constant__ PairArgs P)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp;
-    pair_sphere<LM, AHEAD>(A, P, t, cur, cur ^ 1u, *P.lsel);
+    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    const DevBox &B = A.boxes[box_index(A, i)];
+    pair_sphere<LM, AHEAD>(A, P, B, B, B.P, i, cur, cur ^ 1u, ls);
+}
+
+// k_pair_step of a one-box handle: the box's constants from the arguments.
+template <int LM, int NT, int MINB, bool AHEAD = true>
+__global__ void __launch_bounds__(NT, MINB) k_pair_step1(const __grid_constant__ StepArgs A,
+                                                         const __grid_constant__ PairArgs P,
+                                                         const __grid_constant__ BoxConst C,
+                                                         const __grid_constant__ MixedParams M)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= A.ntot) return;
+    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    pair_sphere<LM, AHEAD>(A, P, A.boxes[0], C, M, i, cur, cur ^ 1u, ls);
 }
 
 // cp.async (global -> shared, issued per thread, completion per thread by
@@ -542,7 +560,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_step_async(StepArgs A, PairAr
         stage(k + D);
     }
     cp_async_wait<0>();
-    finish_sphere<LM>(A, P, B, i, nxt, ls, xa, wa, acc, live_old, live_new);
+    finish_sphere<LM>(A, P, B, B, i, nxt, ls, xa, wa, acc, live_old, live_new);
 }
 
 // Wall-force sum of one chunk of 2^chunk_log2 spheres of one box, and the
@@ -647,7 +665,10 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_persist(StepArgs A, PairArgs 
     const uint32_t cur = *P.pp, nxt = cur ^ 1u, ls = *P.lsel;
     for (uint32_t base = blockIdx.x * NT; base < A.ntot; base += gridDim.x * NT) {
         const uint32_t t = base + threadIdx.x;
-        if (t < A.ntot) pair_sphere<LM>(A, P, t, cur, nxt, ls);
+        if (t >= A.ntot) continue;
+        const uint32_t i = P.order[ls][t];
+        const DevBox &B = A.boxes[box_index(A, i)];
+        pair_sphere<LM, true>(A, P, B, B, B.P, i, cur, nxt, ls);
     }
     if (!grid_barrier(G, gridDim.x, A.err)) return;
     for (uint32_t c = blockIdx.x; c < P.nchunks; c += gridDim.x) chunk_sum(A, P, c, s_w);
@@ -1003,31 +1024,41 @@ void launch_persistent(const StepArgs &A, const PairArgs &P, cudaStream_t st)
     cudaLaunchKernelEx(&c, k_pair_persist<LM, NT, MINB>, A, P, G);
 }
 
-template <int LM>
-void launch_pair_lm(const StepArgs &A, const PairArgs &P, int shape, cudaStream_t st)
+template <int LM, int NT, int MINB, bool AHEAD>
+void launch_pair_step(const StepArgs &A, const PairArgs &P, const DevBox *box0, cudaStream_t st)
 {
-    switch (shape) {
-    case 1: k_pair_step<LM, 128, 5><<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P); break;
-    case 2: k_pair_step<LM, 128, 6><<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P); break;
-    case 3: k_pair_step<LM, 64, 8><<<blocks_for(A.ntot, 64), 64, 0, st>>>(A, P); break;
-    case 4: k_pair_step<LM, 256, 2><<<blocks_for(A.ntot, 256), 256, 0, st>>>(A, P); break;
+    const unsigned g = blocks_for(A.ntot, NT);
+    if (box0)
+        k_pair_step1<LM, NT, MINB, AHEAD><<<g, NT, 0, st>>>(A, P, box_const(*box0), mixed_params(box0->P));
+    else
+        k_pair_step<LM, NT, MINB, AHEAD><<<g, NT, 0, st>>>(A, P);
+}
+
+template <int LM>
+void launch_pair_lm(const StepArgs &A, const PairArgs &P, const StepConfig &cfg, cudaStream_t st)
+{
+    switch (cfg.pair_shape) {
+    case 1: launch_pair_step<LM, 128, 5, true>(A, P, cfg.box0, st); break;
+    case 2: launch_pair_step<LM, 128, 6, true>(A, P, cfg.box0, st); break;
+    case 3: launch_pair_step<LM, 64, 8, true>(A, P, cfg.box0, st); break;
+    case 4: launch_pair_step<LM, 256, 2, true>(A, P, cfg.box0, st); break;
     case 5: launch_staged<LM, 64, 8, 4>(A, P, st); break;
     case 6: launch_staged<LM, 64, 8, 6>(A, P, st); break;
     case 7: launch_staged<LM, 128, 4, 4>(A, P, st); break;
     case 8: launch_staged<LM, 64, 10, 3>(A, P, st); break;
     case 9: launch_persistent<LM, 64, 8>(A, P, st); break;
     case 10: launch_persistent<LM, 128, 4>(A, P, st); break;
-    case 11: k_pair_step<LM, 64, 10, false><<<blocks_for(A.ntot, 64), 64, 0, st>>>(A, P); break;
-    case 12: k_pair_step<LM, 64, 12, false><<<blocks_for(A.ntot, 64), 64, 0, st>>>(A, P); break;
-    default: k_pair_step<LM, 128, 4><<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P); break;
+    case 11: launch_pair_step<LM, 64, 10, false>(A, P, cfg.box0, st); break;
+    case 12: launch_pair_step<LM, 64, 12, false>(A, P, cfg.box0, st); break;
+    default: launch_pair_step<LM, 128, 4, true>(A, P, cfg.box0, st); break;
     }
 }
 
 void launch_pair_kernel(const StepArgs &A, const PairArgs &P, const StepConfig &cfg,
                         cudaStream_t st)
 {
-    if (cfg.lenmode == SPH_LEN_FP64) launch_pair_lm<SPH_LEN_FP64>(A, P, cfg.pair_shape, st);
-    else launch_pair_lm<SPH_LEN_REFERENCE>(A, P, cfg.pair_shape, st);
+    if (cfg.lenmode == SPH_LEN_FP64) launch_pair_lm<SPH_LEN_FP64>(A, P, cfg, st);
+    else launch_pair_lm<SPH_LEN_REFERENCE>(A, P, cfg, st);
 }
 
 }  // namespace

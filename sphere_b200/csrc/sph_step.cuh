@@ -47,7 +47,8 @@ __device__ __forceinline__ double cell_floor(double x, double o, double L, uint3
 
 // Clamped cell coordinates of a position, as the sort stores them, from its
 // cell_floor values; false when some coordinate lies outside the grid.
-__device__ __forceinline__ bool clamp_cell(const DevBox &B, const double f[3], uint32_t c[3])
+template <class BX>
+__device__ __forceinline__ bool clamp_cell(const BX &B, const double f[3], uint32_t c[3])
 {
     bool inside = true;
     for (int d = 0; d < 3; ++d) {
@@ -62,17 +63,19 @@ __device__ __forceinline__ bool clamp_cell(const DevBox &B, const double f[3], u
 // ---------------------------------------------------------------- integrate
 
 // integration.cuh:14-305 integrate (TY3) for one particle.
-__device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevBox &B,
+// (C: the box's constants, the box itself or BoxConst.)
+template <class BX>
+__device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevBox &B, const BX &C,
                                                    uint32_t i, double4 x, double4 vel,
                                                    double4 angvel, d3 F, d3 T)
 {
-    const SphParams &P = B.P;
-    const double dt = B.dt;
+    const SphParams &P = C.P;
+    const double dt = C.dt;
     const double4 angpos = A.angpos[i];
     double4 xyzsum = A.xyzsum[i];
     int wall0mode = 0;
     double wall0mass = 0.0;
-    if (B.nw > 0) {
+    if (C.nw > 0) {
         wall0mode = B.wmode[0];
         wall0mass = B.wmvfd[0][0];
     }
@@ -94,7 +97,7 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     angacc[2] = by_i.div(T.z * 1.0);
     double angacc_w = 0.0;
     if (wall0mode == 3 && vel.w > 0.0001 && x.z > B.L[2] * 0.5) {
-        const double f_tau_x = (B.tau_x + B.tau_eff_x) * B.L[0] * B.L[1];
+        const double f_tau_x = (B.tau_x + B.tau_eff_x) * C.L[0] * C.L[1];
         acc[0] = f_tau_x / wall0mass;
         acc[1] = 0.0;
         acc[2] -= P.g[2];
@@ -133,14 +136,14 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
         wn[d] = wv[d] + angacc[d] * dt + 0.5 * dangacc * dt * dt;
         sv[d] += vv[d] * dt + 0.5 * acc[d] * dt * dt + 1.0 / 6.0 * dacc * dt * dt * dt;
     }
-    if (B.periodic == 1) {
-        if (xn[0] < B.origo[0]) xn[0] += B.L[0];
-        if (xn[0] > B.L[0]) xn[0] -= B.L[0];
-        if (xn[1] < B.origo[1]) xn[1] += B.L[1];
-        if (xn[1] > B.L[1]) xn[1] -= B.L[1];
-    } else if (B.periodic == 2) {
-        if (xn[0] < B.origo[0]) xn[0] += B.L[0];
-        if (xn[0] > B.L[0]) xn[0] -= B.L[0];
+    if (C.periodic == 1) {
+        if (xn[0] < C.origo[0]) xn[0] += C.L[0];
+        if (xn[0] > C.L[0]) xn[0] -= C.L[0];
+        if (xn[1] < C.origo[1]) xn[1] += C.L[1];
+        if (xn[1] > C.L[1]) xn[1] -= C.L[1];
+    } else if (C.periodic == 2) {
+        if (xn[0] < C.origo[0]) xn[0] += C.L[0];
+        if (xn[0] > C.L[0]) xn[0] -= C.L[0];
     }
     if (A.xref) {
         // neighbour-list validity: displacement since the list build
@@ -148,13 +151,13 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
         const float4 r = A.xref[i];
         float ex = (float)xn[0] - r.x, ey = (float)xn[1] - r.y;
         const float ez = (float)xn[2] - r.z;
-        if (B.periodic == 1 || B.periodic == 2) {
-            const float lx = (float)B.L[0];
+        if (C.periodic == 1 || C.periodic == 2) {
+            const float lx = (float)C.L[0];
             if (ex > 0.5f * lx) ex -= lx;
             else if (ex < -0.5f * lx) ex += lx;
         }
-        if (B.periodic == 1) {
-            const float ly = (float)B.L[1];
+        if (C.periodic == 1) {
+            const float ly = (float)C.L[1];
             if (ey > 0.5f * ly) ey -= ly;
             else if (ey < -0.5f * ly) ey += ly;
         }
@@ -165,8 +168,8 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
         double f[3];
         uint32_t c[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) f[d] = cell_floor(xn[d], B.origo[d], B.L[d], B.num[d]);
-        (void)clamp_cell(B, f, c);
+        for (int d = 0; d < 3; ++d) f[d] = cell_floor(xn[d], C.origo[d], C.L[d], C.num[d]);
+        (void)clamp_cell(C, f, c);
         A.cellc[i] = pack_cell(c[0], c[1], c[2]);
     }
     if (vel.w > 5.0 && vel.w < 10.0) {
@@ -453,53 +456,60 @@ __device__ __forceinline__ bool search_contacts(const StepArgs &A, const DevBox 
 // Static and dynamic walls (contactsearch.cuh:428-465 and :602-701) and the
 // bond forces in ascending bond order (cohesion.cuh:220-226), added to acc
 // after the contacts.  Returns the normal force on wall 0.
-template <int LM>
-__device__ __forceinline__ double walls_and_bonds(const StepArgs &A, const DevBox &B, uint32_t i,
+template <int LM, class BX>
+__device__ __forceinline__ double walls_and_bonds(const StepArgs &A, const DevBox &B, const BX &C,
+                                                  uint32_t i,
                                                   double4 xa, d3 vel_a, d3 angvel_a, Acc &acc)
 {
-    const SphParams &P = B.P;
-    const double dt = B.dt;
+    const SphParams &P = C.P;
+    const double dt = C.dt;
     const double radius_a = xa.w;
-    double wnx[5][4] = {{0.0, 0.0, -1.0, B.L[2]}, {-1.0, 0.0, 0.0, B.L[0]}, {1.0, 0.0, 0.0, 0.0},
-                        {0.0, -1.0, 0.0, B.L[1]}, {0.0, 1.0, 0.0, 0.0}};
-    double wvel[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const uint32_t nw = B.nw;
-    for (uint32_t w = 0; w < 5 && w < nw; ++w) {
-        wnx[w][0] = B.wnx[w][0];
-        wnx[w][1] = B.wnx[w][1];
-        wnx[w][2] = B.wnx[w][2];
-        wnx[w][3] = B.wnx[w][3];
-        wvel[w] = B.wmvfd[w][1];
-    }
+    // wall w is the box's wall w when w < nw, else the default plane (top at
+    // L[2], sides at 0 and L); read where it is used
+    const uint32_t nw = C.nw;
+    auto plane = [&](uint32_t w, double dx, double dy, double dz, double dpos, d3 &n, double &pos,
+                     double &vel) {
+        if (w < nw) {
+            n = mk(B.wnx[w][0], B.wnx[w][1], B.wnx[w][2]);
+            pos = B.wnx[w][3];
+            vel = B.wmvfd[w][1];
+        } else {
+            n = mk(dx, dy, dz);
+            pos = dpos;
+            vel = 0.0;
+        }
+    };
     double w0_force = 0.0;
     {
-        double delta_w = wnx[0][3] - (xa.z + radius_a);
+        d3 n;
+        double pos, wv;
+        plane(0, 0.0, 0.0, -1.0, B.L[2], n, pos, wv);
+        double delta_w = pos - (xa.z + radius_a);
         if (delta_w < 0.0)
-            w0_force = contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a,
-                                               mk(wnx[0][0], wnx[0][1], wnx[0][2]), delta_w, wvel[0]);
-        delta_w = xa.z - radius_a - B.origo[2];
+            w0_force = contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, n, delta_w, wv);
+        delta_w = xa.z - radius_a - C.origo[2];
         if (delta_w < 0.0)
             (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, mk(0.0, 0.0, 1.0),
                                           delta_w, 0.0);
-        if (B.periodic == 0) {
-            delta_w = wnx[1][3] - (xa.x + radius_a);
+        if (C.periodic == 0) {
+            plane(1, -1.0, 0.0, 0.0, C.L[0], n, pos, wv);
+            delta_w = pos - (xa.x + radius_a);
             if (delta_w < 0.0)
-                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a,
-                                              mk(wnx[1][0], wnx[1][1], wnx[1][2]), delta_w, wvel[1]);
-            delta_w = xa.x - radius_a - wnx[2][3];
+                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, n, delta_w, wv);
+            plane(2, 1.0, 0.0, 0.0, 0.0, n, pos, wv);
+            delta_w = xa.x - radius_a - pos;
             if (delta_w < 0.0)
-                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a,
-                                              mk(wnx[2][0], wnx[2][1], wnx[2][2]), delta_w, wvel[2]);
+                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, n, delta_w, wv);
         }
-        if (B.periodic == 0 || B.periodic == 2) {
-            delta_w = wnx[3][3] - (xa.y + radius_a);
+        if (C.periodic == 0 || C.periodic == 2) {
+            plane(3, 0.0, -1.0, 0.0, C.L[1], n, pos, wv);
+            delta_w = pos - (xa.y + radius_a);
             if (delta_w < 0.0)
-                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a,
-                                              mk(wnx[3][0], wnx[3][1], wnx[3][2]), delta_w, wvel[3]);
-            delta_w = xa.y - radius_a - wnx[4][3];
+                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, n, delta_w, wv);
+            plane(4, 0.0, 1.0, 0.0, 0.0, n, pos, wv);
+            delta_w = xa.y - radius_a - pos;
             if (delta_w < 0.0)
-                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a,
-                                              mk(wnx[4][0], wnx[4][1], wnx[4][2]), delta_w, wvel[4]);
+                (void)contact_linear_wall<LM>(P, dt, acc, vel_a, angvel_a, radius_a, n, delta_w, wv);
         }
     }
 
@@ -526,7 +536,8 @@ __device__ __forceinline__ double walls_and_bonds(const StepArgs &A, const DevBo
 }
 
 // The per-sphere sums of the step (contactsearch.cuh:707-724).
-__device__ __forceinline__ void store_sums(const StepArgs &A, const DevBox &B, uint32_t i,
+template <class BX>
+__device__ __forceinline__ void store_sums(const StepArgs &A, const BX &B, uint32_t i,
                                            const Acc &acc, double w0_force)
 {
     const double dt = B.dt;
@@ -702,7 +713,7 @@ __global__ void __launch_bounds__(INTERACT_THREADS, MINB) k_interact(StepArgs A)
                 }
     }
 
-    const double w0_force = walls_and_bonds<LM>(A, B, i, xa, vel_a, angvel_a, acc);
+    const double w0_force = walls_and_bonds<LM>(A, B, B, i, xa, vel_a, angvel_a, acc);
 
     if (dirty) {
         uint4 *wrow = reinterpret_cast<uint4 *>(A.slots + (size_t)i * NC);
@@ -714,7 +725,7 @@ __global__ void __launch_bounds__(INTERACT_THREADS, MINB) k_interact(StepArgs A)
 
     store_sums(A, B, i, acc, w0_force);
 
-    if (FUSED) integrate_particle(A, B, i, xa, va4, wa4, acc.F, acc.T);
+    if (FUSED) integrate_particle(A, B, B, i, xa, va4, wa4, acc.F, acc.T);
 }
 
 // ------------------------------------------------------------ split step
@@ -741,7 +752,8 @@ constexpr int FINISH_THREADS = 128;
 
 // In a step without k_hash: its checks of the sphere's position and its cell
 // id.
-__device__ __forceinline__ void position_check(const StepArgs &A, const DevBox &B, uint32_t i,
+template <class BX>
+__device__ __forceinline__ void position_check(const StepArgs &A, const BX &B, uint32_t i,
                                                double4 x)
 {
     const double f[3] = {cell_floor(x.x, B.origo[0], B.L[0], B.num[0]),
@@ -756,7 +768,8 @@ __device__ __forceinline__ void position_check(const StepArgs &A, const DevBox &
 }
 
 // The image shift that brings b nearest to a along the periodic axes.
-__device__ __forceinline__ void nearest_image(const DevBox &B, const double4 &xa, const double4 &xb,
+template <class BX>
+__device__ __forceinline__ void nearest_image(const BX &B, const double4 &xa, const double4 &xb,
                                               int &sx, int &sy)
 {
     sx = sy = 0;
@@ -980,11 +993,11 @@ __device__ __forceinline__ ContactRec get_rec(const RecSlab &S, int t)
 // pair no longer touches (r.nev < 0 then); returns whether it touches.
 // NEAREST: the image is the nearest one (see k_touch) and the slot's code is
 // brought up to date; else the slot's code says it.
-template <int LM, bool MIXED, bool NEAREST>
-__device__ __forceinline__ bool slot_contact(const StepArgs &A, uint32_t i, int s, uint32_t w,
-                                             ContactRec &r)
+// B, M: the box's constants and its contact parameters.
+template <int LM, bool MIXED, bool NEAREST, class BX, class PT>
+__device__ __forceinline__ bool slot_contact(const StepArgs &A, const BX &B, const PT &M, uint32_t i,
+                                             int s, uint32_t w, ContactRec &r)
 {
-    const DevBox &B = A.boxes[box_index(A, i)];
     const SphParams &P = B.P;
     const double dt = B.dt;
     const uint32_t cm = P.contactmodel;
@@ -1030,8 +1043,8 @@ __device__ __forceinline__ bool slot_contact(const StepArgs &A, uint32_t i, int 
     if (MIXED) {
         const MixedPair mp = mixed_pair(x_ab, x_ab_length, delta_n, vel_a, vel_b,
                                         tof(angvel_a), xyzf(wb4), radius_a, xb.w);
-        if (cm == 2) nd = contact_linear_mixed(P, dt, r, mp, h0);
-        else nd = contact_hertz_mixed(P, dt, r, mp, h0);
+        if (cm == 2) nd = contact_linear_mixed(M, dt, r, mp, h0);
+        else nd = contact_hertz_mixed(M, dt, r, mp, h0);
     } else {
         const d3 angvel_b = xyz(wb4);
         if (cm == 2)
@@ -1116,7 +1129,9 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_contacts(StepArgs A)
         ContactRec r = no_rec();
         if (f < total) {
             const uint2 e = ent[f];
-            (void)slot_contact<LM, MIXED, false>(A, e.y & SPLIT_ID_MASK, (int)(e.y >> 27), e.x, r);
+            const uint32_t i = e.y & SPLIT_ID_MASK;
+            const DevBox &B = A.boxes[box_index(A, i)];
+            (void)slot_contact<LM, MIXED, false>(A, B, B.P, i, (int)(e.y >> 27), e.x, r);
         }
         put_rec(S, (int)threadIdx.x, r);
         __syncwarp();
@@ -1149,6 +1164,26 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_contacts(StepArgs A)
 // Contacts are then dealt to the warp's lanes as in k_contacts, contact f of
 // the warp found from the lanes' counts and occupied slots.
 constexpr unsigned long long LMASK_VALID = 1ull << 63;
+// Resident blocks per SM, which sets the registers: 96 or 102 a thread.  With
+// 80 (6 blocks) the FP64 laws spill 60 values: 508 us against 451 at 1e6
+// spheres.
+#ifndef TOUCH_BLOCKS
+#define TOUCH_BLOCKS 5
+#endif
+
+// Where touch_warp finds the constants of sphere i's box and its contact
+// parameters.
+struct TableBoxes {
+    const StepArgs &A;
+    __device__ __forceinline__ const DevBox &box(uint32_t i) const { return A.boxes[box_index(A, i)]; }
+    __device__ __forceinline__ const SphParams &params(uint32_t i) const { return box(i).P; }
+};
+struct OneBox {
+    const BoxConst &C;
+    const MixedParams &M;
+    __device__ __forceinline__ const BoxConst &box(uint32_t) const { return C; }
+    __device__ __forceinline__ const MixedParams &params(uint32_t) const { return M; }
+};
 
 // The search of sphere i on its row in memory; which entries of its list are
 // in the row is found anew.  (Rare: not inlined, for the registers.)
@@ -1175,10 +1210,9 @@ __device__ __noinline__ uint32_t touch_row(const StepArgs &A, uint32_t i)
     return occ;
 }
 
-template <int LM>
-__device__ __forceinline__ uint32_t touch_search(const StepArgs &A, uint32_t i)
+template <int LM, class BX>
+__device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B, uint32_t i)
 {
-    const DevBox &B = A.boxes[box_index(A, i)];
     const unsigned long long m = A.lmask[i];
     const uint32_t vc = A.vcount[i];
     uint32_t occ = A.occ[i];
@@ -1245,17 +1279,16 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, uint32_t i)
     return occ;
 }
 
-template <int LM, bool MIXED>
-__global__ void __launch_bounds__(CONTACT_THREADS, 6) k_touch(const __grid_constant__ StepArgs A)
+// SPW: spheres of a warp (see launch_contacts_lm).
+template <int LM, bool MIXED, int SPW, class Boxes>
+__device__ __forceinline__ void touch_warp(const StepArgs &A, RecSlab &S, const Boxes &at)
 {
-    __shared__ RecSlab S;
-    grid_dependency_wait();
     const uint32_t lane = threadIdx.x & 31u;
     const int wbase = (int)(threadIdx.x & ~31u);
-    const uint32_t i_own = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i0 = i_own - lane;
-    const bool valid = i_own < A.ntot;
-    const uint32_t occ_own = valid ? touch_search<LM>(A, i_own) : 0u;
+    const uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) / 32u * SPW;
+    const uint32_t i_own = i0 + lane;
+    const bool valid = lane < (uint32_t)SPW && i_own < A.ntot;
+    const uint32_t occ_own = valid ? touch_search<LM>(A, at.box(i_own), i_own) : 0u;
     const uint32_t nl_own = (uint32_t)__popc(occ_own);
     const uint32_t incl = warp_inclusive(nl_own, lane);
     const uint32_t excl = incl - nl_own;
@@ -1281,7 +1314,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_touch(const __grid_const
             const int s = __ffs(m) - 1;
             const uint32_t i = i0 + o;
             const uint32_t w = A.slots[(size_t)i * NC + s];
-            if (!slot_contact<LM, MIXED, true>(A, i, s, w, r)) {
+            if (!slot_contact<LM, MIXED, true>(A, at.box(i), at.params(i), i, s, w, r)) {
                 // the contact ended: its entry is no longer in the row
                 const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
                 const uint32_t vc = A.vcount[i];
@@ -1300,28 +1333,56 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_touch(const __grid_const
     if (valid) A.csum[i_own] = acc;
 }
 
-template <int LM>
-__global__ void __launch_bounds__(FINISH_THREADS, 4) k_finish(StepArgs A)
+template <int LM, bool MIXED, int SPW>
+__global__ void __launch_bounds__(CONTACT_THREADS, TOUCH_BLOCKS) k_touch(const __grid_constant__ StepArgs A)
 {
-    // original order: every access of this kernel is to the sphere's own
-    // entries, so they are all coalesced (x, vel, angvel still hold the
-    // state at the start of the step: only this thread rewrites them)
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.ntot) return;
-    const DevBox &B = A.boxes[box_index(A, i)];
+    __shared__ RecSlab S;
+    grid_dependency_wait();
+    touch_warp<LM, MIXED, SPW>(A, S, TableBoxes{A});
+}
+
+// k_touch of a one-box handle: the box's constants from the arguments.
+template <int LM, bool MIXED, int SPW>
+__global__ void __launch_bounds__(CONTACT_THREADS, TOUCH_BLOCKS) k_touch1(const __grid_constant__ StepArgs A,
+                                                                          const __grid_constant__ BoxConst C,
+                                                                          const __grid_constant__ MixedParams M)
+{
+    __shared__ RecSlab S;
+    grid_dependency_wait();
+    touch_warp<LM, MIXED, SPW>(A, S, OneBox{C, M});
+}
+
+// Original order: every access is to the sphere's own entries, so they are
+// all coalesced (x, vel, angvel still hold the state at the start of the
+// step: only this thread rewrites them).
+template <int LM, class BX>
+__device__ __forceinline__ void finish_one(const StepArgs &A, const DevBox &B, const BX &C, uint32_t i)
+{
     const double4 xa = A.x[i];
     const double4 va4 = A.vel[i];
     const double4 wa4 = A.angvel[i];
-    Acc acc;
-    acc.F = mk(0.0, 0.0, 0.0);
-    acc.T = mk(0.0, 0.0, 0.0);
-    acc.es_dot = 0.0;
-    acc.ev_dot = 0.0;
-    acc.p = 0.0;
-    acc = A.csum[i];   // the contacts' sums, added in slot order by k_contacts
-    const double w0_force = walls_and_bonds<LM>(A, B, i, xa, xyz(va4), xyz(wa4), acc);
-    store_sums(A, B, i, acc, w0_force);
-    integrate_particle(A, B, i, xa, va4, wa4, acc.F, acc.T);
+    Acc acc = A.csum[i];   // the contacts' sums, added in slot order
+    const double w0_force = walls_and_bonds<LM>(A, B, C, i, xa, xyz(va4), xyz(wa4), acc);
+    store_sums(A, C, i, acc, w0_force);
+    integrate_particle(A, B, C, i, xa, va4, wa4, acc.F, acc.T);
+}
+
+template <int LM>
+__global__ void __launch_bounds__(FINISH_THREADS, 4) k_finish(const __grid_constant__ StepArgs A)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.ntot) return;
+    const DevBox &B = A.boxes[box_index(A, i)];
+    finish_one<LM>(A, B, B, i);
+}
+
+// k_finish of a one-box handle: the box's constants from the arguments.
+template <int LM>
+__global__ void __launch_bounds__(FINISH_THREADS, 4) k_finish1(const __grid_constant__ StepArgs A,
+                                                               const __grid_constant__ BoxConst C)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.ntot) finish_one<LM>(A, A.boxes[0], C, i);
 }
 
 // Launch variants of k_interact (INTERACT_VARIANTS): the minimum resident
@@ -1337,16 +1398,41 @@ inline void launch_interact_lm(const StepArgs &A, cudaStream_t st, unsigned grid
     else k_interact<LM, FUSED, MIXED, 4><<<grid, INTERACT_THREADS, 0, st>>>(A);
 }
 
-template <bool MIXED>
-inline void launch_contacts(const StepArgs &A, cudaStream_t st, unsigned grid, int lm, bool pdl)
+template <bool MIXED, int LM, int SPW>
+inline void launch_touch(const StepArgs &A, const DevBox *box0, cudaStream_t st, bool pdl)
 {
-    if (A.touch) {
-        if (lm == SPH_LEN_FP64) launch_k(pdl, k_touch<SPH_LEN_FP64, MIXED>, grid, CONTACT_THREADS, st, A);
-        else launch_k(pdl, k_touch<SPH_LEN_REFERENCE, MIXED>, grid, CONTACT_THREADS, st, A);
-        return;
-    }
-    if (lm == SPH_LEN_FP64) launch_k(pdl, k_contacts<SPH_LEN_FP64, MIXED>, grid, CONTACT_THREADS, st, A);
-    else launch_k(pdl, k_contacts<SPH_LEN_REFERENCE, MIXED>, grid, CONTACT_THREADS, st, A);
+    const unsigned per_block = CONTACT_THREADS / 32 * SPW;
+    const unsigned grid = (A.ntot + per_block - 1) / per_block;
+    if (box0)
+        launch_k(pdl, k_touch1<LM, MIXED, SPW>, grid, CONTACT_THREADS, st, A, box_const(*box0),
+                 mixed_params(box0->P));
+    else
+        launch_k(pdl, k_touch<LM, MIXED, SPW>, grid, CONTACT_THREADS, st, A);
+}
+
+template <bool MIXED, int LM>
+inline void launch_contacts_lm(const StepArgs &A, const DevBox *box0, cudaStream_t st, unsigned grid,
+                               bool pdl)
+{
+    // Fewer spheres to a warp while all warps fit on the chip at once
+    // (TOUCH_BLOCKS blocks on each of 148 SMs): their contacts then take fewer
+    // rounds, the warps run side by side.  us of k_touch with 32 / 16 / 8 / 4
+    // spheres a warp: 500 spheres (FP64) 21.0 / 14.5 / 10.9 / 9.4; 60,013: 42.2 /
+    // 43.9 / 46.9 / 55; 1e6: 451 / 559 / 729 / 951.
+    constexpr uint32_t WARPS = 148u * TOUCH_BLOCKS * (CONTACT_THREADS / 32);
+    if (!A.touch) launch_k(pdl, k_contacts<LM, MIXED>, grid, CONTACT_THREADS, st, A);
+    else if (A.ntot <= 4u * WARPS) launch_touch<MIXED, LM, 4>(A, box0, st, pdl);
+    else if (A.ntot <= 8u * WARPS) launch_touch<MIXED, LM, 8>(A, box0, st, pdl);
+    else if (A.ntot <= 16u * WARPS) launch_touch<MIXED, LM, 16>(A, box0, st, pdl);
+    else launch_touch<MIXED, LM, 32>(A, box0, st, pdl);
+}
+
+template <bool MIXED>
+inline void launch_contacts(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, unsigned grid,
+                            bool pdl)
+{
+    if (cfg.lenmode == SPH_LEN_FP64) launch_contacts_lm<MIXED, SPH_LEN_FP64>(A, cfg.box0, st, grid, pdl);
+    else launch_contacts_lm<MIXED, SPH_LEN_REFERENCE>(A, cfg.box0, st, grid, pdl);
 }
 
 template <bool MIXED>
