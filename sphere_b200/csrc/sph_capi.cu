@@ -2065,15 +2065,21 @@ int sph_adjoint_backward(SphHandle *h, const double *dx_final, double *grad_para
         if (kind < 0) {
             for (uint64_t k = 0; k < ns && rst == SPH_OK; ++k) {
                 char *t = tape + step_tape * k;
-                cudaMemcpyAsync(t, h->A.x, n4, cudaMemcpyDeviceToDevice, h->own);
-                cudaMemcpyAsync(t + n4, h->A.vel, n4, cudaMemcpyDeviceToDevice, h->own);
-                cudaMemcpyAsync(t + 2 * n4, h->A.angvel, n4, cudaMemcpyDeviceToDevice, h->own);
                 StepArgs Ar = h->A;
+                const StepConfig cfg = step_config(h);
+                if (cfg.touch) {
+                    // the contact kernel writes the start state itself
+                    Ar.tape_state = (double4 *)t;
+                } else {
+                    cudaMemcpyAsync(t, h->A.x, n4, cudaMemcpyDeviceToDevice, h->own);
+                    cudaMemcpyAsync(t + n4, h->A.vel, n4, cudaMemcpyDeviceToDevice, h->own);
+                    cudaMemcpyAsync(t + 2 * n4, h->A.angvel, n4, cudaMemcpyDeviceToDevice, h->own);
+                }
                 Ar.tape_rows_pre = (uint32_t *)(t + 3 * n4);
                 Ar.tape_rows_post = Ar.tape_rows_pre + (size_t)n * sph::NC;
                 Ar.tape_hist = (double4 *)(Ar.tape_rows_post + (size_t)n * sph::NC);
                 uint64_t nl = 0;
-                rst = sph::launch_step(Ar, step_config(h), h->own, &nl);
+                rst = sph::launch_step(Ar, cfg, h->own, &nl);
             }
         } else {
             const bool first = (kind >> 1) != 0;

@@ -77,6 +77,7 @@ struct StepArgs {
     // tangential histories the interact pass reads
     uint32_t *tape_rows_pre, *tape_rows_post;
     double4 *tape_hist;
+    double4 *tape_state;       // x, vel, angvel at the step's start (k_touch only)
 };
 
 constexpr int VL_MAX = 48;   // neighbour-list capacity per sphere

@@ -1219,6 +1219,11 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
     const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
     const double4 xa = A.x[i];
     position_check(A, B, i, xa);
+    if (A.tape_state) {
+        A.tape_state[i] = xa;
+        A.tape_state[A.ntot + i] = A.vel[i];
+        A.tape_state[2 * (size_t)A.ntot + i] = A.angvel[i];
+    }
     if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return touch_row<LM>(A, i);
     // the first entry that is not in the row and touches, and its slot word
     uint32_t found = 0, kf = 0, wf = 0;
@@ -1258,8 +1263,12 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
     // several new contacts take their slots in the cells' visit order
     if (found > 1u || (found == 1u && occ == 0xffffffffu)) return touch_row<LM>(A, i);
     uint32_t *row = A.slots + (size_t)i * NC;
-    if (A.tape_rows_pre)
-        for (int s = 0; s < NC; ++s) A.tape_rows_pre[(size_t)i * NC + s] = row[s];
+    const uint4 *row4 = reinterpret_cast<const uint4 *>(row);
+    if (A.tape_rows_pre) {
+        uint4 *t = reinterpret_cast<uint4 *>(A.tape_rows_pre + (size_t)i * NC);
+#pragma unroll
+        for (int q = 0; q < NC / 4; ++q) t[q] = row4[q];
+    }
     if (found) {
         // one: the highest free slot
         const int s = 31 - __clz((int)~occ);
@@ -1269,11 +1278,12 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
         A.lmask[i] = m | (1ull << kf);
     }
     if (A.tape_rows_post) {
-        const double4 *hist = A.hist + (size_t)i * NC;
-        for (int s = 0; s < NC; ++s) {
-            const uint32_t w = row[s];
-            A.tape_rows_post[(size_t)i * NC + s] = w;
-            if (w != EMPTY) A.tape_hist[(size_t)i * NC + s] = hist[s];
+        uint4 *t = reinterpret_cast<uint4 *>(A.tape_rows_post + (size_t)i * NC);
+#pragma unroll
+        for (int q = 0; q < NC / 4; ++q) t[q] = row4[q];
+        for (uint32_t m2 = occ; m2; m2 &= m2 - 1u) {
+            const size_t q = (size_t)i * NC + (size_t)(__ffs(m2) - 1);
+            A.tape_hist[q] = A.hist[q];
         }
     }
     return occ;
