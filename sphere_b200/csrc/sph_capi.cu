@@ -206,11 +206,12 @@ static int ensure_pair(SphHandle *h)
         (st = dalloc(h, &P.hist[1], 3 * n * sph::VL_MAX)) || (st = dalloc(h, &words, 5)) ||
         (st = dalloc(h, &P.chunk_part, cbox.size())) || (st = dalloc(h, &chunk_box, cbox.size())) ||
         (st = dalloc(h, &box_chunk0, h->nbox)) || (st = dalloc(h, &key_base, h->nbox)) ||
-        (st = dalloc(h, &P.src, n)) || (st = dalloc(h, &P.dst, n)) ||
+        (st = dalloc(h, &P.box_done, h->nbox)) || (st = dalloc(h, &P.src, n)) || (st = dalloc(h, &P.dst, n)) ||
         (st = dalloc(h, &P.key_count, nkeys)) || (st = dalloc(h, &P.key_off, nkeys + 1)) ||
         (st = dalloc(h, &P.key_scan, nkeys / 4096 + 2)))
         return st;
     P.key_base = key_base;
+    CUDA_TRY(h, cudaMemset(P.box_done, 0, sizeof(uint32_t) * h->nbox));
     P.nkeys = (uint32_t)nkeys;
     CUDA_TRY(h, cudaMemcpy(key_base, kb.data(), 4 * kb.size(), cudaMemcpyHostToDevice));
     P.pp = words;

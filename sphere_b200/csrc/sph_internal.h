@@ -138,6 +138,7 @@ struct PairArgs {
     uint32_t *from_rows;       // != 0: the next rebuild takes histories from A.slots / A.hist
     uint32_t *bar;             // grid-barrier words of the persistent shapes: count, generation
     double *chunk_part;        // [nchunks]
+    uint32_t *box_done;        // per box its chunks summed so far in this wall stage
     const uint32_t *chunk_box; // box of each chunk
     uint32_t nchunks;
     uint32_t chunk_log2;       // chunk = 1 << chunk_log2 spheres of one box

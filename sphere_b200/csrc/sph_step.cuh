@@ -201,8 +201,10 @@ __device__ __forceinline__ void advance_box(DevBox &B, double fsum)
             if (wmode == 0) continue;
             const double acc0 = B.iter == 0 ? 0.0 : B.wacc[w];
             B.wmvfd[w][2] = fsum;
-            const double sigma_0 =
-                B.wmvfd[w][3] + B.P.sigma0_A * sin(2.0 * PI * B.P.sigma0_f * B.t_current);
+            // (without modulation the product is a zero, whatever the sine)
+            const double mod =
+                B.P.sigma0_A == 0.0 ? 0.0 : B.P.sigma0_A * sin(2.0 * PI * B.P.sigma0_f * B.t_current);
+            const double sigma_0 = B.wmvfd[w][3] + mod;
             const double N = -sigma_0 * B.L[0] * B.L[1];
             double acc = (B.wmvfd[w][2] + N) / B.wmvfd[w][0];
             if (wmode == 2) acc = 0.0;
