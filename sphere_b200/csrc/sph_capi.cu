@@ -76,6 +76,12 @@ struct SphHandle {
     bool variant_set = false;   // cfg.variant was chosen by the caller or the tuner
     std::string err;
     std::vector<void *> allocs;
+    // the chunk that small device arrays are cut from (dalloc), and scratch of
+    // the analysis calls, kept and grown as they need it (scratch_mem)
+    char *chunk = nullptr;
+    size_t chunk_left = 0;
+    char *scratch = nullptr;
+    size_t scratch_bytes = 0;
     unsigned long long *d_count = nullptr;
     uint32_t *vlist_mem = nullptr;   // neighbour-list storage (A.vlist is null when off)
     std::vector<double> rmax_box;    // largest radius per box (at upload)
@@ -134,17 +140,52 @@ static int fail(SphHandle *h, int code, const std::string &msg)
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
     } while (0)
 
+// A device array of the handle, freed with it.  Arrays up to half a chunk are
+// cut from 16 MB chunks (256-byte aligned, as cudaMalloc's): a handle of 50,000
+// spheres makes some 70 arrays, and each allocation of its own costs about
+// 80 us to make and as much to free.
+constexpr size_t CHUNK_BYTES = 16u << 20;
+
 template <typename T>
 static int dalloc(SphHandle *h, T **p, uint64_t count)
 {
     if (count == 0) count = 1;
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, sizeof(T) * count);
-    if (e != cudaSuccess)
-        return fail(h, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    h->allocs.push_back(q);
-    *p = static_cast<T *>(q);
+    const size_t bytes = (sizeof(T) * count + 255) & ~(size_t)255;
+    const bool own = bytes > CHUNK_BYTES / 2;
+    if (own || bytes > h->chunk_left) {
+        void *q = nullptr;
+        cudaError_t e = cudaMalloc(&q, own ? bytes : CHUNK_BYTES);
+        if (e != cudaSuccess)
+            return fail(h, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        h->allocs.push_back(q);
+        if (own) {
+            *p = static_cast<T *>(q);
+            return SPH_OK;
+        }
+        h->chunk = static_cast<char *>(q);
+        h->chunk_left = CHUNK_BYTES;
+    }
+    *p = reinterpret_cast<T *>(h->chunk);
+    h->chunk += bytes;
+    h->chunk_left -= bytes;
     return SPH_OK;
+}
+
+// At least `bytes` of device scratch for one call (256-byte aligned), kept for
+// the next; its contents are the caller's only until the call returns.  Null
+// when the device has no room.
+static char *scratch_mem(SphHandle *h, size_t bytes)
+{
+    if (bytes > h->scratch_bytes) {
+        cudaFree(h->scratch);
+        h->scratch = nullptr;
+        h->scratch_bytes = 0;
+        void *q = nullptr;
+        if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+        h->scratch = static_cast<char *>(q);
+        h->scratch_bytes = bytes;
+    }
+    return h->scratch;
 }
 
 // Whether the list step (launch variant 4) can run this handle: the
@@ -457,6 +498,7 @@ void sph_destroy(SphHandle *h)
     if (h->adj_snaps) cudaFree(h->adj_snaps);
     if (h->snap_ev) cudaEventDestroy(h->snap_ev);
     if (h->snap_stream) cudaStreamDestroy(h->snap_stream);
+    cudaFree(h->scratch);
     for (void *p : h->allocs) cudaFree(p);
     if (h->own) cudaStreamDestroy(h->own);
     delete h;
@@ -2388,12 +2430,9 @@ int sph_porosity(SphHandle *h, uint32_t box, uint32_t z_slices, double *z_pos, d
     if (h_slice <= h->rmax_box[box] * 2.0)
         return fail(h, SPH_ERR_INPUT, "the number of z-slices is too high (slab <= 2 r_max)");
     const double V_slice = h_slice * d.L[0] * d.L[1];
-    double *dz = nullptr, *dp = nullptr;
-    if (cudaMalloc((void **)&dz, sizeof(double) * z_slices) != cudaSuccess ||
-        cudaMalloc((void **)&dp, sizeof(double) * z_slices) != cudaSuccess) {
-        cudaFree(dz);
-        return fail(h, SPH_ERR_NOMEM, "porosity buffers");
-    }
+    double *dz = (double *)scratch_mem(h, 2 * sizeof(double) * (size_t)z_slices);
+    if (!dz) return fail(h, SPH_ERR_NOMEM, "porosity buffers");
+    double *dp = dz + z_slices;
     int st = sph::porosity_profile(h->A.x, d.p_base, d.np, h_slice, V_slice, z_slices, dz, dp,
                                    h->stream);
     cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -2402,8 +2441,6 @@ int sph_porosity(SphHandle *h, uint32_t box, uint32_t z_slices, double *z_pos, d
         if (e == cudaSuccess)
             e = cudaMemcpy(porosity, dp, sizeof(double) * z_slices, cudaMemcpyDeviceToHost);
     }
-    cudaFree(dz);
-    cudaFree(dp);
     if (st != SPH_OK) return fail(h, st, "porosity kernel launch failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     return SPH_OK;
@@ -2440,30 +2477,29 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
     const uint64_t ncells = (uint64_t)d.num[0] * d.num[1] * d.num[2];
     const uint64_t n = d.np ? d.np : 1;
     if (n > 4096ull * 4096ull) return fail(h, SPH_ERR_UNSUPPORTED, "box too large for sph_overlaps");
-    std::vector<void *> mine;
-    auto get = [&](size_t bytes) -> void * {
-        void *q = nullptr;
-        if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
-        mine.push_back(q);
-        return q;
+    // the arrays in one piece of scratch
+    size_t used = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = used;
+        used += (bytes + 255) & ~(size_t)255;
+        return at;
     };
-    auto release = [&]() {
-        for (void *q : mine) cudaFree(q);
-    };
-    O.cell_of = (uint32_t *)get(4 * n);
-    O.slot = (uint32_t *)get(4 * n);
-    O.count = (uint32_t *)get(4 * (ncells + 1));
-    O.coff = (uint32_t *)get(4 * (ncells + 1));
-    O.items = (uint32_t *)get(4 * n);
-    O.xs = (double4 *)get(sizeof(double4) * n);
-    O.npair = (uint32_t *)get(4 * (n + 1));
-    O.poff = (uint32_t *)get(4 * (n + 1));
-    uint32_t *scan_tmp = (uint32_t *)get(4 * (ncells / 4096 + n / 4096 + 2));
-    if (!O.cell_of || !O.slot || !O.count || !O.coff || !O.items || !O.xs || !O.npair || !O.poff ||
-        !scan_tmp) {
-        release();
-        return fail(h, SPH_ERR_NOMEM, "overlap-search buffers");
-    }
+    const size_t o_cell = place(4 * n), o_slot = place(4 * n), o_count = place(4 * (ncells + 1)),
+                 o_coff = place(4 * (ncells + 1)), o_items = place(4 * n), o_xs = place(sizeof(double4) * n),
+                 o_npair = place(4 * (n + 1)), o_poff = place(4 * (n + 1)),
+                 o_scan = place(4 * (ncells / 4096 + n / 4096 + 2));
+    char *mem = scratch_mem(h, used);
+    if (!mem) return fail(h, SPH_ERR_NOMEM, "overlap-search buffers");
+    O.cell_of = (uint32_t *)(mem + o_cell);
+    O.slot = (uint32_t *)(mem + o_slot);
+    O.count = (uint32_t *)(mem + o_count);
+    O.coff = (uint32_t *)(mem + o_coff);
+    O.items = (uint32_t *)(mem + o_items);
+    O.xs = (double4 *)(mem + o_xs);
+    O.npair = (uint32_t *)(mem + o_npair);
+    O.poff = (uint32_t *)(mem + o_poff);
+    uint32_t *scan_tmp = (uint32_t *)(mem + o_scan);
+    char *list = nullptr;   // the pairs: where the scratch has room behind the arrays, else their own
     int st = sph::find_overlaps(O, (uint32_t)ncells, scan_tmp, h->stream, 0);
     uint32_t total = 0;
     cudaError_t e = cudaSuccess;
@@ -2473,12 +2509,15 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
     if (st == SPH_OK && e == cudaSuccess && total > 0 && max_pairs > 0 && (pairs || delta_n)) {
-        O.pairs = (uint32_t *)get(8 * (size_t)total);
-        O.delta = (double *)get(8 * (size_t)total);
-        if (!O.pairs || !O.delta) {
-            release();
-            return fail(h, SPH_ERR_NOMEM, "overlap list buffers");
+        const size_t half = (8 * (size_t)total + 255) & ~(size_t)255;
+        if (used + 2 * half <= h->scratch_bytes) {
+            O.pairs = (uint32_t *)(mem + used);
+        } else {
+            if (cudaMalloc((void **)&list, 2 * half) != cudaSuccess)
+                return fail(h, SPH_ERR_NOMEM, "overlap list buffers");
+            O.pairs = (uint32_t *)list;
         }
+        O.delta = (double *)((char *)O.pairs + half);
         st = sph::find_overlaps(O, (uint32_t)ncells, scan_tmp, h->stream, 1);
         const uint64_t m = total < max_pairs ? total : max_pairs;
         if (st == SPH_OK && pairs)
@@ -2487,7 +2526,12 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
             e = cudaMemcpyAsync(delta_n, O.delta, 8 * m, cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
-    release();
+    if (list) {
+        // room for as many pairs in the next call
+        const size_t want = used + 2 * ((8 * (size_t)total + 255) & ~(size_t)255);
+        cudaFree(list);
+        (void)scratch_mem(h, want);
+    }
     if (st != SPH_OK) return fail(h, st, "overlap-search launch failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     *npairs = total;
@@ -2516,16 +2560,20 @@ int sph_render(SphHandle *h, uint32_t box, int method, float maxval, float lower
     const double *d_L = reinterpret_cast<const double *>(
         reinterpret_cast<const char *>(h->A.boxes + box) + offsetof(DevBox, L));
     const size_t bytes = (size_t)width * height * 3;
-    uint8_t *img = nullptr;
-    if (cudaMalloc((void **)&img, bytes) != cudaSuccess)
-        return fail(h, SPH_ERR_NOMEM, "image buffer");
+    const size_t img_bytes = (bytes + 255) & ~(size_t)255;
+    const size_t rt_bytes = sph::render_scratch(d.np, width, height);
+    uint8_t *img = (uint8_t *)scratch_mem(h, img_bytes + rt_bytes);
+    if (!img) return fail(h, SPH_ERR_NOMEM, "image buffer");
     sph::RenderStats rs;
     int st = sph::render_image(h->A, d.p_base, d.np, d_L, method, maxval, lower_cutoff, width,
-                               height, img, h->stream, &rs);
+                               height, img, (char *)img + img_bytes,
+                               h->scratch_bytes - img_bytes, h->stream, &rs);
     h->launches += (uint64_t)rs.launches;
     cudaError_t e = cudaSuccess;
     if (st == SPH_OK) e = cudaMemcpy(rgb, img, bytes, cudaMemcpyDeviceToHost);
-    cudaFree(img);
+    // room for as many tile-list entries in the next call
+    const size_t want = img_bytes + rt_bytes + 256 + sizeof(uint32_t) * (size_t)rs.entries;
+    if (st == SPH_OK && e == cudaSuccess && want > h->scratch_bytes) (void)scratch_mem(h, want);
     if (st != SPH_OK) return fail(h, st, "ray-tracing kernels failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     return SPH_OK;

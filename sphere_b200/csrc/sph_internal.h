@@ -339,11 +339,14 @@ struct RenderStats {
     int launches = 0;
 };
 // Renders spheres [p0, p0 + np) into d_img (width * height * 3 bytes,
-// row-major RGB).  d_L is the box's grid.L in device memory.  Allocates and
-// frees its own scratch; synchronises st once (to size the tile lists) and
-// at the end.
+// row-major RGB).  d_L is the box's grid.L in device memory.  scratch: device
+// memory of at least render_scratch bytes; the tile lists go behind them where
+// scratch_bytes has room, else into memory of their own.  Synchronises st once
+// (to size the tile lists) and at the end.
+size_t render_scratch(uint32_t np, uint32_t width, uint32_t height);
 int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L, int method,
                  float maxval, float lower_cutoff, uint32_t width, uint32_t height,
-                 uint8_t *d_img, cudaStream_t st, RenderStats *stats);
+                 uint8_t *d_img, char *scratch, size_t scratch_bytes, cudaStream_t st,
+                 RenderStats *stats);
 
 }  // namespace sph

@@ -314,9 +314,19 @@ __global__ void __launch_bounds__(TILE * TILE) k_rt_trace(RtArgs R)
 
 }  // namespace
 
+// Scratch of render_image but for the tile lists: maxbits[3] | camera | xf[np] |
+// tcount, tfill, toff[ntiles + 1].
+constexpr size_t RT_CAM = 32, RT_XF = 256;
+static size_t rt_tiles(uint32_t width) { return ((size_t)width + TILE - 1) / TILE * (((size_t)width + TILE - 1) / TILE); }
+
+size_t render_scratch(uint32_t np, uint32_t width, uint32_t)
+{
+    return RT_XF + sizeof(float4) * (size_t)np + sizeof(uint32_t) * (3 * rt_tiles(width) + 1);
+}
+
 int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L, int method,
                  float maxval, float lower_cutoff, uint32_t width, uint32_t height, uint8_t *d_img,
-                 cudaStream_t st, RenderStats *stats)
+                 char *buf, size_t buf_bytes, cudaStream_t st, RenderStats *stats)
 {
     RtArgs R{};
     R.x = A.x;
@@ -337,16 +347,12 @@ int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L,
     R.lower_cutoff = lower_cutoff;
     R.img = d_img;
     const uint32_t ntiles = R.tx * R.ty;
-    // scratch: maxbits[3] | camera | xf[np] | tcount, tfill, toff[ntiles + 1]
-    static_assert(sizeof(Camera) <= 224, "camera slot");
-    const size_t off_cam = 32, off_xf = 256;
-    const size_t off_t = off_xf + sizeof(float4) * (size_t)np;
-    const size_t bytes = off_t + sizeof(uint32_t) * (3 * (size_t)ntiles + 1);
-    char *buf = nullptr;
-    if (cudaMalloc((void **)&buf, bytes) != cudaSuccess) return SPH_ERR_NOMEM;
+    static_assert(sizeof(Camera) <= RT_XF - RT_CAM, "camera slot");
+    const size_t off_t = RT_XF + sizeof(float4) * (size_t)np;
+    const size_t bytes = render_scratch(np, width, height);
     R.maxbits = (unsigned long long *)buf;
-    R.cam = (Camera *)(buf + off_cam);
-    R.xf = (float4 *)(buf + off_xf);
+    R.cam = (Camera *)(buf + RT_CAM);
+    R.xf = (float4 *)(buf + RT_XF);
     R.tcount = (uint32_t *)(buf + off_t);
     R.tfill = R.tcount + ntiles;
     R.toff = R.tfill + ntiles;
@@ -368,16 +374,17 @@ int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L,
     cudaMemcpyAsync(&total, R.toff + ntiles, sizeof total, cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        cudaFree(buf);
-        return SPH_ERR_CUDA;
-    }
+    if (e != cudaSuccess) return SPH_ERR_CUDA;
+    // the tile lists: behind the rest where there is room
     uint32_t *list = nullptr;
-    if (cudaMalloc((void **)&list, sizeof(uint32_t) * (total ? total : 1)) != cudaSuccess) {
-        cudaFree(buf);
-        return SPH_ERR_NOMEM;
+    const size_t off_list = (bytes + 255) & ~(size_t)255;
+    if (off_list + sizeof(uint32_t) * (size_t)total <= buf_bytes) {
+        R.tlist = (uint32_t *)(buf + off_list);
+    } else {
+        if (cudaMalloc((void **)&list, sizeof(uint32_t) * (total ? total : 1)) != cudaSuccess)
+            return SPH_ERR_NOMEM;
+        R.tlist = list;
     }
-    R.tlist = list;
     if (np) {
         k_rt_bin<true><<<gb, 256, 0, st>>>(R);
         ++launches;
@@ -388,7 +395,6 @@ int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L,
     e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     cudaFree(list);
-    cudaFree(buf);
     if (stats) {
         stats->tiles = ntiles;
         stats->entries = total;

@@ -279,15 +279,19 @@ class Stepper(object):
 
     def overlaps(self, box=0):
         """(pairs [n, 2] uint32, delta_n [n]) of box `box` (sph_overlaps)."""
+        # one call where the pairs fit the room made for them (touched pages
+        # only cost memory), a second one with the number known where not
         n = C.c_uint64(0)
-        self._check(self.lib.sph_overlaps(self.h, int(box), 0, None, None, C.byref(n)),
-                    "sph_overlaps")
-        m = int(n.value)
-        pairs = numpy.zeros((max(m, 1), 2), dtype=numpy.uint32)
-        d = numpy.zeros(max(m, 1))
-        if m:
-            self._check(self.lib.sph_overlaps(self.h, int(box), m, _abi.uptr(pairs), _abi.dptr(d),
-                                              C.byref(n)), "sph_overlaps")
+        room = 8 * max(int(self.np[box]) if 0 <= int(box) < len(self.np) else 0, 1)
+        while True:
+            pairs = numpy.zeros((room, 2), dtype=numpy.uint32)
+            d = numpy.zeros(room)
+            self._check(self.lib.sph_overlaps(self.h, int(box), room, _abi.uptr(pairs),
+                                              _abi.dptr(d), C.byref(n)), "sph_overlaps")
+            m = int(n.value)
+            if m <= room:
+                break
+            room = m
         return pairs[:m], d[:m]
 
     def render(self, box=0, method=1, maxval=1.0e3, lower_cutoff=0.0, width=800, height=800,
