@@ -76,7 +76,8 @@ struct DevBox {
 struct BoxConst {
     SphParams P;
     double origo[3], L[3];
-    double dt;
+    double dt, inv_dt;          // 1 / dt
+    double cell_rate[3];        // num / L
     uint32_t num[3];
     int32_t periodic;
     uint32_t nw;
@@ -90,8 +91,10 @@ inline BoxConst box_const(const DevBox &B)
         c.origo[k] = B.origo[k];
         c.L[k] = B.L[k];
         c.num[k] = B.num[k];
+        c.cell_rate[k] = (double)B.num[k] / B.L[k];
     }
     c.dt = B.dt;
+    c.inv_dt = 1.0 / B.dt;
     c.periodic = B.periodic;
     c.nw = B.nw;
     c.cell_base = B.cell_base;
@@ -122,7 +125,8 @@ __device__ __forceinline__ d3 muls(d3 a, double s) { return mk(a.x * s, a.y * s,
 struct Divisor {
     double b, r;
     bool ok;
-    __device__ __forceinline__ explicit Divisor(double b_) : b(b_), r(1.0 / b_)
+    __device__ __forceinline__ explicit Divisor(double b_) : Divisor(b_, 1.0 / b_) {}
+    __device__ __forceinline__ Divisor(double b_, double r_) : b(b_), r(r_)
     {
         ok = fabs(r) > 0x1p-1000 && fabs(r) < 0x1p+1000;
     }
@@ -136,6 +140,8 @@ struct Divisor {
         return a / b;
     }
 };
+__device__ __forceinline__ Divisor divisor_dt(const DevBox &B) { return Divisor(B.dt); }
+__device__ __forceinline__ Divisor divisor_dt(const BoxConst &C) { return Divisor(C.dt, C.inv_dt); }
 __device__ __forceinline__ d3 divs(d3 a, double s)
 {
     const Divisor q(s);

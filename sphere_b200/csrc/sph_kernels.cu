@@ -266,7 +266,7 @@ __global__ void k_integrate(StepArgs A)
     const uint32_t i = A.perm[a];
     const DevBox &B = A.boxes[A.box_of[i]];
     const double4 f = A.force[i], t = A.torque[i];
-    integrate_particle(A, B, B, i, A.xs[a], A.vs[a], A.ws[a], xyz(f), xyz(t));
+    integrate_particle(A, B, B, i, load_own(A, i), A.xs[a], A.vs[a], A.ws[a], xyz(f), xyz(t));
 }
 
 // integration.cuh:457-484 findShearStressOnFixedMovingParticles

@@ -188,21 +188,34 @@ __device__ __forceinline__ double walls_pair(const DevBox &B, const BX &C, doubl
     return w0_force;
 }
 
+// What the end of a list step reads of the sphere's own state, loaded before
+// its first store (see OwnState).
+struct PairOwn {
+    double4 vel, xyzsum;
+    float4 angpos, acc, angacc, xref;
+    double2 eacc;
+};
+__device__ __forceinline__ PairOwn load_own(const StepArgs &A, const PairArgs &P, uint32_t i)
+{
+    return PairOwn{P.vel[i], P.xyzsum[i], P.angpos[i], P.acc[i], P.angacc[i], A.xref[i], P.eacc[i]};
+}
+
 // integration.cuh:14-305 (TY3) for one sphere of the list step: FP64
 // arithmetic on the compact state; the new state goes to the [nxt] half of
 // the ping-pong arrays and to the sphere's own arrays.
 template <class BX>
 __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs &P,
                                                const DevBox &B, const BX &C, uint32_t i, uint32_t nxt,
-                                               double4 x, double4 vel, float4 wf, d3 F, d3 T)
+                                               const PairOwn &own, double4 x, float4 wf, d3 F, d3 T)
 {
     const SphParams &Pm = C.P;
     const double dt = C.dt;
-    const float4 apf = P.angpos[i];
-    double4 xyzsum = P.xyzsum[i];
+    const double4 vel = own.vel;
+    const float4 apf = own.angpos;
+    const double4 xyzsum = own.xyzsum;
     double a0[3] = {0.0, 0.0, 0.0}, w0[3] = {0.0, 0.0, 0.0};
     if (B.iter != 0) {
-        const float4 q = P.acc[i], r = P.angacc[i];
+        const float4 q = own.acc, r = own.angacc;
         a0[0] = q.x; a0[1] = q.y; a0[2] = q.z;
         w0[0] = r.x; w0[1] = r.y; w0[2] = r.z;
     }
@@ -262,7 +275,7 @@ __device__ __forceinline__ void integrate_pair(const StepArgs &A, const PairArgs
     {
         // neighbour-list validity: displacement since the list build
         // (nearest periodic image), FP32
-        const float4 r = A.xref[i];
+        const float4 r = own.xref;
         float ex = (float)xn[0] - r.x, ey = (float)xn[1] - r.y;
         const float ez = (float)xn[2] - r.z;
         if (C.periodic == 1 || C.periodic == 2) {
@@ -301,16 +314,16 @@ __device__ __forceinline__ void finish_sphere(const StepArgs &A, const PairArgs 
 {
     const double dt = C.dt;
     if (__popcll(live_new) > NC) raise_flag(A.err, SPH_ERR_NC_OVERFLOW);
+    const PairOwn own = load_own(A, P, i);
     if (live_new != live_old) P.live[ls][i] = live_new;
-    const double4 vel = P.vel[i];
-    const double w0_force = walls_pair<LM>(B, C, xa, xyz(vel), mk(wa.x, wa.y, wa.z), acc);
+    const double w0_force = walls_pair<LM>(B, C, xa, xyz(own.vel), mk(wa.x, wa.y, wa.z), acc);
     P.force[i] = make_float4((float)acc.F.x, (float)acc.F.y, (float)acc.F.z, 0.f);
     P.torque[i] = make_float4((float)acc.T.x, (float)acc.T.y, (float)acc.T.z, 0.f);
     P.epp[i] = make_float4(acc.es_dot, acc.ev_dot, acc.p, 0.f);
-    const double2 e0 = P.eacc[i];
+    const double2 e0 = own.eacc;
     P.eacc[i] = make_double2(e0.x + (double)acc.es_dot * dt, e0.y + (double)acc.ev_dot * dt);
     if (C.nw > 0) A.wf_pp[i] = w0_force;
-    integrate_pair(A, P, B, C, i, nxt, xa, vel, wa, acc.F, acc.T);
+    integrate_pair(A, P, B, C, i, nxt, own, xa, wa, acc.F, acc.T);
 }
 
 // One sphere of the list step (thread slot t of the ordering): its list
@@ -947,9 +960,9 @@ __global__ void k_pair_key(StepArgs A, PairArgs P)
     const uint32_t bx = box_index(A, i);
     const DevBox &B = A.boxes[bx];
     const double4 x = A.x[i];
-    const double f[3] = {cell_floor(x.x, B.origo[0], B.L[0], B.num[0]),
-                         cell_floor(x.y, B.origo[1], B.L[1], B.num[1]),
-                         cell_floor(x.z, B.origo[2], B.L[2], B.num[2])};
+    const double f[3] = {cell_floor(B, x.x, 0),
+                         cell_floor(B, x.y, 1),
+                         cell_floor(B, x.z, 2)};
     uint32_t c[3];
     (void)clamp_cell(B, f, c);
     const uint32_t tx = (B.num[0] + 7u) >> 3, ty = (B.num[1] + 7u) >> 3;

@@ -68,6 +68,7 @@ struct RtArgs {
     unsigned long long *maxbits;         // maxPos(), as bits of non-negative doubles
     Camera *cam;
     float4 *xf;                          // (float) centre and radius
+    float4 *ef;                          // eye - centre and |eye - centre|^2 - radius^2
     uint32_t *tcount, *toff, *tfill, *tlist;
     uint8_t *img;
 };
@@ -193,7 +194,12 @@ __global__ void __launch_bounds__(256) k_rt_bin(RtArgs R)
     if (k >= R.np) return;
     const uint32_t g = R.p0 + k;
     const double4 x = R.x[g];
-    if (FILL) R.xf[k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+    if (FILL) {
+        const float4 s = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+        const float3 ec = sub(R.cam->eye, f3(s.x, s.y, s.z));
+        R.xf[k] = s;
+        R.ef[k] = make_float4(ec.x, ec.y, ec.z, dotf(ec, ec) - s.w * s.w);
+    }
     if (R.method != 0 && R.lower_cutoff > 0.0f) {
         const float val = (float)colour_value(R, g);
         const float fixvel = (float)R.vel[g].w;
@@ -252,35 +258,69 @@ __device__ __forceinline__ float t_minus_of(float3 d, float3 ec, float r)
 // One 16 x 16 block of pixels per thread block: src/raytracer.cuh:29-56
 // (rayInitPerspective), :14-27 (imageInit), :59-144 (rayIntersectSpheres)
 // and :146-288 (rayIntersectSpheresColormap).
+//
+// Bound by the tests, hundreds of spheres deep for each pixel.  What a test
+// needs of a sphere whatever the ray (ef) is made once, and the block brings
+// its tile's entries into shared memory 256 at a time, so that a test is one
+// broadcast read, a dot product and the discriminant: RT_AFTER us for 200,000
+// spheres at 800 x 800, 978 with each thread reading index and sphere from
+// memory, one after the other.  (The row of a pixel is rounded as the
+// reference rounds it; should the pixels of a block belong to different
+// tiles, each reads its own list.)
 __global__ void __launch_bounds__(TILE * TILE) k_rt_trace(RtArgs R)
 {
+    __shared__ float4 s_ef[TILE * TILE];
+    __shared__ uint32_t s_k[TILE * TILE];
     const uint32_t i = blockIdx.x * TILE + threadIdx.x;
     const uint32_t row = blockIdx.y * TILE + threadIdx.y;
-    if (i >= R.width || row >= R.height) return;
-    const uint32_t mempos = row * R.width + i;
+    const bool inside = i < R.width && row < R.height;
+    const uint32_t mempos = inside ? row * R.width + i : blockIdx.y * TILE * R.width + blockIdx.x * TILE;
     const Camera c = *R.cam;
     const uint32_t j = (uint32_t)((int)floorf((float)mempos / R.width)) % R.width;
     const float p_u = c.imgplane.x + (c.imgplane.y - c.imgplane.x) * (i + 0.5f) / R.width;
     const float p_v = c.imgplane.z + (c.imgplane.w - c.imgplane.z) * (j + 0.5f) / R.height;
     const float3 e = c.eye;
     const float3 d = add(add(mul(-c.d, c.w), mul(p_u, c.u)), mul(p_v, c.v));
+    const float dd = dotf(d, d), fdd = 4.0f * dd;
     float tdist = 1e10f;
     uint32_t hit = 0xffffffffu;
-    const uint32_t t = (j / TILE) * R.tx + i / TILE;
-    const uint32_t q1 = R.toff[t + 1];
-    for (uint32_t q = R.toff[t]; q < q1; ++q) {
-        const uint32_t k = R.tlist[q];
-        const float4 s = R.xf[k];
-        const float3 ec = sub(e, f3(s.x, s.y, s.z));
-        const float Delta =
-            (2.0f * dotf(d, ec)) * (2.0f * dotf(d, ec)) - 4.0f * dotf(d, d) * (dotf(ec, ec) - s.w * s.w);
-        if (!(Delta > 0.0f)) continue;
-        const float at = fabsf(t_minus_of(d, ec, s.w));
+    // dotf(-d, ec) is -dotf(d, ec) to the bit
+    auto test = [&](float4 s, uint32_t k) {
+        const float de = d.x * s.x + d.y * s.y + d.z * s.z;
+        const float Delta = (2.0f * de) * (2.0f * de) - fdd * s.w;
+        if (!(Delta > 0.0f)) return;
+        const float at = fabsf((-de - sqrtf(de * de - dd * s.w)) / dd);
         if (at < tdist || (at == tdist && k < hit)) {
             tdist = at;
             hit = k;
         }
+    };
+    const uint32_t t = (j / TILE) * R.tx + i / TILE;
+    const uint32_t t0 = (blockIdx.y * TILE % R.width / TILE) * R.tx + blockIdx.x;
+    if (__syncthreads_and(!inside || t == t0)) {
+        const uint32_t q1 = R.toff[t0 + 1], tid = threadIdx.y * TILE + threadIdx.x;
+        for (uint32_t q0 = R.toff[t0]; q0 < q1; q0 += TILE * TILE) {
+            const uint32_t n = min(q1 - q0, (uint32_t)(TILE * TILE));
+            if (tid < n) {
+                const uint32_t k = R.tlist[q0 + tid];
+                s_k[tid] = k;
+                s_ef[tid] = R.ef[k];
+            }
+            __syncthreads();
+            if (inside) {
+#pragma unroll 4
+                for (uint32_t q = 0; q < n; ++q) test(s_ef[q], s_k[q]);
+            }
+            __syncthreads();
+        }
+    } else if (inside) {
+        const uint32_t q1 = R.toff[t + 1];
+        for (uint32_t q = R.toff[t]; q < q1; ++q) {
+            const uint32_t k = R.tlist[q];
+            test(R.ef[k], k);
+        }
     }
+    if (!inside) return;
     uint8_t *px = R.img + 3 * (size_t)mempos;
     if (!(tdist < 1e10f)) {
         px[0] = px[1] = px[2] = 255;   // background
@@ -315,13 +355,13 @@ __global__ void __launch_bounds__(TILE * TILE) k_rt_trace(RtArgs R)
 }  // namespace
 
 // Scratch of render_image but for the tile lists: maxbits[3] | camera | xf[np] |
-// tcount, tfill, toff[ntiles + 1].
-constexpr size_t RT_CAM = 32, RT_XF = 256;
+// ef[np] | tcount, tfill, toff[ntiles + 1].
+constexpr size_t RT_CAM = 32, RT_XF = 256;   // (xf, then ef[np])
 static size_t rt_tiles(uint32_t width) { return ((size_t)width + TILE - 1) / TILE * (((size_t)width + TILE - 1) / TILE); }
 
 size_t render_scratch(uint32_t np, uint32_t width, uint32_t)
 {
-    return RT_XF + sizeof(float4) * (size_t)np + sizeof(uint32_t) * (3 * rt_tiles(width) + 1);
+    return RT_XF + 2 * sizeof(float4) * (size_t)np + sizeof(uint32_t) * (3 * rt_tiles(width) + 1);
 }
 
 int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L, int method,
@@ -348,11 +388,12 @@ int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L,
     R.img = d_img;
     const uint32_t ntiles = R.tx * R.ty;
     static_assert(sizeof(Camera) <= RT_XF - RT_CAM, "camera slot");
-    const size_t off_t = RT_XF + sizeof(float4) * (size_t)np;
+    const size_t off_t = RT_XF + 2 * sizeof(float4) * (size_t)np;
     const size_t bytes = render_scratch(np, width, height);
     R.maxbits = (unsigned long long *)buf;
     R.cam = (Camera *)(buf + RT_CAM);
     R.xf = (float4 *)(buf + RT_XF);
+    R.ef = R.xf + np;
     R.tcount = (uint32_t *)(buf + off_t);
     R.tfill = R.tcount + ntiles;
     R.toff = R.tfill + ntiles;

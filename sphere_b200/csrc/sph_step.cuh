@@ -36,13 +36,17 @@ __device__ __forceinline__ uint32_t box_index(const StepArgs &A, uint32_t i)
 // from a product with num / L: that differs from the quotient by a few units
 // in the last place, so away from an integer (by 1e-6, with |t| < 1e9) the
 // floors are equal; else (and for NaN) the quotient itself.
-__device__ __forceinline__ double cell_floor(double x, double o, double L, uint32_t num)
+__device__ __forceinline__ double cell_rate(const DevBox &B, int d) { return (double)B.num[d] / B.L[d]; }
+__device__ __forceinline__ double cell_rate(const BoxConst &C, int d) { return C.cell_rate[d]; }
+
+template <class BX>
+__device__ __forceinline__ double cell_floor(const BX &B, double x, int k)
 {
-    const double d = x - o;
-    const double t = d * ((double)num / L);
+    const double d = x - B.origo[k];
+    const double t = d * cell_rate(B, k);
     const double f = floor(t);
     if (fabs(t) < 1e9 && fabs((t - f) - 0.5) < 0.5 - 1e-6) return f;
-    return floor(d / (L / num));
+    return floor(d / (B.L[k] / B.num[k]));
 }
 
 // Clamped cell coordinates of a position, as the sort stores them, from its
@@ -62,17 +66,38 @@ __device__ __forceinline__ bool clamp_cell(const BX &B, const double f[3], uint3
 
 // ---------------------------------------------------------------- integrate
 
+// What the end of a step reads of the sphere's own state.  Loaded in one go
+// before the first store of the sphere's results: a load after a store waits
+// for the loads before it, since the compiler cannot tell the arrays apart.
+struct OwnState {
+    double4 angpos, xyzsum, acc, angacc;
+    float4 xref;
+    double es, ev;
+};
+__device__ __forceinline__ OwnState load_own(const StepArgs &A, uint32_t i)
+{
+    OwnState o;
+    o.angpos = A.angpos[i];
+    o.xyzsum = A.xyzsum[i];
+    o.acc = A.acc[i];
+    o.angacc = A.angacc[i];
+    o.xref = A.xref ? A.xref[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    o.es = A.es[i];
+    o.ev = A.ev[i];
+    return o;
+}
+
 // integration.cuh:14-305 integrate (TY3) for one particle.
 // (C: the box's constants, the box itself or BoxConst.)
 template <class BX>
 __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevBox &B, const BX &C,
-                                                   uint32_t i, double4 x, double4 vel,
-                                                   double4 angvel, d3 F, d3 T)
+                                                   uint32_t i, const OwnState &own, double4 x,
+                                                   double4 vel, double4 angvel, d3 F, d3 T)
 {
     const SphParams &P = C.P;
     const double dt = C.dt;
-    const double4 angpos = A.angpos[i];
-    double4 xyzsum = A.xyzsum[i];
+    const double4 angpos = own.angpos;
+    double4 xyzsum = own.xyzsum;
     int wall0mode = 0;
     double wall0mass = 0.0;
     if (C.nw > 0) {
@@ -81,14 +106,14 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     }
     double4 acc0 = make_double4(0.0, 0.0, 0.0, 0.0), angacc0 = acc0;
     if (B.iter != 0) {
-        acc0 = A.acc[i];
-        angacc0 = A.angacc[i];
+        acc0 = own.acc;
+        angacc0 = own.angacc;
     }
     const double radius = x.w;
     const double m = 4.0 / 3.0 * PI * radius * radius * radius * P.rho;
     double acc[3], angacc[3];
     // (twelve quotients by three divisors)
-    const Divisor by_m(m), by_i(2.0 / 5.0 * m * radius * radius), by_dt(dt);
+    const Divisor by_m(m), by_i(2.0 / 5.0 * m * radius * radius), by_dt = divisor_dt(C);
     acc[0] = by_m.div(F.x) + P.g[0];
     acc[1] = by_m.div(F.y) + P.g[1];
     acc[2] = by_m.div(F.z) + P.g[2];
@@ -148,7 +173,7 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     if (A.xref) {
         // neighbour-list validity: displacement since the list build
         // (nearest periodic image), FP32
-        const float4 r = A.xref[i];
+        const float4 r = own.xref;
         float ex = (float)xn[0] - r.x, ey = (float)xn[1] - r.y;
         const float ez = (float)xn[2] - r.z;
         if (C.periodic == 1 || C.periodic == 2) {
@@ -168,7 +193,7 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
         double f[3];
         uint32_t c[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) f[d] = cell_floor(xn[d], C.origo[d], C.L[d], C.num[d]);
+        for (int d = 0; d < 3; ++d) f[d] = cell_floor(C, xn[d], d);
         (void)clamp_cell(C, f, c);
         A.cellc[i] = pack_cell(c[0], c[1], c[2]);
     }
@@ -540,15 +565,15 @@ __device__ __forceinline__ double walls_and_bonds(const StepArgs &A, const DevBo
 // The per-sphere sums of the step (contactsearch.cuh:707-724).
 template <class BX>
 __device__ __forceinline__ void store_sums(const StepArgs &A, const BX &B, uint32_t i,
-                                           const Acc &acc, double w0_force)
+                                           const OwnState &own, const Acc &acc, double w0_force)
 {
     const double dt = B.dt;
     A.force[i] = make_double4(acc.F.x, acc.F.y, acc.F.z, 0.0);
     A.torque[i] = make_double4(acc.T.x, acc.T.y, acc.T.z, 0.0);
     A.es_dot[i] = acc.es_dot;
     A.ev_dot[i] = acc.ev_dot;
-    A.es[i] += acc.es_dot * dt;
-    A.ev[i] += acc.ev_dot * dt;
+    A.es[i] = own.es + acc.es_dot * dt;
+    A.ev[i] = own.ev + acc.ev_dot * dt;
     A.p[i] = acc.p;
     if (B.nw > 0) A.wf_pp[i] = w0_force;
 
@@ -725,9 +750,10 @@ __global__ void __launch_bounds__(INTERACT_THREADS, MINB) k_interact(StepArgs A)
                                  row[(4 * q + 3) * RS]);
     }
 
-    store_sums(A, B, i, acc, w0_force);
+    const OwnState own = load_own(A, i);
+    store_sums(A, B, i, own, acc, w0_force);
 
-    if (FUSED) integrate_particle(A, B, B, i, xa, va4, wa4, acc.F, acc.T);
+    if (FUSED) integrate_particle(A, B, B, i, own, xa, va4, wa4, acc.F, acc.T);
 }
 
 // ------------------------------------------------------------ split step
@@ -758,9 +784,9 @@ template <class BX>
 __device__ __forceinline__ void position_check(const StepArgs &A, const BX &B, uint32_t i,
                                                double4 x)
 {
-    const double f[3] = {cell_floor(x.x, B.origo[0], B.L[0], B.num[0]),
-                         cell_floor(x.y, B.origo[1], B.L[1], B.num[1]),
-                         cell_floor(x.z, B.origo[2], B.L[2], B.num[2])};
+    const double f[3] = {cell_floor(B, x.x, 0),
+                         cell_floor(B, x.y, 1),
+                         cell_floor(B, x.z, 2)};
     uint32_t c[3];
     const bool inside = clamp_cell(B, f, c);
     if (!isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z)) raise_flag(A.err, SPH_ERR_NAN);
@@ -817,9 +843,9 @@ __device__ __forceinline__ uint32_t search_sphere(const StepArgs &A, uint32_t i,
         for (int q = 0; q < NC / 4; ++q) tp[q] = grow[q];
     }
     double gf[3];
-    gf[0] = cell_floor(xa.x, B.origo[0], B.L[0], B.num[0]);
-    gf[1] = cell_floor(xa.y, B.origo[1], B.L[1], B.num[1]);
-    gf[2] = cell_floor(xa.z, B.origo[2], B.L[2], B.num[2]);
+    gf[0] = cell_floor(B, xa.x, 0);
+    gf[1] = cell_floor(B, xa.y, 1);
+    gf[2] = cell_floor(B, xa.z, 2);
     const int g[3] = {(int)gf[0], (int)gf[1], (int)gf[2]};
     if (!IN_PLACE && A.lazy_sort) position_check(A, B, i, xa);
     const uint32_t *lst = A.vlist ? A.vlist + (size_t)i * VL_MAX : nullptr;
@@ -1374,9 +1400,10 @@ __device__ __forceinline__ void finish_one(const StepArgs &A, const DevBox &B, c
     const double4 va4 = A.vel[i];
     const double4 wa4 = A.angvel[i];
     Acc acc = A.csum[i];   // the contacts' sums, added in slot order
+    const OwnState own = load_own(A, i);
     const double w0_force = walls_and_bonds<LM>(A, B, C, i, xa, xyz(va4), xyz(wa4), acc);
-    store_sums(A, C, i, acc, w0_force);
-    integrate_particle(A, B, C, i, xa, va4, wa4, acc.F, acc.T);
+    store_sums(A, C, i, own, acc, w0_force);
+    integrate_particle(A, B, C, i, own, xa, va4, wa4, acc.F, acc.T);
 }
 
 template <int LM>
