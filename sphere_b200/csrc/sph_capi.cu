@@ -251,6 +251,13 @@ static int ensure_pair(SphHandle *h)
         (st = dalloc(h, &P.key_count, nkeys)) || (st = dalloc(h, &P.key_off, nkeys + 1)) ||
         (st = dalloc(h, &P.key_scan, nkeys / 4096 + 2)))
         return st;
+    {
+        std::vector<char> host(sph::pair_consts_bytes(h->nbox));
+        char *dev = nullptr;
+        if ((st = dalloc(h, &dev, host.size()))) return st;
+        sph::pair_consts(h->dbox.data(), h->nbox, P, host.data(), dev);
+        CUDA_TRY(h, cudaMemcpy(dev, host.data(), host.size(), cudaMemcpyHostToDevice));
+    }
     P.key_base = key_base;
     CUDA_TRY(h, cudaMemset(P.box_done, 0, sizeof(uint32_t) * h->nbox));
     P.nkeys = (uint32_t)nkeys;
@@ -752,6 +759,23 @@ __global__ void k_pack3(double *dst, const double4 *src, uint64_t n)
         dst[3 * i + 1] = v.y;
         dst[3 * i + 2] = v.z;
     }
+}
+
+// Bond states (xyz, w) into the host's separate arrays.
+__global__ void k_pack_bonds(const double4 *delta, const double4 *omega, uint64_t nb, double *dt,
+                             double *dn, double *ot, double *on)
+{
+    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nb) return;
+    const double4 d = delta[q], o = omega[q];
+    dt[3 * q] = d.x;
+    dt[3 * q + 1] = d.y;
+    dt[3 * q + 2] = d.z;
+    dn[q] = d.w;
+    ot[3 * q] = o.x;
+    ot[3 * q + 1] = o.y;
+    ot[3 * q + 2] = o.z;
+    on[q] = o.w;
 }
 
 // The image code of every occupied slot (sph_set_contacts): the nearest
@@ -1555,18 +1579,23 @@ static int download_from(SphHandle *h, const StepArgs &S, cudaStream_t cs, SphPa
         CUDA_TRY(h, cudaStreamSynchronize(s));
     }
     if (b && nb) {
-        std::vector<uint2> pairs(nb);
-        std::vector<double4> dl(nb), om(nb);
-        CUDA_TRY(h, d2h(pairs.data(), S.bonds, sizeof(uint2) * nb));
-        CUDA_TRY(h, d2h(dl.data(), S.bdelta, sizeof(double4) * nb));
-        CUDA_TRY(h, d2h(om.data(), S.bomega, sizeof(double4) * nb));
-        for (uint64_t q = 0; q < nb; ++q) {
-            if (b->pairs) { b->pairs[2 * q] = pairs[q].x; b->pairs[2 * q + 1] = pairs[q].y; }
-            if (b->delta_n) b->delta_n[q] = dl[q].w;
-            if (b->delta_t) { b->delta_t[3 * q] = dl[q].x; b->delta_t[3 * q + 1] = dl[q].y; b->delta_t[3 * q + 2] = dl[q].z; }
-            if (b->omega_n) b->omega_n[q] = om[q].w;
-            if (b->omega_t) { b->omega_t[3 * q] = om[q].x; b->omega_t[3 * q + 1] = om[q].y; b->omega_t[3 * q + 2] = om[q].z; }
-        }
+        // repacked on the device, then copied to the caller's arrays
+        const cudaStream_t s = cs ? cs : h->stream;
+        double *buf = (double *)scratch_mem(h, 8 * sizeof(double) * nb);
+        if (!buf) return fail(h, SPH_ERR_NOMEM, "bond staging");
+        double *dt = buf, *ot = dt + 3 * nb, *dn = ot + 3 * nb, *on = dn + nb;
+        k_pack_bonds<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(S.bdelta, S.bomega, nb, dt, dn, ot, on);
+        CUDA_TRY(h, cudaGetLastError());
+        auto get = [&](void *dst, const void *src, size_t bytes) {
+            return dst ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s) : cudaSuccess;
+        };
+        cudaError_t e = get(b->pairs, S.bonds, sizeof(uint2) * nb);
+        if (e == cudaSuccess) e = get(b->delta_n, dn, sizeof(double) * nb);
+        if (e == cudaSuccess) e = get(b->delta_t, dt, 3 * sizeof(double) * nb);
+        if (e == cudaSuccess) e = get(b->omega_n, on, sizeof(double) * nb);
+        if (e == cudaSuccess) e = get(b->omega_t, ot, 3 * sizeof(double) * nb);
+        const cudaError_t es = cudaStreamSynchronize(s);
+        CUDA_TRY(h, e != cudaSuccess ? e : es);
     }
     return SPH_OK;
 }

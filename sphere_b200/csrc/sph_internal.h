@@ -10,6 +10,8 @@
 namespace sph {
 
 struct DevBox;
+struct BoxConst;
+struct MixedParams;
 struct Acc;
 
 // Device pointers of one handle, passed by value to every step kernel.
@@ -134,6 +136,8 @@ struct PairArgs {
     uint32_t *key_count, *key_off, *key_scan;
     const uint32_t *key_base;
     uint32_t nkeys;
+    const BoxConst *box_const;   // per box what a run does not change
+    const MixedParams *mixed_params;
     uint32_t *pp, *lsel;
     uint32_t *from_rows;       // != 0: the next rebuild takes histories from A.slots / A.hist
     uint32_t *bar;             // grid-barrier words of the persistent shapes: count, generation
@@ -317,6 +321,10 @@ int launch_step_mixed(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
 // compact state and back; the number of touching list entries.
 int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg, cudaStream_t st,
                      uint64_t *launches, Prof *prof);
+// The boxes' constants (P.box_const, P.mixed_params, at dev) made in host for
+// the caller to copy.
+size_t pair_consts_bytes(uint32_t nbox);
+void pair_consts(const DevBox *boxes, uint32_t nbox, PairArgs &P, char *host, char *dev);
 int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st);
 // (all: clear the history of every free slot)
 int pair_flush(const StepArgs &A, const PairArgs &P, bool all, cudaStream_t st);

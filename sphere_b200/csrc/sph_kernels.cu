@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
     __shared__ double s_part[BOX_STAGE];
     const uint32_t b = blockIdx.x;
     if (b >= A.nboxes) return;
-    DevBox &B = A.boxes[b];
+    __shared__ DevBox B;
+    stage_box(B, A.boxes[b]);
     bool any = false;
     for (uint32_t w = 0; w < B.nw; ++w) any = any || B.wmode[w] != 0;
     double fsum = 0.0;
@@ -376,8 +377,8 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
             if (threadIdx.x == 0) fsum = ordered_sum(s_part, cnt, fsum);
         }
     }
-    if (threadIdx.x != 0) return;
-    advance_box(B, fsum);
+    if (threadIdx.x == 0) advance_box(B, fsum);
+    unstage_box(A.boxes[b], B);
 }
 
 // ------------------------------------------------------------- scene packing
@@ -401,19 +402,15 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
 // division then run over the noted ones, all lanes of a warp at work, where
 // in the candidate loop one lane of nine was (a sweep of 1e6 spheres: 1.26
 // ms with the FP64 test on every candidate, 0.70 with it on those that pass,
-// RELAX_MS with the notes).  The notes keep the cells' visit order, so the
+// 0.62 with the notes).  The notes keep the cells' visit order, so the
 // sums are those of the plain loop.  The cells of a row (dx = -1, 0, 1) are
 // neighbours in the cell order, so away from the grid's x edges a row is
 // one range of candidates.
 constexpr int RELAX_THREADS = 128;
-#ifndef RB
-#define RB 8
-#define RM 4
-#endif
-constexpr int RELAX_BATCH = RB;
+constexpr int RELAX_BATCH = 4;
 constexpr int RELAX_NOTES = 24;
 
-__global__ void __launch_bounds__(RELAX_THREADS, RM) k_relax(StepArgs A, double alpha, double z_top,
+__global__ void __launch_bounds__(RELAX_THREADS, 5) k_relax(StepArgs A, double alpha, double z_top,
                                                             unsigned long long *max_ov, bool next)
 {
     __shared__ unsigned long long s_max[RELAX_THREADS / 32];

@@ -446,16 +446,19 @@ __device__ __forceinline__ void pair_sphere(const StepArgs &A, const PairArgs &P
 
 template <int LM, int NT, int MINB, bool AHEAD = true>
 __global__ void __launch_bounds__(NT, MINB) k_pair_step(const __grid_constant__ StepArgs A,
-                                                        const __grid_constant__ PairArgs P)
+                                                        const __grid_constant__ PairArgs P,
+                                                        const BoxConst *__restrict__ Cs,
+                                                        const MixedParams *__restrict__ Ms)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.ntot) return;
     const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
-    const DevBox &B = A.boxes[box_index(A, i)];
-    pair_sphere<LM, AHEAD>(A, P, B, B, B.P, i, cur, cur ^ 1u, ls);
+    const uint32_t bx = box_index(A, i);
+    pair_sphere<LM, AHEAD>(A, P, A.boxes[bx], Cs[bx], Ms[bx], i, cur, cur ^ 1u, ls);
 }
 
-// k_pair_step of a one-box handle: the box's constants from the arguments.
+// k_pair_step of a one-box handle: the box's constants from the arguments
+// (of several boxes: from tables of them that no store can change).
 template <int LM, int NT, int MINB, bool AHEAD = true>
 __global__ void __launch_bounds__(NT, MINB) k_pair_step1(const __grid_constant__ StepArgs A,
                                                          const __grid_constant__ PairArgs P,
@@ -568,13 +571,15 @@ constexpr int GROUP_THREADS = 128;
 
 template <int LM>
 __global__ void __launch_bounds__(GROUP_THREADS, 4) k_pair_group(const __grid_constant__ StepArgs A,
-                                                                 const __grid_constant__ PairArgs P)
+                                                                 const __grid_constant__ PairArgs P,
+                                                                 const BoxConst *__restrict__ Cs,
+                                                                 const MixedParams *__restrict__ Ms)
 {
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_GROUP;
     if (t >= A.ntot) return;
     const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
-    const DevBox &B = A.boxes[box_index(A, i)];
-    pair_group<LM>(A, P, B, B, B.P, i, cur, cur ^ 1u, ls);
+    const uint32_t bx = box_index(A, i);
+    pair_group<LM>(A, P, A.boxes[bx], Cs[bx], Ms[bx], i, cur, cur ^ 1u, ls);
 }
 
 template <int LM>
@@ -759,7 +764,8 @@ __device__ __forceinline__ void chunk_sum(const StepArgs &A, const PairArgs &P, 
 __device__ __forceinline__ void box_sum_advance(const StepArgs &A, const PairArgs &P, uint32_t bx,
                                                 double *s_w)
 {
-    DevBox &B = A.boxes[bx];
+    __shared__ DevBox B;
+    stage_box(B, A.boxes[bx]);
     bool any = false;
     for (uint32_t w = 0; w < B.nw; ++w) any = any || B.wmode[w] != 0;
     uint32_t nch = 0;
@@ -767,6 +773,8 @@ __device__ __forceinline__ void box_sum_advance(const StepArgs &A, const PairArg
     const double *part = P.chunk_part + P.box_chunk0[bx];
     const double fsum = ordered_sum<PBOX_THREADS>(nch, [&](uint32_t k) { return __ldcg(part + k); }, s_w);
     if (threadIdx.x == 0) advance_box(B, fsum);
+    unstage_box(A.boxes[bx], B);
+    __syncthreads();   // before the staging of the block's next box
 }
 
 // The wall stage: a block per chunk, and the block that finishes a box's last
@@ -1188,7 +1196,7 @@ void launch_pair_step(const StepArgs &A, const PairArgs &P, const DevBox *box0, 
     if (box0)
         k_pair_step1<LM, NT, MINB, AHEAD><<<g, NT, 0, st>>>(A, P, box_const(*box0), mixed_params(box0->P));
     else
-        k_pair_step<LM, NT, MINB, AHEAD><<<g, NT, 0, st>>>(A, P);
+        k_pair_step<LM, NT, MINB, AHEAD><<<g, NT, 0, st>>>(A, P, P.box_const, P.mixed_params);
 }
 
 template <int LM>
@@ -1212,7 +1220,7 @@ void launch_pair_lm(const StepArgs &A, const PairArgs &P, const StepConfig &cfg,
             k_pair_group1<LM><<<g, GROUP_THREADS, 0, st>>>(A, P, box_const(*cfg.box0),
                                                            mixed_params(cfg.box0->P));
         else
-            k_pair_group<LM><<<g, GROUP_THREADS, 0, st>>>(A, P);
+            k_pair_group<LM><<<g, GROUP_THREADS, 0, st>>>(A, P, P.box_const, P.mixed_params);
         break;
     }
     default: launch_pair_step<LM, 128, 4, true>(A, P, cfg.box0, st); break;
@@ -1293,6 +1301,23 @@ int barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds,
     if (cudaLaunchKernelEx(&c, k_barrier_check, G, expected, rounds, d_err) != cudaSuccess)
         return SPH_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
+}
+
+size_t pair_consts_bytes(uint32_t nbox)
+{
+    return nbox * (sizeof(BoxConst) + sizeof(MixedParams));
+}
+
+void pair_consts(const DevBox *boxes, uint32_t nbox, PairArgs &P, char *host, char *dev)
+{
+    BoxConst *c = reinterpret_cast<BoxConst *>(host);
+    MixedParams *m = reinterpret_cast<MixedParams *>(host + nbox * sizeof(BoxConst));
+    for (uint32_t k = 0; k < nbox; ++k) {
+        c[k] = box_const(boxes[k]);
+        m[k] = mixed_params(boxes[k].P);
+    }
+    P.box_const = reinterpret_cast<const BoxConst *>(dev);
+    P.mixed_params = reinterpret_cast<const MixedParams *>(dev + nbox * sizeof(BoxConst));
 }
 
 int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st)

@@ -259,11 +259,16 @@ template <class... Par, class... Arg>
 inline void launch_resort(void (*kern)(Par...), uint64_t n, cudaStream_t st, Arg... args)
 {
     const size_t sm = sizeof(uint32_t) * ((size_t)VL_MAX * RESORT_THREADS + 64);
-    int dev = 0, sms = 0, per_sm = 0;
+    // (per thread and kernel: the device's answers, asked for once)
+    static thread_local int for_dev = -1, sms = 0, per_sm = 0;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RESORT_THREADS, sm);
+    if (dev != for_dev) {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RESORT_THREADS, sm);
+        for_dev = dev;
+    }
     const uint64_t need = (n + RESORT_THREADS - 1) / RESORT_THREADS;
     const uint64_t cap = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)sms;
     cudaLaunchConfig_t c = {};

@@ -213,6 +213,26 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
     A.x[i] = make_double4(xn[0], xn[1], xn[2], x.w);
 }
 
+// A box copied to shared memory by the block and back: the one thread that
+// advances it reads and writes some twenty fields, and in memory each of
+// those reads waits for the write before it (k_box_step 4.5 us at 500
+// spheres, WALL_MS with the copy).
+__device__ __forceinline__ void stage_box(DevBox &s, const DevBox &g)
+{
+    static_assert(sizeof(DevBox) % 8 == 0, "copied in 8-byte words");
+    unsigned long long *d = reinterpret_cast<unsigned long long *>(&s);
+    const unsigned long long *q = reinterpret_cast<const unsigned long long *>(&g);
+    for (uint32_t k = threadIdx.x; k < sizeof(DevBox) / 8; k += blockDim.x) d[k] = q[k];
+    __syncthreads();
+}
+__device__ __forceinline__ void unstage_box(DevBox &g, const DevBox &s)
+{
+    __syncthreads();
+    unsigned long long *d = reinterpret_cast<unsigned long long *>(&g);
+    const unsigned long long *q = reinterpret_cast<const unsigned long long *>(&s);
+    for (uint32_t k = threadIdx.x; k < sizeof(DevBox) / 8; k += blockDim.x) d[k] = q[k];
+}
+
 // integration.cuh:344-450 integrateWalls with the wall-force total fsum,
 // then the loop bookkeeping of device.cu:2536-2538, the adaptive grid of
 // device.cu:1050 and the velocity-step state of device.cu:2455-2462 for
@@ -1192,12 +1212,12 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_contacts(StepArgs A)
 // Contacts are then dealt to the warp's lanes as in k_contacts, contact f of
 // the warp found from the lanes' counts and occupied slots.
 constexpr unsigned long long LMASK_VALID = 1ull << 63;
-// Resident blocks per SM, which sets the registers: 96 or 102 a thread.  With
-// 80 (6 blocks) the FP64 laws spill 60 values: 508 us against 451 at 1e6
-// spheres.
-#ifndef TOUCH_BLOCKS
-#define TOUCH_BLOCKS 5
-#endif
+// Resident blocks per SM, which sets the registers: 4 (128 a thread) for the
+// FP64 laws, 5 (96) for the mixed ones.  us of k_touch with 6 / 5 / 4 blocks:
+// FP64, 1e6 spheres 508 / 451 / 436, 60,013 spheres 50 / 42 / 36 (60 values
+// spilled with 6, 13 with 5, none with 4); mixed, 200,000 bonded spheres 80 /
+// 78 / 84.
+constexpr int touch_blocks(bool mixed) { return mixed ? 5 : 4; }
 
 // Where touch_warp finds the constants of sphere i's box and its contact
 // parameters.
@@ -1372,7 +1392,7 @@ __device__ __forceinline__ void touch_warp(const StepArgs &A, RecSlab &S, const 
 }
 
 template <int LM, bool MIXED, int SPW>
-__global__ void __launch_bounds__(CONTACT_THREADS, TOUCH_BLOCKS) k_touch(const __grid_constant__ StepArgs A)
+__global__ void __launch_bounds__(CONTACT_THREADS, touch_blocks(MIXED)) k_touch(const __grid_constant__ StepArgs A)
 {
     __shared__ RecSlab S;
     grid_dependency_wait();
@@ -1381,7 +1401,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS, TOUCH_BLOCKS) k_touch(const _
 
 // k_touch of a one-box handle: the box's constants from the arguments.
 template <int LM, bool MIXED, int SPW>
-__global__ void __launch_bounds__(CONTACT_THREADS, TOUCH_BLOCKS) k_touch1(const __grid_constant__ StepArgs A,
+__global__ void __launch_bounds__(CONTACT_THREADS, touch_blocks(MIXED)) k_touch1(const __grid_constant__ StepArgs A,
                                                                           const __grid_constant__ BoxConst C,
                                                                           const __grid_constant__ MixedParams M)
 {
@@ -1454,11 +1474,11 @@ inline void launch_contacts_lm(const StepArgs &A, const DevBox *box0, cudaStream
                                bool pdl)
 {
     // Fewer spheres to a warp while all warps fit on the chip at once
-    // (TOUCH_BLOCKS blocks on each of 148 SMs): their contacts then take fewer
+    // (touch_blocks on each of 148 SMs): their contacts then take fewer
     // rounds, the warps run side by side.  us of k_touch with 32 / 16 / 8 / 4
     // spheres a warp: 500 spheres (FP64) 21.0 / 14.5 / 10.9 / 9.4; 60,013: 42.2 /
     // 43.9 / 46.9 / 55; 1e6: 451 / 559 / 729 / 951.
-    constexpr uint32_t WARPS = 148u * TOUCH_BLOCKS * (CONTACT_THREADS / 32);
+    constexpr uint32_t WARPS = 148u * touch_blocks(MIXED) * (CONTACT_THREADS / 32);
     if (!A.touch) launch_k(pdl, k_contacts<LM, MIXED>, grid, CONTACT_THREADS, st, A);
     else if (A.ntot <= 4u * WARPS) launch_touch<MIXED, LM, 4>(A, box0, st, pdl);
     else if (A.ntot <= 8u * WARPS) launch_touch<MIXED, LM, 8>(A, box0, st, pdl);

@@ -1,0 +1,117 @@
+"""The split step with its sort and list rebuild on demand (k_resort) and the
+search in the contact kernel (k_touch), FP64, bit for bit: against the CPU
+oracle at sphere counts around a warp's and a block's share; against the
+fused kernel (which sorts at every step) at the counts where the spheres per
+warp change, with spheres in random order; and over changes of launch
+variant, contact rows set by the caller and the sort products read in
+between.  The list step in random sphere order against the FP64 form."""
+import numpy
+import pytest
+
+import cases
+import oracle as O
+from sphere_b200 import scenes
+from sphere_b200.runner import Stepper
+from test_gpu_parity import check_same
+
+pytestmark = pytest.mark.gpu
+
+
+def _pack(n, seed=5, order="lattice"):
+    s = scenes.lattice_pack(n, seed=seed, periodic=1, nw=1, wmode=1)
+    if order == "random":
+        p = numpy.random.default_rng(seed).permutation(n)
+        for name in ("x", "radius", "vel", "angvel", "fixvel"):
+            setattr(s, name, numpy.ascontiguousarray(getattr(s, name)[p]))
+    return s
+
+
+def _stepper(s, variant, **kw):
+    st = Stepper([s], precision="fp64", **kw)
+    st.set_variant(variant)
+    st.upload()
+    return st
+
+
+def _state(st):
+    hp, _ = st.download()
+    c, h, d = st.contacts()
+    return [getattr(hp, k) for k in ("x", "vel", "angvel", "force", "torque", "es", "ev", "p")] + [c, h, d]
+
+
+def _same(a, b):
+    for u, v in zip(_state(a), _state(b)):
+        assert numpy.array_equal(u, v)
+
+
+@pytest.mark.parametrize("length", ["reference", "fp64"])
+@pytest.mark.parametrize("n", [27, 64, 65, 127, 343])
+def test_touch_step_matches_oracle(n, length):
+    s = _pack(n, order="random")
+    cpu = O.CpuRun(s, "oracle", length_mode=0 if length == "reference" else 1)
+    st = _stepper(s, 3, length=length)
+    for k in (1, 2, 40):
+        st.step(k)
+        cpu.step(k)
+        check_same(st, cpu, s)
+    st.close()
+
+
+@pytest.mark.parametrize("n", [11840, 11841, 23681, 47361])
+def test_touch_step_matches_fused_kernel(n):
+    s = _pack(n, order="random")
+    a, b = _stepper(s, 1), _stepper(s, 3)
+    for k in (1, 30):
+        a.step(k)
+        b.step(k)
+        _same(a, b)
+        for u, v in zip(a.sort_products(), b.sort_products()):
+            assert numpy.array_equal(u, v)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("name", ["fast_spheres", "periodic_xy_wall_stress", "adaptive_grid"])
+def test_variant_changes_keep_the_bits(name):
+    s, _, _ = cases.make(name)
+    a, b = _stepper(s, 1), _stepper(s, 1)
+    for variant, lists, k in ((3, 48, 7), (1, 48, 3), (3, 48, 1), (3, 3, 9), (3, 0, 2), (3, 48, 6)):
+        b.set_variant(variant)
+        b.set_neighbor_lists(lists)
+        a.step(k)
+        b.step(k)
+        _same(a, b)
+        # the rows handed back through the caller: k_touch must take them anew
+        c, h, _ = b.contacts()
+        b.set_contacts(c, h)
+        a.set_contacts(c, h)
+    a.close()
+    b.close()
+
+
+def test_list_step_in_random_order_matches_fp64_form():
+    """One step from the same state: the mixed form's force bound (1e-5), the
+    same contact sets, the caller's sphere numbering throughout."""
+    n = 3000
+    s = _pack(n, order="random")
+    a = _stepper(s, 1)
+    m = Stepper([s], precision="mixed", length="reference")
+    m.set_variant(4)
+    m.upload()
+    a.step(1)
+    m.step(1)
+    ha, hm = a.download()[0], m.download()[0]
+    assert numpy.linalg.norm(hm.force - ha.force) <= 1e-5 * numpy.linalg.norm(ha.force)
+    # a position moves by (2/3) F / m dt^2 in the step
+    m_s = 4.0 / 3.0 * numpy.pi * s.radius ** 3 * float(s.rho[0])
+    move = numpy.linalg.norm(ha.force / m_s[:, None]) * float(s.time_dt[0]) ** 2
+    assert numpy.linalg.norm(hm.x - ha.x) <= 1e-5 * move + 1e-15 * numpy.linalg.norm(ha.x)
+    ca, cm = (numpy.sort(q.contacts()[0].reshape(n, -1), axis=1) for q in (a, m))
+    assert numpy.array_equal(ca, cm)
+    cid, perm, start, _ = m.sort_products()
+    assert numpy.array_equal(numpy.sort(perm), numpy.arange(n))
+    assert (numpy.diff(cid[perm].astype(numpy.int64)) >= 0).all()
+    for u, v in zip(a.sort_products(), (cid, perm, start, _)):
+        assert numpy.array_equal(u, v)
+    a.close()
+    m.close()
