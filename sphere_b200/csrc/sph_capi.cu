@@ -603,7 +603,7 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
         (st = dalloc(h, &A.cell_count, h->ncells)) || (st = dalloc(h, &A.cell_off, h->ncells + 1)) ||
         (st = dalloc(h, &A.scan_tmp, scan_blocks + 1)) || (st = dalloc(h, &A.perm, n)) ||
         (st = dalloc(h, &A.rank, n)) || (st = dalloc(h, &A.xs, n)) || (st = dalloc(h, &A.vs, n)) ||
-        (st = dalloc(h, &A.ws, n)) || (st = dalloc(h, &A.xf, n)) ||
+        (st = dalloc(h, &A.ws, n)) || (st = dalloc(h, &A.xf, n + 8)) ||
         (st = dalloc(h, &A.slots, n * sph::NC)) ||
         (st = dalloc(h, &A.hist, n * sph::NC)) || (st = dalloc(h, &A.wf_pp, n)) ||
         (st = dalloc(h, &A.wall_partial, h->npartials)) || (st = dalloc(h, &A.tau_pp, n)) ||
@@ -2634,6 +2634,7 @@ int sph_relax(SphHandle *h, uint32_t sweeps, double alpha, double z_top, double 
         int st0 = sync_public(h);
         if (st0 != SPH_OK) return st0;
         invalidate_pair(h);   // the sweeps move the spheres in the FP64 arrays
+        h->list_use = SphHandle::LISTS_NONE;   // the sweeps' sort is the last one
     }
     uint64_t nl = 0;
     {

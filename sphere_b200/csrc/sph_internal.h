@@ -30,7 +30,9 @@ struct StepArgs {
     uint32_t *cell_id, *local_off, *cell_count, *cell_off, *scan_tmp, *perm, *rank;
     uint32_t *unsorted;        // ids by cell in arrival order (k_scatter)
     double4 *xs, *vs, *ws;     // sorted copies
-    float4 *xf;                // sorted FP32 copy of x+r for the candidate prefilter
+    // sorted FP32 copy of x+r for the candidate prefilter (room for a batch of
+    // eight candidates past the end)
+    float4 *xf;
     // contact rows: slot word = partner | image code << 28, EMPTY when free
     uint32_t *slots;
     double4 *hist;             // tangential displacement per slot (w unused)

@@ -396,18 +396,19 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
 //
 // Bound by the candidates' loads and tests: in a pack with a spread of radii
 // the 27 cells around a sphere hold about 200 candidates, of which six
-// overlap.  Each is tested in FP32 on the 16-byte copy (maybe_touching:
-// never false for an overlapping pair), RELAX_BATCH loads in flight, and
+// overlap.  Each is tested in FP32 on the 16-byte copy (as maybe_touching:
+// never negative for an overlapping pair), RELAX_BATCH loads in flight, and
 // those that pass are noted in shared memory; the FP64 test, square root and
 // division then run over the noted ones, all lanes of a warp at work, where
 // in the candidate loop one lane of nine was (a sweep of 1e6 spheres: 1.26
 // ms with the FP64 test on every candidate, 0.70 with it on those that pass,
-// 0.62 with the notes).  The notes keep the cells' visit order, so the
+// 0.62 with the notes, 0.47 with the tests of a batch as the sign bits of d^2 -
+// r^2 instead of a branch each).  The notes keep the cells' visit order, so the
 // sums are those of the plain loop.  The cells of a row (dx = -1, 0, 1) are
 // neighbours in the cell order, so away from the grid's x edges a row is
 // one range of candidates.
 constexpr int RELAX_THREADS = 128;
-constexpr int RELAX_BATCH = 4;
+constexpr int RELAX_BATCH = 8;
 constexpr int RELAX_NOTES = 24;
 
 __global__ void __launch_bounds__(RELAX_THREADS, 5) k_relax(StepArgs A, double alpha, double z_top,
@@ -449,20 +450,30 @@ __global__ void __launch_bounds__(RELAX_THREADS, 5) k_relax(StepArgs A, double a
         }
         noted = 0;
     };
-    // the candidates [b0, b1) under image (sx, sy)
+    // the candidates [b0, b1) under image (sx, sy): maybe_touching as the sign
+    // of d^2 - r^2, RELAX_BATCH bits at a time (A.xf has room for a batch past
+    // its end)
     auto range = [&](uint32_t b0, uint32_t b1, int sx, int sy) {
         const uint32_t code = shift_code(sx, sy) << CODE_SHIFT;
-        const float fsx = sx == 0 ? 0.f : (sx > 0 ? Lf0 : -Lf0);
-        const float fsy = sy == 0 ? 0.f : (sy > 0 ? Lf1 : -Lf1);
+        const float ax = xaf.x + (sx == 0 ? 0.f : (sx > 0 ? Lf0 : -Lf0));
+        const float ay = xaf.y + (sy == 0 ? 0.f : (sy > 0 ? Lf1 : -Lf1));
+        const float aw = xaf.w + margin;
         for (uint32_t b = b0; b < b1; b += RELAX_BATCH) {
+            const float4 *p = A.xf + b;
             float4 xf[RELAX_BATCH];
 #pragma unroll
-            for (int j = 0; j < RELAX_BATCH; ++j) xf[j] = A.xf[min(b + j, b1 - 1u)];
-            if (noted + RELAX_BATCH > RELAX_NOTES) push_apart();
+            for (int j = 0; j < RELAX_BATCH; ++j) xf[j] = p[j];
+            uint32_t m = 0;
 #pragma unroll
-            for (int j = 0; j < RELAX_BATCH; ++j)
-                if (b + j < b1 && maybe_touching(xaf, xf[j], fsx, fsy, margin))
-                    s_note[noted++][threadIdx.x] = (b + j) | code;
+            for (int j = 0; j < RELAX_BATCH; ++j) {
+                const float cx = ax - xf[j].x, cy = ay - xf[j].y, cz = xaf.z - xf[j].z;
+                const float rr = aw + xf[j].w;
+                const float d2 = __fmaf_rn(cz, cz, __fmaf_rn(cy, cy, cx * cx));
+                m |= (__float_as_uint(__fmaf_rn(-rr, rr, d2)) >> 31) << j;
+            }
+            m &= (1u << min(b1 - b, (uint32_t)RELAX_BATCH)) - 1u;
+            if (noted + (uint32_t)__popc(m) > RELAX_NOTES) push_apart();
+            for (; m; m &= m - 1u) s_note[noted++][threadIdx.x] = (b + (uint32_t)(__ffs(m) - 1)) | code;
         }
     };
     if (valid) {

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_step1(const __grid_constant__
 // entries in turn, PAIR_GROUP at a time, and each lane adds the round's
 // contacts to the sums in list order (shuffled from their lanes), so that
 // the sums are those of one thread.  The first lane finishes the sphere.
-// 20,011 spheres: GROUP_MS us against 22.9 of the fastest other shape; at 1e6
+// 20,011 spheres: 17.4 us against 19.2 of the fastest other shape; at 1e6
 // the idle lanes of the finish cost more than the shorter walk gives, which
 // is what the tuner finds.
 constexpr int PAIR_GROUP = 4;
@@ -761,11 +761,10 @@ __device__ __forceinline__ void chunk_sum(const StepArgs &A, const PairArgs &P, 
 
 // Box bx by the calling block: its chunks' sums in a fixed order (FP64),
 // then integrateWalls and the time bookkeeping (advance_box).
+// B: the box, staged in shared memory.
 __device__ __forceinline__ void box_sum_advance(const StepArgs &A, const PairArgs &P, uint32_t bx,
-                                                double *s_w)
+                                                DevBox &B, double *s_w)
 {
-    __shared__ DevBox B;
-    stage_box(B, A.boxes[bx]);
     bool any = false;
     for (uint32_t w = 0; w < B.nw; ++w) any = any || B.wmode[w] != 0;
     uint32_t nch = 0;
@@ -780,29 +779,34 @@ __device__ __forceinline__ void box_sum_advance(const StepArgs &A, const PairArg
 // The wall stage: a block per chunk, and the block that finishes a box's last
 // chunk advances the box; the blocks past the chunks advance the boxes that
 // have none.  Block 0 hands the ping-pong state to the next step.  One launch
-// in the place of two (3.0 and 4.4 us at 20,011 spheres).
+// in the place of two (8.0 us together at 20,011 spheres, 7.8 as one, and a
+// launch less).
 __global__ void __launch_bounds__(PBOX_THREADS) k_pair_walls(StepArgs A, PairArgs P)
 {
-    grid_dependency_wait();
     __shared__ double s_w[32];
     __shared__ bool s_last;
+    __shared__ DevBox B;
+    // The box is staged before the wait for the step kernel, which only reads
+    // it: it was last written by the wall stage before that kernel.
+    const bool chunk = blockIdx.x < P.nchunks;
+    const uint32_t bx = chunk ? P.chunk_box[blockIdx.x] : blockIdx.x - P.nchunks;
+    stage_box(B, A.boxes[bx]);
+    grid_dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *P.pp ^= 1u;
-    if (blockIdx.x >= P.nchunks) {
-        const uint32_t bx = blockIdx.x - P.nchunks;
-        if (A.boxes[bx].np == 0) box_sum_advance(A, P, bx, s_w);
+    if (!chunk) {
+        if (B.np == 0) box_sum_advance(A, P, bx, B, s_w);
         return;
     }
     chunk_sum(A, P, blockIdx.x, s_w);
-    const uint32_t bx = P.chunk_box[blockIdx.x];
     if (threadIdx.x == 0) {
-        const uint32_t nch = (A.boxes[bx].np + (1u << P.chunk_log2) - 1) >> P.chunk_log2;
+        const uint32_t nch = (B.np + (1u << P.chunk_log2) - 1) >> P.chunk_log2;
         __threadfence();
         s_last = atomicAdd(&P.box_done[bx], 1u) == nch - 1u;
         if (s_last) P.box_done[bx] = 0u;   // for the next step
         __threadfence();
     }
     __syncthreads();
-    if (s_last) box_sum_advance(A, P, bx, s_w);
+    if (s_last) box_sum_advance(A, P, bx, B, s_w);
 }
 
 // Boxes without walls: time only; block 0 hands over the ping-pong state.
@@ -811,7 +815,9 @@ __global__ void __launch_bounds__(PBOX_THREADS) k_pair_box(StepArgs A, PairArgs 
 {
     grid_dependency_wait();
     __shared__ double s_w[32];
-    box_sum_advance(A, P, blockIdx.x, s_w);
+    __shared__ DevBox B;
+    stage_box(B, A.boxes[blockIdx.x]);
+    box_sum_advance(A, P, blockIdx.x, B, s_w);
     if (blockIdx.x == 0 && threadIdx.x == 0) *P.pp ^= 1u;
 }
 
@@ -835,7 +841,11 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_persist(StepArgs A, PairArgs 
     if (!grid_barrier(G, gridDim.x, A.err)) return;
     for (uint32_t c = blockIdx.x; c < P.nchunks; c += gridDim.x) chunk_sum(A, P, c, s_w);
     if (!grid_barrier(G, gridDim.x, A.err)) return;
-    for (uint32_t bx = blockIdx.x; bx < A.nboxes; bx += gridDim.x) box_sum_advance(A, P, bx, s_w);
+    __shared__ DevBox B;
+    for (uint32_t bx = blockIdx.x; bx < A.nboxes; bx += gridDim.x) {
+        stage_box(B, A.boxes[bx]);
+        box_sum_advance(A, P, bx, B, s_w);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) *P.pp ^= 1u;
 }
 
@@ -1035,7 +1045,7 @@ __global__ void k_pair_load(StepArgs A, PairArgs P)
 // with their histories and image codes.  A free slot's history is zero by
 // construction (upload, ended contacts), so only the slots that the row
 // held and no longer holds are cleared (all: every free slot): 1 KB per sphere less to write (885
-// -> 190 us at 1e6 spheres).
+// -> 436 us at 1e6 spheres).
 __global__ void k_pair_flush(StepArgs A, PairArgs P, bool all)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;

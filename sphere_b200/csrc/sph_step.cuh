@@ -216,7 +216,7 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &A, const DevB
 // A box copied to shared memory by the block and back: the one thread that
 // advances it reads and writes some twenty fields, and in memory each of
 // those reads waits for the write before it (k_box_step 4.5 us at 500
-// spheres, WALL_MS with the copy).
+// spheres, 3.3 with the copy).
 __device__ __forceinline__ void stage_box(DevBox &s, const DevBox &g)
 {
     static_assert(sizeof(DevBox) % 8 == 0, "copied in 8-byte words");
@@ -1476,7 +1476,7 @@ inline void launch_contacts_lm(const StepArgs &A, const DevBox *box0, cudaStream
     // Fewer spheres to a warp while all warps fit on the chip at once
     // (touch_blocks on each of 148 SMs): their contacts then take fewer
     // rounds, the warps run side by side.  us of k_touch with 32 / 16 / 8 / 4
-    // spheres a warp: 500 spheres (FP64) 21.0 / 14.5 / 10.9 / 9.4; 60,013: 42.2 /
+    // spheres a warp (at five blocks per SM): 500 spheres (FP64) 21.0 / 14.5 / 10.9 / 9.4; 60,013: 42.2 /
     // 43.9 / 46.9 / 55; 1e6: 451 / 559 / 729 / 951.
     constexpr uint32_t WARPS = 148u * touch_blocks(MIXED) * (CONTACT_THREADS / 32);
     if (!A.touch) launch_k(pdl, k_contacts<LM, MIXED>, grid, CONTACT_THREADS, st, A);
