@@ -306,7 +306,9 @@ int sph_neighbor_stats(SphHandle *h, uint64_t *stats);
  * (contact search, one thread per contact for the contact laws, one thread
  * per sphere for the sums and integration), for contact models 2 and 3
  * with neighbour lists on, which allocates 332 B per sphere when first
- * chosen.  Variants 0-3 have the same arithmetic and results.
+ * chosen.  Variants 0-3 have the same arithmetic: the same bits in the FP64
+ * form, compiled without FMA contraction; in the mixed form, compiled with
+ * it, each within the form's stated error.
  * 4 = the list step of the FP32-mixed form (SPH_PREC_MIXED only; contact
  * models 2 and 3, neighbour lists on, no bonds, no shear-stress wall, no
  * adaptive grid; other handles run variant 1 when it is chosen): the
@@ -321,7 +323,9 @@ int sph_neighbor_stats(SphHandle *h, uint64_t *stats);
  * sph_autotune times `steps` steps with each applicable variant from the
  * current state, keeps the fastest for this handle and puts the state back
  * as it was (ms_per_step[SPH_TUNE_VARIANTS] may be NULL; -1 for a variant
- * not tried).  sph_set_variant picks one directly.  Default 1. */
+ * not tried).  sph_set_variant picks one directly.  Without either the
+ * FP64 form runs variant 3 where that can run and variant 1 elsewhere, the
+ * mixed form variant 1. */
 #define SPH_TUNE_VARIANTS 5
 int sph_autotune(SphHandle *h, uint32_t steps, double *ms_per_step, int *chosen);
 int sph_set_variant(SphHandle *h, int variant);

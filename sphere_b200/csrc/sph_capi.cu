@@ -1001,13 +1001,17 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
     // the caller's buffers are read only during the call
     CUDA_TRY(h, cudaStreamSynchronize(cs));
     h->uploaded = true;
-    // Unless a variant was chosen: the split step wherever it can run.  It
-    // gives the fused kernel's bits at every size and is faster at every
-    // size measured, since no thread walks a sphere's contacts one after the
-    // other (us a step, fused / split, shear pack, FP64: 500 spheres 66 / 45,
-    // 10,000 125 / 56, 60,000 181 / 80, 200,000 361 / 167; without contacts,
-    // 10,000 settling: 33 / 22).
-    if (!h->variant_set && n > 0 && h->cfg.all_cm23 && !h->cfg.unfused && A.vlist &&
+    // Unless a variant was chosen: in the FP64 form the split step wherever it
+    // can run.  It gives the fused kernel's bits at every size and is faster at
+    // every size measured, since no thread walks a sphere's contacts one after
+    // the other (us a step, fused / split, shear pack, FP64: 500 spheres 66 /
+    // 45, 10,000 125 / 56, 60,000 181 / 80, 200,000 361 / 167; without
+    // contacts, 10,000 settling: 33 / 22).  The mixed form stays with the fused
+    // kernel: its file is compiled with FMA contraction, which the two kernels
+    // need not fuse alike, and with lengths rounded to 32 bits a last bit moves
+    // a force by a tenth (100 steps: forces differ by 2e-4 at 5,000 spheres, by
+    // 6e-3 in an ensemble).
+    if (!h->variant_set && h->precision == SPH_PREC_FP64 && n > 0 && h->cfg.all_cm23 && !h->cfg.unfused && A.vlist &&
         h->cfg.variant != sph::SPLIT_VARIANT && ensure_split(h) == SPH_OK) {
         h->cfg.variant = sph::SPLIT_VARIANT;
         return drop_graphs(h);

@@ -4,7 +4,9 @@ oracle at sphere counts around a warp's and a block's share; against the
 fused kernel (which sorts at every step) at the counts where the spheres per
 warp change, with spheres in random order; and over changes of launch
 variant, contact rows set by the caller and the sort products read in
-between.  The list step in random sphere order against the FP64 form."""
+between.  The list step in random sphere order against the FP64 form.  What
+a handle runs that chooses no variant: the split step in the FP64 form, the
+fused kernel, bit for bit, in the mixed form."""
 import numpy
 import pytest
 
@@ -115,3 +117,22 @@ def test_list_step_in_random_order_matches_fp64_form():
         assert numpy.array_equal(u, v)
     a.close()
     m.close()
+
+
+@pytest.mark.parametrize("length", ["reference", "fp64"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_default_variant_keeps_the_fused_kernel_bits(precision, length):
+    """Against variant 1 over 60 steps of a pack in contact and of a bonded
+    one.  In the mixed form the split step's contractions need not be the
+    fused kernel's, so only the fused kernel itself gives its bits."""
+    bonded = scenes.bonded_pack(2000, nbonds=3000, seed=1, device=0)
+    for s in (_pack(3000, order="random"), bonded):
+        a, b = (Stepper([s], precision=precision, length=length) for _ in range(2))
+        a.set_variant(1)
+        for st in (a, b):
+            st.upload()
+            st.step(60)
+        assert b.tuning()[0] == (3 if precision == "fp64" else 1)
+        _same(a, b)
+        a.close()
+        b.close()
