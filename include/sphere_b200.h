@@ -323,7 +323,9 @@ int sph_neighbor_stats(SphHandle *h, uint64_t *stats);
  * sph_autotune times `steps` steps with each applicable variant from the
  * current state, keeps the fastest for this handle and puts the state back
  * as it was (ms_per_step[SPH_TUNE_VARIANTS] may be NULL; -1 for a variant
- * not tried).  sph_set_variant picks one directly.  Without either the
+ * not tried).  Variant 4, where it can run, gives way only to a variant
+ * that is faster by a quarter, so that a handle's results do not hang on
+ * the scatter of the timings.  sph_set_variant picks one directly.  Without either the
  * FP64 form runs variant 3 where that can run and variant 1 elsewhere, the
  * mixed form variant 1. */
 #define SPH_TUNE_VARIANTS 5

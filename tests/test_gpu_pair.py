@@ -170,6 +170,25 @@ def test_pair_hands_state_to_the_split_step_and_back():
     st.close()
 
 
+@pytest.mark.parametrize("n", [700, 3000])
+def test_tuner_keeps_the_list_step_where_the_split_step_is_as_fast(n):
+    """Small packs, where the list step and the split step take the same time
+    to the resolution of the events: every tuning ends at the list step, so
+    that tuned runs repeat to the bit."""
+    s = scenes.sheared_dense_pack(n, seed=0, device=0)
+    out = []
+    for _ in range(6):
+        st = Stepper([copy.deepcopy(s)], precision="mixed")
+        st.upload()
+        st.autotune(steps=5)
+        assert st.tuning()[0] == PAIR
+        st.step(20)
+        out.append(st.download()[0])
+        st.close()
+    for o in out[1:]:
+        assert numpy.array_equal(o.x, out[0].x) and numpy.array_equal(o.force, out[0].force)
+
+
 def test_pair_ensemble_box_by_box():
     sims = scenes.shear_ensemble(nboxes=6, seed=2, device=0, counts=(300, 3000), sweeps=400)
     a = Stepper(sims, precision="fp64")
