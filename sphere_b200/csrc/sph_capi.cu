@@ -58,6 +58,8 @@ struct SphHandle {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint64_t launches_per_step = 0;
+    // what the captured graphs took from the state (step_key)
+    uint32_t graph_key = 0;
     uint64_t launches = 0;
     // the last sph_autotune's time per step of the list step at each launch
     // shape (-1: not tried)
@@ -323,6 +325,14 @@ static StepConfig step_config(const SphHandle *h)
     }
     cfg.touch = cfg.touch && cfg.lazy_sort;
     return cfg;
+}
+
+// What a captured step takes from the uploaded state besides its arguments:
+// an upload with other radii changes it (and the first upload does).
+static uint32_t step_key(const SphHandle *h)
+{
+    const StepConfig cfg = step_config(h);
+    return (cfg.lazy_sort ? 1u : 0u) | (cfg.touch ? 2u : 0u) | (pair_active(h) ? 4u : 0u);
 }
 
 // The next steps use the lists as `use` says: the list step keeps lists of
@@ -1056,8 +1066,17 @@ static int capture_step(SphHandle *h, sph::Prof *prof, cudaGraph_t *g, cudaGraph
     return SPH_OK;
 }
 
+// The step graph for the state as it is now; the graphs of another step key
+// are dropped first (every path to a captured step comes through here).
 static int build_graph(SphHandle *h)
 {
+    const uint32_t key = step_key(h);
+    if (key != h->graph_key) {
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        h->graph_key = key;
+        const int st = drop_graphs(h);
+        if (st != SPH_OK) return st;
+    }
     if (h->gexec) return SPH_OK;
     uint64_t nl = 0;
     int st = capture_step(h, nullptr, &h->graph, &h->gexec, &nl);
@@ -2296,6 +2315,9 @@ static int ensure_split(SphHandle *h)
     if ((st = dalloc(h, &lent, n * sph::NC)) || (st = dalloc(h, &nlive, n)) ||
         (st = dalloc(h, &csum, n)) || (st = dalloc(h, &h->A.lmask, n)) || (st = dalloc(h, &h->A.occ, n)))
         return st;
+    // (no sphere's row is known before the first rebuild)
+    CUDA_TRY(h, cudaMemset(h->A.lmask, 0, sizeof(unsigned long long) * (n ? n : 1)));
+    CUDA_TRY(h, cudaMemset(h->A.occ, 0, sizeof(uint32_t) * (n ? n : 1)));
     h->A.lent = lent;
     h->A.nlive = nlive;
     h->A.csum = csum;

@@ -6,7 +6,11 @@ warp change, with spheres in random order; and over changes of launch
 variant, contact rows set by the caller and the sort products read in
 between.  The list step in random sphere order against the FP64 form.  What
 a handle runs that chooses no variant: the split step in the FP64 form, the
-fused kernel, bit for bit, in the mixed form."""
+fused kernel, bit for bit, in the mixed form.  Captured steps when the state
+they were captured for changes: radii that no longer fit the cells, and
+graphs captured before there was a state."""
+import copy
+
 import numpy
 import pytest
 
@@ -136,3 +140,56 @@ def test_default_variant_keeps_the_fused_kernel_bits(precision, length):
         _same(a, b)
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("profile", [False, True])
+def test_upload_of_radii_wider_than_a_cell_on_the_same_handle(profile):
+    """k_touch asks for cells wider than the largest diameter; the second
+    upload's spheres are wider, so that pairs two cells apart overlap which
+    the +-1 cell search does not visit; the third's fit again."""
+    s = scenes.gravity_settling(400, seed=3)
+    wide = copy.deepcopy(s)
+    wide.radius = s.radius * 1.6
+    cell = numpy.asarray(s.L) / numpy.asarray(s.num)
+    assert (2.0 * s.radius.max() < cell).all() and (cell < 2.0 * wide.radius.max()).all()
+    c = numpy.floor(s.x / cell)
+    apart = numpy.abs(c[:, None] - c[None]).max(-1) > 1
+    dist = numpy.linalg.norm(s.x[:, None] - s.x[None], axis=-1)
+    assert (apart & (dist < wide.radius[:, None] + wide.radius[None])).any()
+    st = Stepper([s], precision="fp64")
+    st.set_variant(3)
+    if profile:
+        st.profile(True)
+    for q in (s, wide, s):
+        st.sims[:] = [q]
+        st.upload()
+        ref = _stepper(q, 1)
+        for k in (1, 5, 20):
+            st.step(k)
+            ref.step(k)
+            _same(ref, st)
+            for u, v in zip(ref.sort_products(), st.sort_products()):
+                assert numpy.array_equal(u, v)
+        ref.close()
+    st.close()
+
+
+@pytest.mark.parametrize("precision,variant", [("fp64", 3), ("mixed", 4)])
+def test_graphs_captured_before_the_first_upload(precision, variant):
+    """sph_profile captures its steps; before an upload these cannot be the
+    lazily sorted step or the list step, which the handle then runs."""
+    s = _pack(343)
+    out = []
+    for early in (True, False):
+        st = Stepper([s], precision=precision)
+        st.set_variant(variant)
+        if early:
+            st.profile(True)
+        st.upload()
+        st.step(2)
+        st.profile(False)
+        st.step(9)
+        out.append(_state(st))
+        st.close()
+    for u, v in zip(*out):
+        assert numpy.array_equal(u, v)
