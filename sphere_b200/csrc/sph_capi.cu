@@ -99,6 +99,9 @@ struct SphHandle {
     char *adj_snaps = nullptr;
     uint64_t adj_nsteps = 0, adj_iter0 = 0;
     uint32_t adj_ckpt = 0;
+    // its box and largest radius as uploaded for it
+    DevBox adj_box{};
+    double adj_rmax = 0.0;
     // the list step of the FP32-mixed form (launch variant 4): its compact
     // state (allocated when the variant is first chosen); pair_valid: the
     // compact arrays hold the current state; pair_ahead: the FP64 arrays
@@ -2061,6 +2064,8 @@ int sph_adjoint_forward(SphHandle *h, uint64_t nsteps, uint32_t ckpt, double *fo
     DevBox box0;
     CUDA_TRY(h, cudaMemcpy(&box0, h->A.boxes, sizeof box0, cudaMemcpyDeviceToHost));
     h->adj_iter0 = box0.iter;
+    h->adj_box = h->dbox[0];
+    h->adj_rmax = h->rmax_box[0];
     h->adj_nsteps = nsteps;
     h->adj_ckpt = ckpt;
     cudaEvent_t ev[2];
@@ -2094,6 +2099,9 @@ int sph_adjoint_backward(SphHandle *h, const double *dx_final, double *grad_para
     const uint32_t n = (uint32_t)h->ntot;
     const uint64_t nsteps = h->adj_nsteps, ckpt = h->adj_ckpt;
     const uint64_t nseg = (nsteps + ckpt - 1) / ckpt;
+    // the state becomes the forward's again, whatever was uploaded since
+    h->dbox[0] = h->adj_box;
+    h->rmax_box[0] = h->adj_rmax;
     const size_t n4 = sizeof(double4) * (n ? n : 1);
     const size_t step_tape = 3 * n4 + 2 * sizeof(uint32_t) * n * sph::NC + n4 * sph::NC;
     std::vector<void *> mine;

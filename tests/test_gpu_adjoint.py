@@ -2,7 +2,10 @@
 behind sphere_b200.adjoint.rollout) against (1) FP64 torch autograd through
 the dense restatement torch_dem.py at N = 2000, (2) central finite
 differences of the GPU forward with relative step 1e-6, (3) itself with
-other checkpoint intervals, and the state it leaves behind."""
+other checkpoint intervals, the state it leaves behind, and an upload between
+the two passes."""
+import copy
+
 import numpy
 import pytest
 import torch
@@ -145,3 +148,36 @@ def test_adjoint_rejects_unsupported_setups():
     with pytest.raises(SphereError):
         st.adjoint_forward(10, 5)
     st.close()
+
+
+def test_backward_after_an_upload_of_other_radii():
+    """The reverse pass replays the forward's steps: an upload in between,
+    with spheres that fit the cells where the forward's do not (the contact
+    search then runs in another kernel), changes neither the gradients nor
+    the steps after it.  Soft contacts, so that the wide spheres stay in the
+    box.  The gradients' sums are atomic: 1e-12."""
+    s = scenes.loose_pack(400, seed=0)
+    s.k_n[0] = s.k_t[0] = 1.0e4
+    wide, small = copy.deepcopy(s), copy.deepcopy(s)
+    wide.radius, small.radius = s.radius * 1.4, s.radius * 0.9
+    cell = numpy.asarray(s.L) / numpy.asarray(s.num)
+    assert 2.0 * small.radius.max() < cell.min() and cell.max() < 2.0 * wide.radius.max()
+    dx = numpy.random.default_rng(3).normal(0.0, 1.0, (400, 3))
+    out = []
+    for between in (False, True):
+        st = Stepper([wide], precision="fp64", length="fp64", device=DEV)
+        st.upload()
+        st.adjoint_forward(30, ckpt=10)
+        if between:
+            st.sims[:] = [small]
+            st.upload()
+        g, gv, _ = st.adjoint_backward(dx)
+        st.step(10)
+        hp, _ = st.download()
+        out.append((numpy.array([g[k] for k in ("k_n", "gamma_n", "mu")]), gv, hp))
+        st.close()
+    (ga, va, ha), (gb, vb, hb) = out
+    assert (numpy.abs(gb - ga) <= 1e-12 * numpy.abs(ga)).all()
+    assert numpy.linalg.norm(vb - va) <= 1e-12 * numpy.linalg.norm(va)
+    for name in ("x", "vel", "force"):
+        assert numpy.array_equal(getattr(ha, name), getattr(hb, name)), name
