@@ -357,13 +357,20 @@ int sph_get_shape_times(const SphHandle *h, double *ms, int n);
  * in turn, then meet at a grid-wide barrier, sum the wall forces, meet
  * again and advance the walls.  A block waits at a barrier at most 1 s; a
  * wait that runs out raises SPH_ERR_TIMEOUT (the launch ends, the device
- * stays usable, the handle needs sph_upload).  sph_barrier_check runs
+ * stays usable, the handle needs sph_upload).  The rebuilds of the
+ * neighbour lists of variants 3 and 4 are cooperative launches with such
+ * barriers too.  One that gives up leaves the state as it was before its
+ * step (downloads return that state), and every later step of these variants
+ * returns SPH_ERR_TIMEOUT without stepping until sph_upload.
+ * sph_set_rebuild_limit sets how long their blocks wait (0 .. 10 s, 1 s by
+ * default).  sph_barrier_check runs
  * `rounds` such barriers among `blocks` resident blocks of 32 threads on
  * the current device, each waiting for `expected` arrivals for at most
  * limit_s seconds: SPH_OK when they all open, SPH_ERR_TIMEOUT when
  * expected > blocks (no barrier can open; every block gives up after the
  * limit), SPH_ERR_INPUT for blocks outside 1 .. the number of SMs or a
  * limit outside (0, 10] s. */
+int sph_set_rebuild_limit(SphHandle *h, double seconds);
 int sph_barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds, double limit_s);
 
 /* Output snapshot, the output path of the reference's loop

@@ -289,6 +289,8 @@ def load_library():
     lib.sph_barrier_check.argtypes = [C.c_uint32, C.c_uint32, C.c_uint32, C.c_double]
     lib.sph_barrier_check.restype = C.c_int
     lib.sph_set_neighbor_lists.restype = C.c_int
+    lib.sph_set_rebuild_limit.argtypes = [H, C.c_double]
+    lib.sph_set_rebuild_limit.restype = C.c_int
     lib.sph_adjoint_forward.argtypes = [H, C.c_uint64, C.c_uint32, _dp]
     lib.sph_cell_offsets_static.argtypes = [C.c_void_p, C.c_uint64, C.c_void_p, C.c_void_p]
     lib.sph_cell_offsets_static.restype = C.c_int

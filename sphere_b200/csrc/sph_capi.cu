@@ -628,12 +628,13 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
         (st = dalloc(h, &bcsr_off, n + 1)) || (st = dalloc(h, &bcsr_ent, 2 * nb)) ||
         (st = dalloc(h, &A.err, 1)) || (st = dalloc(h, &h->d_count, 1)) ||
         (st = dalloc(h, &A.vlist, n * sph::VL_MAX)) || (st = dalloc(h, &A.vcount, n)) ||
-        (st = dalloc(h, &A.vflag, 3)) || (st = dalloc(h, &A.sort_bar, 2)) || (st = dalloc(h, &A.xref, n)) ||
+        (st = dalloc(h, &A.vflag, sph::VFLAGS)) || (st = dalloc(h, &A.sort_bar, 2)) || (st = dalloc(h, &A.xref, n)) ||
         (st = dalloc(h, &A.cellc, n))) {
         fprintf(stderr, "sphere_b200: %s\n", h->err.c_str());
         return bail(st);
     }
     A.vcap = sph::VL_MAX;
+    A.sort_limit_ns = sph::BARRIER_LIMIT_NS;
     h->vlist_mem = A.vlist;
     A.box_of = box_of;
     A.part_owner = part_owner;
@@ -652,7 +653,9 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
         cudaMemcpy(part_owner, hp.data(), sizeof(uint32_t) * hp.size(), cudaMemcpyHostToDevice) ||
         cudaMemcpy(bond_box, hbb.data(), sizeof(uint32_t) * hbb.size(), cudaMemcpyHostToDevice) ||
         cudaMemcpy(A.boxes, h->dbox.data(), sizeof(DevBox) * nboxes, cudaMemcpyHostToDevice) ||
-        cudaMemset(A.err, 0, sizeof(uint32_t)))
+        cudaMemset(A.err, 0, sizeof(uint32_t)) ||
+        cudaMemset(A.cell_id, 0, sizeof(uint32_t) * (n ? n : 1)) ||
+        cudaMemset(A.vcount, 0, sizeof(uint32_t) * (n ? n : 1)))
         return bail(SPH_ERR_CUDA);
     *out = h;
     return SPH_OK;
@@ -1009,7 +1012,7 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
                                 cudaMemcpyHostToDevice, cs));
     CUDA_TRY(h, cudaMemsetAsync(A.err, 0, sizeof(uint32_t), cs));
     CUDA_TRY(h, cudaMemsetAsync(A.sort_bar, 0, 2 * sizeof(uint32_t), cs));
-    CUDA_TRY(h, cudaMemsetAsync(A.vflag, 0, 3 * sizeof(uint32_t), cs));
+    CUDA_TRY(h, cudaMemsetAsync(A.vflag, 0, sph::VFLAGS * sizeof(uint32_t), cs));
     CUDA_TRY(h, cudaMemsetAsync(A.vflag, 1, 1, cs));   // build the lists in the first step
     // the caller's buffers are read only during the call
     CUDA_TRY(h, cudaStreamSynchronize(cs));
@@ -1152,9 +1155,6 @@ static int collect_errors(SphHandle *h)
     CUDA_TRY(h, cudaMemcpy(&bits, h->A.err, sizeof bits, cudaMemcpyDeviceToHost));
     CUDA_TRY(h, cudaMemset(h->A.err, 0, sizeof(uint32_t)));
     if (!bits) return SPH_OK;
-    // a rebuild that gave up left its barrier half counted
-    if (bits & (1u << SPH_ERR_TIMEOUT))
-        CUDA_TRY(h, cudaMemset(h->A.sort_bar, 0, 2 * sizeof(uint32_t)));
     static const int order[] = {SPH_ERR_TIMEOUT, SPH_ERR_NAN, SPH_ERR_OUT_OF_GRID, SPH_ERR_INPUT,
                                 SPH_ERR_NC_OVERFLOW};
     for (int code : order)
@@ -1885,6 +1885,16 @@ int sph_barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds, doubl
     cudaFree(d);
     if (st != SPH_OK) return st;
     return err & (1u << SPH_ERR_TIMEOUT) ? SPH_ERR_TIMEOUT : SPH_OK;
+}
+
+int sph_set_rebuild_limit(SphHandle *h, double seconds)
+{
+    if (!h) return SPH_ERR_INPUT;
+    if (!(seconds >= 0.0) || seconds > 10.0) return fail(h, SPH_ERR_INPUT, "limit outside 0 .. 10 s");
+    cudaSetDevice(h->device);
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    h->A.sort_limit_ns = (unsigned long long)(seconds * 1e9);
+    return drop_graphs(h);
 }
 
 uint64_t sph_total_cells(const SphHandle *h) { return h ? h->ncells : 0; }

@@ -66,6 +66,8 @@ struct DevBox {
     uint64_t iter;
     int32_t velocity_state;
     int32_t change_velocity_state;
+    // != 0: the step's rebuild gave up, its wall stage is left out (k_finish)
+    uint32_t halt, pad;
 };
 
 // What a run never changes of a box (L[2] of an adaptive grid excepted: it is

@@ -53,8 +53,14 @@ struct StepArgs {
     // coordinates of the current step (k_hash); vflag[0] != 0 requests a
     // rebuild before the next contact search, vflag[1] counts rebuilds
     // vflag[2] != 0: some sphere had no list at the last build
+    // vflag[3] != 0: a one-launch rebuild gave up at a barrier, so that its
+    // lists and its barrier words are half done; the steps that would read
+    // them return with the state as it was, until the next upload.  The wall
+    // stage of the split step hears of it from k_finish (DevBox::halt), since
+    // that of the step before may run beside the rebuild
     uint32_t *vlist, *vcount, *vflag;
     uint32_t *sort_bar;        // grid-barrier words of the one-launch rebuilds
+    unsigned long long sort_limit_ns;   // ... and how long their blocks wait
     float4 *xref;
     uint64_t *cellc;
     uint32_t vcap;             // list capacity in use (<= VL_MAX)
@@ -85,6 +91,7 @@ struct StepArgs {
 };
 
 constexpr int VL_MAX = 48;   // neighbour-list capacity per sphere
+constexpr int VFLAGS = 4;    // words of vflag (read in one go by the rebuilds)
 constexpr int INTERACT_VARIANTS = 5;   // launch variants of the interact stage (sph_autotune)
 constexpr int SPLIT_VARIANT = 3;       // the split step (k_search / k_contacts / k_finish)
 constexpr int PAIR_VARIANT = 4;        // the list step of the FP32-mixed form (sph_pair.cu)

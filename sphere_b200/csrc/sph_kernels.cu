@@ -155,10 +155,15 @@ __global__ void __launch_bounds__(RESORT_THREADS) k_resort(StepArgs A, GridSync 
 {
     extern __shared__ uint32_t s_mem[];
     uint32_t *s_scan = s_mem + VL_MAX * RESORT_THREADS;
-    const uint32_t rebuild = A.vflag[0];
-    if ((rebuild | A.vflag[2]) == 0u) return;
+    const uint4 flags = *reinterpret_cast<const uint4 *>(A.vflag);
+    const uint32_t rebuild = flags.x;
+    if ((rebuild | flags.z | flags.w) == 0u) return;
+    if (flags.w != 0u) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_flag(A.err, SPH_ERR_TIMEOUT);
+        return;
+    }
     // (sort_all's barriers lie between these reads and the writes below)
-    if (!sort_all<false>(A, G, s_scan, [&](uint32_t i) { return A.x[i]; })) return;
+    if (!sort_all<false>(A, G, s_scan, [&](uint32_t i) { return A.x[i]; })) return stop_steps(A);
     if (rebuild == 0u) return;
     uint32_t none = 0;
     for (uint32_t a = blockIdx.x * RESORT_THREADS + threadIdx.x; a < A.ntot;
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(RESORT_THREADS) k_resort(StepArgs A, GridSync 
         A.lmask[A.perm[a]] = 0ull;   // new lists: k_touch goes through the row
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) A.vflag[2] = 0u;
-    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    if (!grid_barrier(G, gridDim.x, A.err)) return stop_steps(A);
     if (none) A.vflag[2] = 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.vflag[0] = 0u;
@@ -200,6 +205,7 @@ __global__ void k_bonds(StepArgs A)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= A.nbonds) return;
+    if (A.lazy_sort && A.vflag[3] != 0u) return;
     const DevBox &B = A.boxes[A.bond_box[k]];
     const SphParams &P = B.P;
     const double dt = B.dt;
@@ -363,6 +369,7 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(StepArgs A)
     if (b >= A.nboxes) return;
     __shared__ DevBox B;
     stage_box(B, A.boxes[b]);
+    if (A.lazy_sort && B.halt) return;
     bool any = false;
     for (uint32_t w = 0; w < B.nw; ++w) any = any || B.wmode[w] != 0;
     double fsum = 0.0;

@@ -452,7 +452,9 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_step(const __grid_constant__ 
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    const uint32_t cur = *P.pp, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
+    const uint32_t i = P.order[ls][t];
     const uint32_t bx = box_index(A, i);
     pair_sphere<LM, AHEAD>(A, P, A.boxes[bx], Cs[bx], Ms[bx], i, cur, cur ^ 1u, ls);
 }
@@ -467,7 +469,9 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_step1(const __grid_constant__
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    const uint32_t cur = *P.pp, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
+    const uint32_t i = P.order[ls][t];
     pair_sphere<LM, AHEAD>(A, P, A.boxes[0], C, M, i, cur, cur ^ 1u, ls);
 }
 
@@ -577,7 +581,9 @@ __global__ void __launch_bounds__(GROUP_THREADS, 4) k_pair_group(const __grid_co
 {
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_GROUP;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    const uint32_t cur = *P.pp, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
+    const uint32_t i = P.order[ls][t];
     const uint32_t bx = box_index(A, i);
     pair_group<LM>(A, P, A.boxes[bx], Cs[bx], Ms[bx], i, cur, cur ^ 1u, ls);
 }
@@ -590,7 +596,9 @@ __global__ void __launch_bounds__(GROUP_THREADS, 4) k_pair_group1(const __grid_c
 {
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_GROUP;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp, ls = *P.lsel, i = P.order[ls][t];
+    const uint32_t cur = *P.pp, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
+    const uint32_t i = P.order[ls][t];
     pair_group<LM>(A, P, A.boxes[0], C, M, i, cur, cur ^ 1u, ls);
 }
 
@@ -634,7 +642,8 @@ __global__ void __launch_bounds__(NT, MINB) k_pair_step_async(StepArgs A, PairAr
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const int tx = (int)threadIdx.x;
     if (t >= A.ntot) return;
-    const uint32_t cur = *P.pp, nxt = cur ^ 1u, ls = *P.lsel;
+    const uint32_t cur = *P.pp, nxt = cur ^ 1u, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
     const uint32_t i = P.order[ls][t];
     const double4 *__restrict__ xr = P.xr[cur];
     const float4 *__restrict__ vw = P.vw[cur];
@@ -792,12 +801,14 @@ __global__ void __launch_bounds__(PBOX_THREADS) k_pair_walls(StepArgs A, PairArg
     const uint32_t bx = chunk ? P.chunk_box[blockIdx.x] : blockIdx.x - P.nchunks;
     stage_box(B, A.boxes[bx]);
     grid_dependency_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *P.pp ^= 1u;
+    const uint32_t stop = A.vflag[3];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !stop) *P.pp ^= 1u;
     if (!chunk) {
-        if (B.np == 0) box_sum_advance(A, P, bx, B, s_w);
+        if (B.np == 0 && !stop) box_sum_advance(A, P, bx, B, s_w);
         return;
     }
     chunk_sum(A, P, blockIdx.x, s_w);
+    if (stop) return;
     if (threadIdx.x == 0) {
         const uint32_t nch = (B.np + (1u << P.chunk_log2) - 1) >> P.chunk_log2;
         __threadfence();
@@ -816,6 +827,7 @@ __global__ void __launch_bounds__(PBOX_THREADS) k_pair_box(StepArgs A, PairArgs 
     grid_dependency_wait();
     __shared__ double s_w[32];
     __shared__ DevBox B;
+    if (A.vflag[3] != 0u) return;
     stage_box(B, A.boxes[blockIdx.x]);
     box_sum_advance(A, P, blockIdx.x, B, s_w);
     if (blockIdx.x == 0 && threadIdx.x == 0) *P.pp ^= 1u;
@@ -830,7 +842,8 @@ template <int LM, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_pair_persist(StepArgs A, PairArgs P, GridSync G)
 {
     __shared__ double s_w[32];
-    const uint32_t cur = *P.pp, nxt = cur ^ 1u, ls = *P.lsel;
+    const uint32_t cur = *P.pp, nxt = cur ^ 1u, ls = *P.lsel, stop = A.vflag[3];
+    if (stop) return;
     for (uint32_t base = blockIdx.x * NT; base < A.ntot; base += gridDim.x * NT) {
         const uint32_t t = base + threadIdx.x;
         if (t >= A.ntot) continue;
@@ -935,23 +948,28 @@ __device__ __forceinline__ void order_sphere(const StepArgs &A, const PairArgs &
 __global__ void __launch_bounds__(RESORT_THREADS) k_pair_resort(StepArgs A, PairArgs P, GridSync G)
 {
     extern __shared__ uint32_t s_mem[];
-    if (A.vflag[0] == 0u) return;
+    const uint4 flags = *reinterpret_cast<const uint4 *>(A.vflag);
+    if ((flags.x | flags.w) == 0u) return;
+    if (flags.w != 0u) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_flag(A.err, SPH_ERR_TIMEOUT);
+        return;
+    }
     const uint32_t ls = *P.lsel, nw = ls ^ 1u;
     const double4 *xr = P.xr[*P.pp];
     if (!sort_all<true>(A, G, s_mem + VL_MAX * RESORT_THREADS, [&](uint32_t i) { return xr[i]; }))
-        return;
+        return stop_steps(A);
     const uint32_t nt = gridDim.x * RESORT_THREADS, t0 = blockIdx.x * RESORT_THREADS + threadIdx.x;
     for (uint32_t a = t0; a < A.ntot; a += nt)
         vlist_build_one(A, a, s_mem + threadIdx.x, P.ids[nw], P.cnt[nw], VL_MAX, 1u, P.nrow,
                         RESORT_THREADS);
-    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    if (!grid_barrier(G, gridDim.x, A.err)) return stop_steps(A);
     for (uint32_t i = t0; i < A.ntot; i += nt) remap_sphere(A, P, i, ls);
     // RESORT_THREADS is a multiple of the group; the loop is uniform in a block
     for (uint32_t base = blockIdx.x * RESORT_THREADS; base < A.ntot; base += nt) {
         const uint32_t g = threadIdx.x / PAIR_ORDER_GROUP * PAIR_ORDER_GROUP;
         order_sphere(A, P, nw, base + g, threadIdx.x - g, s_mem + g);
     }
-    if (!grid_barrier(G, gridDim.x, A.err)) return;
+    if (!grid_barrier(G, gridDim.x, A.err)) return stop_steps(A);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *P.lsel = nw;
         *P.from_rows = 0u;
@@ -1070,6 +1088,7 @@ __global__ void k_pair_flush(StepArgs A, PairArgs P, bool all)
     A.p[i] = e.z;
     A.es[i] = ea.x;
     A.ev[i] = ea.y;
+    if (*P.from_rows) return;   // the rows were not taken over yet
     const DevBox &B = A.boxes[box_index(A, j)];
     const ListRow L(P, ls, j);
     const uint32_t nn = min(P.cnt[ls][j], (uint32_t)VL_MAX);

@@ -176,6 +176,13 @@ __device__ __forceinline__ bool vlist_build_one(const StepArgs &A, uint32_t a, u
     return true;
 }
 
+// A rebuild whose barrier gave up: the steps return as they are from here
+// on (StepArgs::vflag).
+__device__ __forceinline__ void stop_steps(const StepArgs &A)
+{
+    if (threadIdx.x == 0) A.vflag[3] = 1u;
+}
+
 // The whole sort by one cooperative launch of RESORT_THREADS-thread blocks:
 // cell ids and counts, the exclusive scan, the stable placement and the
 // sorted copies, with a grid barrier between the passes (false: a barrier
@@ -289,7 +296,7 @@ inline GridSync resort_sync(const StepArgs &A)
     GridSync G;
     G.count = A.sort_bar;
     G.gen = A.sort_bar + 1;
-    G.limit_ns = BARRIER_LIMIT_NS;
+    G.limit_ns = A.sort_limit_ns;
     return G;
 }
 

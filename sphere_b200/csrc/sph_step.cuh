@@ -66,6 +66,13 @@ __device__ __forceinline__ bool clamp_cell(const BX &B, const double f[3], uint3
 
 // ---------------------------------------------------------------- integrate
 
+// Keeps a load where it stands: a value that is used only behind a branch is
+// else loaded behind it, one memory latency after the branch's own condition.
+__device__ __forceinline__ void loaded(const double4 &v)
+{
+    asm volatile("" ::"d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w));
+}
+
 // What the end of a step reads of the sphere's own state.  Loaded in one go
 // before the first store of the sphere's results: a load after a store waits
 // for the loads before it, since the compiler cannot tell the arrays apart.
@@ -973,6 +980,7 @@ __global__ void __launch_bounds__(SEARCH_THREADS) k_search(StepArgs A)
     __shared__ uint32_t s_row[NC * SEARCH_THREADS];
     __shared__ uint16_t s_keys[VL_MAX * SEARCH_THREADS];
     grid_dependency_wait();
+    if (A.lazy_sort && A.vflag[3] != 0u) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     const int RS = SEARCH_THREADS;
@@ -1161,6 +1169,7 @@ __global__ void __launch_bounds__(CONTACT_THREADS, 6) k_contacts(StepArgs A)
 {
     __shared__ RecSlab S;
     grid_dependency_wait();
+    if (A.lazy_sort && A.vflag[3] != 0u) return;
     const uint32_t lane = threadIdx.x & 31u;
     const int wbase = (int)(threadIdx.x & ~31u);
     const uint32_t i_own = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1266,16 +1275,19 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
     uint32_t occ = A.occ[i];
     const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
     const double4 xa = A.x[i];
+    // after a rebuild that gave up: no contacts and no row is written (as a
+    // value in what follows, not as a branch ahead of the loads)
+    const bool go = A.vflag[3] == 0u;
     position_check(A, B, i, xa);
     if (A.tape_state) {
         A.tape_state[i] = xa;
         A.tape_state[A.ntot + i] = A.vel[i];
         A.tape_state[2 * (size_t)A.ntot + i] = A.angvel[i];
     }
-    if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return touch_row<LM>(A, i);
+    if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return go ? touch_row<LM>(A, i) : 0u;
     // the first entry that is not in the row and touches, and its slot word
     uint32_t found = 0, kf = 0, wf = 0;
-    for (unsigned long long todo = ((1ull << vc) - 1ull) & ~m; todo;) {
+    for (unsigned long long todo = go ? ((1ull << vc) - 1ull) & ~m : 0ull; todo;) {
         // the next KB entries' gathers in flight together
         uint32_t bo[KB], ke[KB];
         double4 xb[KB];
@@ -1334,7 +1346,7 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
             A.tape_hist[q] = A.hist[q];
         }
     }
-    return occ;
+    return go ? occ : 0u;
 }
 
 // SPW: spheres of a warp (see launch_contacts_lm).
@@ -1421,7 +1433,17 @@ __device__ __forceinline__ void finish_one(const StepArgs &A, const DevBox &B, c
     const double4 wa4 = A.angvel[i];
     Acc acc = A.csum[i];   // the contacts' sums, added in slot order
     const OwnState own = load_own(A, i);
+    const uint32_t stop = A.lazy_sort ? A.vflag[3] : 0u;
+    loaded(own.angpos);
+    loaded(own.xyzsum);
+    loaded(own.acc);
+    loaded(own.angacc);
+    asm volatile("" ::"d"(own.es), "d"(own.ev), "f"(own.xref.x), "r"(stop));
     const double w0_force = walls_and_bonds<LM>(A, B, C, i, xa, xyz(va4), xyz(wa4), acc);
+    if (stop) {   // (here, where every load ahead of the first store is under way)
+        for (uint32_t b = i; b < A.nboxes; b += A.ntot) A.boxes[b].halt = 1u;
+        return;
+    }
     store_sums(A, C, i, own, acc, w0_force);
     integrate_particle(A, B, C, i, own, xa, va4, wa4, acc.F, acc.T);
 }

@@ -268,6 +268,11 @@ class Stepper(object):
         self._check(self.lib.sph_set_neighbor_lists(self.h, int(capacity)),
                     "sph_set_neighbor_lists")
 
+    def set_rebuild_limit(self, seconds):
+        """How long the blocks of a list rebuild wait at its grid barriers
+        (default 1 s), sph_set_rebuild_limit."""
+        self._check(self.lib.sph_set_rebuild_limit(self.h, float(seconds)), "sph_set_rebuild_limit")
+
     def porosity(self, slices, box=0):
         """(z positions, porosities) of box `box` in `slices` slabs
         (sph_porosity)."""
