@@ -140,9 +140,11 @@ static int fail(SphHandle *h, int code, const std::string &msg)
 #define CUDA_TRY(h, call)                                                                   \
     do {                                                                                    \
         cudaError_t e_ = (call);                                                            \
-        if (e_ != cudaSuccess)                                                              \
+        if (e_ != cudaSuccess) {                                                            \
+            (void)cudaGetLastError();                                                       \
             return fail((h), e_ == cudaErrorMemoryAllocation ? SPH_ERR_NOMEM : SPH_ERR_CUDA, \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
+        }                                                                                   \
     } while (0)
 
 // A device array of the handle, freed with it.  Arrays up to half a chunk are
@@ -159,7 +161,7 @@ static int dalloc(SphHandle *h, T **p, uint64_t count)
     const bool own = bytes > CHUNK_BYTES / 2;
     if (own || bytes > h->chunk_left) {
         void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, own ? bytes : CHUNK_BYTES);
+        cudaError_t e = sph::dev_alloc(&q, own ? bytes : CHUNK_BYTES);
         if (e != cudaSuccess)
             return fail(h, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         h->allocs.push_back(q);
@@ -186,7 +188,7 @@ static char *scratch_mem(SphHandle *h, size_t bytes)
         h->scratch = nullptr;
         h->scratch_bytes = 0;
         void *q = nullptr;
-        if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+        if (sph::dev_alloc(&q, bytes) != cudaSuccess) return nullptr;
         h->scratch = static_cast<char *>(q);
         h->scratch_bytes = bytes;
     }
@@ -1876,7 +1878,7 @@ int sph_barrier_check(uint32_t blocks, uint32_t expected, uint32_t rounds, doubl
     if (blocks == 0 || (int)blocks > sms || !(limit_s > 0.0) || limit_s > 10.0 || expected == 0)
         return SPH_ERR_INPUT;
     uint32_t *d = nullptr;
-    if (cudaMalloc(&d, 3 * sizeof(uint32_t)) != cudaSuccess) return SPH_ERR_NOMEM;
+    if (sph::dev_alloc((void **)&d, 3 * sizeof(uint32_t)) != cudaSuccess) return SPH_ERR_NOMEM;
     int st = sph::barrier_check(blocks, expected, rounds, (unsigned long long)(limit_s * 1e9), d,
                                 d + 2, nullptr);
     uint32_t err = 0;
@@ -1914,7 +1916,7 @@ int sph_get_sort(SphHandle *h, uint32_t *cell_id, uint32_t *perm, uint32_t *cell
         StepArgs T = h->A;
         int st = SPH_OK;
         if (h->list_use == SphHandle::LISTS_PAIR) {
-            CUDA_TRY(h, cudaMalloc((void **)&ids, 4 * n));
+            CUDA_TRY(h, sph::dev_alloc((void **)&ids, 4 * n));
             st = sph::pair_public_ids(h->A, h->P, ids, h->stream);
             T.cell_id = ids;
         }
@@ -2068,7 +2070,7 @@ int sph_adjoint_forward(SphHandle *h, uint64_t nsteps, uint32_t ckpt, double *fo
     const uint64_t nseg = (nsteps + ckpt - 1) / ckpt;
     const size_t sb = state_bytes(h);
     void *q = nullptr;
-    if (cudaMalloc(&q, sb * (nseg + 1)) != cudaSuccess)
+    if (sph::dev_alloc(&q, sb * (nseg + 1)) != cudaSuccess)
         return fail(h, SPH_ERR_NOMEM, "adjoint checkpoints do not fit in device memory");
     h->adj_snaps = (char *)q;
     DevBox box0;
@@ -2117,7 +2119,7 @@ int sph_adjoint_backward(SphHandle *h, const double *dx_final, double *grad_para
     std::vector<void *> mine;
     auto get = [&](size_t bytes) -> void * {
         void *q = nullptr;
-        if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+        if (sph::dev_alloc(&q, bytes) != cudaSuccess) return nullptr;
         mine.push_back(q);
         return q;
     };
@@ -2406,7 +2408,7 @@ int sph_autotune(SphHandle *h, uint32_t steps, double *ms_per_step, int *chosen)
     }
     const size_t sb = state_bytes(h);
     char *snap = nullptr;
-    if (cudaMalloc((void **)&snap, sb) != cudaSuccess)
+    if (sph::dev_alloc((void **)&snap, sb) != cudaSuccess)
         return fail(h, SPH_ERR_NOMEM, "no device memory for the autotune snapshot");
     const std::vector<double> t_saved = h->t_host;
     const uint64_t launches_saved = h->launches;
@@ -2595,7 +2597,7 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
         if (used + 2 * half <= h->scratch_bytes) {
             O.pairs = (uint32_t *)(mem + used);
         } else {
-            if (cudaMalloc((void **)&list, 2 * half) != cudaSuccess)
+            if (sph::dev_alloc((void **)&list, 2 * half) != cudaSuccess)
                 return fail(h, SPH_ERR_NOMEM, "overlap list buffers");
             O.pairs = (uint32_t *)list;
         }

@@ -296,6 +296,18 @@ int launch_step(const StepArgs &A, const StepConfig &cfg, cudaStream_t st, uint6
 typedef void (*ContactLauncher)(const StepArgs &A, const StepConfig &cfg, cudaStream_t st,
                                 unsigned grid, bool pdl);
 
+// cudaMalloc whose failure the caller reports or does without: it leaves
+// nothing behind for the next launch check (cudaGetLastError) to find.
+inline cudaError_t dev_alloc(void **p, size_t bytes)
+{
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        (void)cudaGetLastError();
+    }
+    return e;
+}
+
 // Launch kern<<<grid, block, 0, st>>>(args...); with pdl, as a programmatic
 // dependent launch: the grid may be scheduled while the kernel before it
 // in the stream finishes, and waits (grid_dependency_wait) before reading

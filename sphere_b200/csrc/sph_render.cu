@@ -422,7 +422,7 @@ int render_image(const StepArgs &A, uint32_t p0, uint32_t np, const double *d_L,
     if (off_list + sizeof(uint32_t) * (size_t)total <= buf_bytes) {
         R.tlist = (uint32_t *)(buf + off_list);
     } else {
-        if (cudaMalloc((void **)&list, sizeof(uint32_t) * (total ? total : 1)) != cudaSuccess)
+        if (dev_alloc((void **)&list, sizeof(uint32_t) * (total ? total : 1)) != cudaSuccess)
             return SPH_ERR_NOMEM;
         R.tlist = list;
     }
