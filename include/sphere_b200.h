@@ -305,8 +305,8 @@ int sph_neighbor_stats(SphHandle *h, uint64_t *stats);
  * 80 registers per thread (different occupancy); 3 = the split step
  * (contact search, one thread per contact for the contact laws, one thread
  * per sphere for the sums and integration), for contact models 2 and 3
- * with neighbour lists on, which allocates 332 B per sphere when first
- * chosen.  Variants 0-3 have the same arithmetic: the same bits in the FP64
+ * with neighbour lists on, which allocates 84 B per sphere when first
+ * chosen, and 260 B more where a cell is no wider than the largest diameter.  Variants 0-3 have the same arithmetic: the same bits in the FP64
  * form, compiled without FMA contraction; in the mixed form, compiled with
  * it, each within the form's stated error.
  * 4 = the list step of the FP32-mixed form (SPH_PREC_MIXED only; contact

@@ -76,6 +76,7 @@ struct SphHandle {
     uint64_t pcount = 0;
     bool uploaded = false;
     bool variant_set = false;   // cfg.variant was chosen by the caller or the tuner
+    static constexpr int FUSED_VARIANT = 1;   // ... and what runs where nothing else is
     std::string err;
     std::vector<void *> allocs;
     // the chunk that small device arrays are cut from (dalloc), and scratch of
@@ -176,6 +177,24 @@ static int dalloc(SphHandle *h, T **p, uint64_t count)
     h->chunk += bytes;
     h->chunk_left -= bytes;
     return SPH_OK;
+}
+
+// Gives back what the handle allocated since the mark was taken (an array
+// that did not fit among several that are needed together).
+struct AllocMark {
+    size_t count;
+    char *chunk;
+    size_t left;
+};
+static AllocMark alloc_mark(const SphHandle *h) { return {h->allocs.size(), h->chunk, h->chunk_left}; }
+static void alloc_rewind(SphHandle *h, const AllocMark &m)
+{
+    while (h->allocs.size() > m.count) {
+        cudaFree(h->allocs.back());
+        h->allocs.pop_back();
+    }
+    h->chunk = m.chunk;
+    h->chunk_left = m.left;
 }
 
 // At least `bytes` of device scratch for one call (256-byte aligned), kept for
@@ -311,33 +330,47 @@ static void invalidate_pair(SphHandle *h)
     h->pair_ahead = false;
 }
 
-// The launch settings of a step: the split step sorts lazily unless some
-// box's grid is adaptive or some populated box cannot have neighbour lists.
-static StepConfig step_config(const SphHandle *h)
+// Whether the split step can sort lazily: no box's grid is adaptive and every
+// populated box can have neighbour lists.
+static bool lazy_fits(const SphHandle *h)
 {
-    StepConfig cfg = h->cfg;
-    cfg.box0 = h->nbox == 1 ? &h->dbox[0] : nullptr;
-    cfg.lazy_sort = h->uploaded && !pair_active(h) && sph::split_active(h->A, cfg);
-    cfg.touch = true;
+    for (uint32_t k = 0; k < h->nbox; ++k)
+        if (h->boxes[k].grid.adaptive || (h->dbox[k].np > 0 && h->dbox[k].vrange < 1)) return false;
+    return true;
+}
+
+// Whether k_touch can run: every cell wider than the largest diameter.
+static bool touch_fits(const SphHandle *h)
+{
     for (uint32_t k = 0; k < h->nbox; ++k) {
         const DevBox &d = h->dbox[k];
-        if (h->boxes[k].grid.adaptive || (d.np > 0 && d.vrange < 1)) cfg.lazy_sort = false;
         // a touching pair's distance, as the reference rounds it to FP32,
         // may exceed 2 r_max by 6e-8 of itself
         for (int c = 0; c < 3; ++c)
             if (d.np > 0 && h->uploaded && !(d.L[c] / d.num[c] > 2.0 * h->rmax_box[k] * (1.0 + 1e-6)))
-                cfg.touch = false;
+                return false;
     }
-    cfg.touch = cfg.touch && cfg.lazy_sort;
+    return true;
+}
+
+// The launch settings of a step.
+static StepConfig step_config(const SphHandle *h)
+{
+    StepConfig cfg = h->cfg;
+    cfg.box0 = h->nbox == 1 ? &h->dbox[0] : nullptr;
+    cfg.lazy_sort = h->uploaded && !pair_active(h) && sph::split_active(h->A, cfg) && lazy_fits(h);
+    cfg.touch = cfg.lazy_sort && touch_fits(h);
     return cfg;
 }
 
 // What a captured step takes from the uploaded state besides its arguments:
-// an upload with other radii changes it (and the first upload does).
+// an upload with other radii changes it (and the first upload does); with the
+// split step's lists, which such an upload may ask for.
 static uint32_t step_key(const SphHandle *h)
 {
     const StepConfig cfg = step_config(h);
-    return (cfg.lazy_sort ? 1u : 0u) | (cfg.touch ? 2u : 0u) | (pair_active(h) ? 4u : 0u);
+    return (cfg.lazy_sort ? 1u : 0u) | (cfg.touch ? 2u : 0u) | (pair_active(h) ? 4u : 0u) |
+           (h->A.lent ? 8u : 0u);
 }
 
 // The next steps use the lists as `use` says: the list step keeps lists of
@@ -1029,10 +1062,14 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
     // need not fuse alike, and with lengths rounded to 32 bits a last bit moves
     // a force by a tenth (100 steps: forces differ by 2e-4 at 5,000 spheres, by
     // 6e-3 in an ensemble).
-    if (!h->variant_set && h->precision == SPH_PREC_FP64 && n > 0 && h->cfg.all_cm23 && !h->cfg.unfused && A.vlist &&
-        h->cfg.variant != sph::SPLIT_VARIANT && ensure_split(h) == SPH_OK) {
-        h->cfg.variant = sph::SPLIT_VARIANT;
-        return drop_graphs(h);
+    // Where its buffers do not fit, the fused kernel runs.
+    if (!h->variant_set && h->precision == SPH_PREC_FP64 && n > 0 && h->cfg.all_cm23 && !h->cfg.unfused &&
+        A.vlist) {
+        const int v = ensure_split(h) == SPH_OK ? sph::SPLIT_VARIANT : SphHandle::FUSED_VARIANT;
+        if (v != h->cfg.variant) {
+            h->cfg.variant = v;
+            return drop_graphs(h);
+        }
     }
     return SPH_OK;
 }
@@ -1078,6 +1115,11 @@ static int capture_step(SphHandle *h, sph::Prof *prof, cudaGraph_t *g, cudaGraph
 // are dropped first (every path to a captured step comes through here).
 static int build_graph(SphHandle *h)
 {
+    if (h->uploaded && h->cfg.variant == sph::SPLIT_VARIANT && sph::split_active(h->A, h->cfg)) {
+        // (an upload may have brought radii that do not fit k_touch)
+        const int st = ensure_split(h);
+        if (st != SPH_OK) return st;
+    }
     const uint32_t key = step_key(h);
     if (key != h->graph_key) {
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1232,6 +1274,9 @@ static int queue_steps_now(SphHandle *h, uint64_t nsteps, uint8_t *states)
     if (nsteps == 0) return SPH_OK;
     if (h->eager) {
         // kernel by kernel on the handle's stream (no graphs)
+        if (h->cfg.variant == sph::SPLIT_VARIANT && sph::split_active(h->A, h->cfg) &&
+            (st = ensure_split(h)) != SPH_OK)
+            return st;
         if ((st = prepare_steps(h)) != SPH_OK) return st;
         const size_t bytes = sizeof(DevBox) * h->nbox;
         const StepConfig cfg = step_config(h);
@@ -2320,27 +2365,42 @@ static int drop_graphs(SphHandle *h)
     return SPH_OK;
 }
 
-// Buffers of the split step, allocated when that variant is first chosen.
+// Buffers of the split step, allocated when it is first chosen: the contacts'
+// sums and k_touch's record of the rows (84 bytes a sphere), and the lists of
+// live contacts that k_search hands to k_contacts (260 bytes) where k_touch
+// cannot run.  What was got is given back when the rest does not fit.
 static int ensure_split(SphHandle *h)
 {
-    if (h->A.csum) return SPH_OK;
     const uint64_t n = h->ntot;
+    StepArgs &A = h->A;
     // a live entry holds the sphere index in 27 bits
     if (n > (uint64_t)sph::SPLIT_ID_MASK + 1u)
         return fail(h, SPH_ERR_UNSUPPORTED, "split step: more than 2^27 spheres");
+    int st;
+    if (!A.csum) {
+        const AllocMark m = alloc_mark(h);
+        sph::Acc *csum = nullptr;
+        if ((st = dalloc(h, &csum, n)) || (st = dalloc(h, &A.lmask, n)) || (st = dalloc(h, &A.occ, n))) {
+            alloc_rewind(h, m);
+            A.lmask = nullptr;
+            A.occ = nullptr;
+            return st;
+        }
+        // (no sphere's row is known before the first rebuild)
+        CUDA_TRY(h, cudaMemset(A.lmask, 0, sizeof(unsigned long long) * (n ? n : 1)));
+        CUDA_TRY(h, cudaMemset(A.occ, 0, sizeof(uint32_t) * (n ? n : 1)));
+        A.csum = csum;
+    }
+    if (A.lent || !h->uploaded || (touch_fits(h) && lazy_fits(h))) return SPH_OK;
+    const AllocMark m = alloc_mark(h);
     uint2 *lent = nullptr;
     uint32_t *nlive = nullptr;
-    sph::Acc *csum = nullptr;
-    int st;
-    if ((st = dalloc(h, &lent, n * sph::NC)) || (st = dalloc(h, &nlive, n)) ||
-        (st = dalloc(h, &csum, n)) || (st = dalloc(h, &h->A.lmask, n)) || (st = dalloc(h, &h->A.occ, n)))
+    if ((st = dalloc(h, &lent, n * sph::NC)) || (st = dalloc(h, &nlive, n))) {
+        alloc_rewind(h, m);
         return st;
-    // (no sphere's row is known before the first rebuild)
-    CUDA_TRY(h, cudaMemset(h->A.lmask, 0, sizeof(unsigned long long) * (n ? n : 1)));
-    CUDA_TRY(h, cudaMemset(h->A.occ, 0, sizeof(uint32_t) * (n ? n : 1)));
-    h->A.lent = lent;
-    h->A.nlive = nlive;
-    h->A.csum = csum;
+    }
+    A.lent = lent;
+    A.nlive = nlive;
     return SPH_OK;
 }
 

@@ -1,7 +1,10 @@
 """Calls that find no device memory: they report it or do without, and leave
-nothing behind that a later call would take for an error of its own."""
+nothing behind that a later call would take for an error of its own.  What a
+handle allocates that it does not need."""
 import numpy
 import pytest
+
+import torch
 
 from sphere_b200 import scenes
 from sphere_b200.runner import SphereError, Stepper
@@ -24,3 +27,72 @@ def test_a_failed_allocation_is_reported_once():
     assert st.relax(1, alpha=0.1, z_top=float(s.L[2])) >= 0.0
     assert st.count_contacts() >= 0
     st.close()
+
+
+def _free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _fill():
+    """All but a few MB of the device's free memory."""
+    return torch.empty((_free() // (2 << 20) - 2) * (2 << 20), dtype=torch.uint8, device="cuda")
+
+
+def _give_back():
+    torch.cuda.empty_cache()
+
+
+def _lattice(n, **kw):
+    return scenes.lattice_pack(n, seed=1, periodic=1, nw=1, wmode=1, **kw)
+
+
+def test_split_step_buffers_by_need():
+    """The default variant's buffers, taken by the first upload with lists on:
+    84 bytes a sphere, and 260 more for spheres wider than a cell."""
+    n = 400000
+    s = _lattice(n)
+    st = Stepper([s], precision="fp64")
+    st.set_neighbor_lists(0)
+    st.upload()
+    st.set_neighbor_lists(48)
+    free = [_free()]
+    for r in (1.0, 1.15):
+        st.sims[0].radius = s.radius * r
+        st.upload()
+        assert st.tuning()[0] == 3
+        free.append(_free())
+    assert free[0] - free[1] <= 84 * n + (4 << 20)
+    assert 256 * n <= free[1] - free[2] <= 260 * n + (4 << 20)   # (the counts may fit a chunk)
+    st.close()
+
+
+def test_default_upload_without_room_for_the_split_step():
+    s = _lattice(150000)
+    ref = Stepper([s], precision="fp64")
+    ref.set_variant(1)
+    st = Stepper([s], precision="fp64")
+    st.set_neighbor_lists(0)      # no split step, so none of its buffers yet
+    for q in (ref, st):
+        q.upload()
+    ref.step(3)
+    st.set_neighbor_lists(48)
+    pad = _fill()
+    before = _free()
+    st.upload()
+    assert st.tuning()[0] == 1 and _free() == before
+    assert st.count_contacts() == 0
+    st.step(3)
+    del pad
+    _give_back()
+    out = [st.download()[0]]
+    st.upload()
+    assert st.tuning()[0] == 3
+    st.step(3)
+    out.append(st.download()[0])
+    want = ref.download()[0]
+    for o in out:
+        for name in ("x", "vel", "force"):
+            assert numpy.array_equal(getattr(o, name), getattr(want, name)), name
+    st.close()
+    ref.close()
