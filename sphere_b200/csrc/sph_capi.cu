@@ -82,7 +82,7 @@ struct SphHandle {
     // the chunk that small device arrays are cut from (dalloc), and scratch of
     // the analysis calls, kept and grown as they need it (scratch_mem)
     char *chunk = nullptr;
-    size_t chunk_left = 0;
+    size_t chunk_left = 0, chunk_bytes = 0;
     char *scratch = nullptr;
     size_t scratch_bytes = 0;
     unsigned long long *d_count = nullptr;
@@ -149,20 +149,29 @@ static int fail(SphHandle *h, int code, const std::string &msg)
     } while (0)
 
 // A device array of the handle, freed with it.  Arrays up to half a chunk are
-// cut from 16 MB chunks (256-byte aligned, as cudaMalloc's): a handle of 50,000
+// cut from chunks (256-byte aligned, as cudaMalloc's): a handle of 50,000
 // spheres makes some 70 arrays, and each allocation of its own costs about
-// 80 us to make and as much to free.
-constexpr size_t CHUNK_BYTES = 16u << 20;
+// 80 us to make and as much to free.  A chunk holds what a small handle
+// allocates in all (chunk_size), at most 16 MB, so that hundreds of small
+// handles take no more memory than their arrays.
+constexpr size_t CHUNK_MAX = 16u << 20;
+
+static size_t chunk_size(uint64_t n, uint64_t ncells, uint64_t nbonds)
+{
+    // sph_create's arrays, the staging of the uploads, the split step's sums
+    const uint64_t b = 70 * 256 + 2100 * n + 8 * ncells + 200 * nbonds;
+    return (size_t)std::min<uint64_t>((b + 0xffff) & ~0xffffull, CHUNK_MAX);
+}
 
 template <typename T>
 static int dalloc(SphHandle *h, T **p, uint64_t count)
 {
     if (count == 0) count = 1;
     const size_t bytes = (sizeof(T) * count + 255) & ~(size_t)255;
-    const bool own = bytes > CHUNK_BYTES / 2;
+    const bool own = bytes > h->chunk_bytes / 2;
     if (own || bytes > h->chunk_left) {
         void *q = nullptr;
-        cudaError_t e = sph::dev_alloc(&q, own ? bytes : CHUNK_BYTES);
+        cudaError_t e = sph::dev_alloc(&q, own ? bytes : h->chunk_bytes);
         if (e != cudaSuccess)
             return fail(h, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         h->allocs.push_back(q);
@@ -171,7 +180,7 @@ static int dalloc(SphHandle *h, T **p, uint64_t count)
             return SPH_OK;
         }
         h->chunk = static_cast<char *>(q);
-        h->chunk_left = CHUNK_BYTES;
+        h->chunk_left = h->chunk_bytes;
     }
     *p = reinterpret_cast<T *>(h->chunk);
     h->chunk += bytes;
@@ -604,6 +613,7 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
     h->ncells = cb;
     h->nbonds = bb;
     h->npartials = qb;
+    h->chunk_bytes = chunk_size(pb, cb, bb);
     if (pb >= sph::ID_MASK) return bail(SPH_ERR_UNSUPPORTED);
     if (cb >= 0xffffffffull || cb > 4096ull * 4096ull) return bail(SPH_ERR_UNSUPPORTED);
     h->cfg.lenmode = length_mode;

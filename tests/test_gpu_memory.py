@@ -96,3 +96,17 @@ def test_default_upload_without_room_for_the_split_step():
             assert numpy.array_equal(getattr(o, name), getattr(want, name)), name
     st.close()
     ref.close()
+
+
+def test_small_handles_take_little_memory():
+    """100 spheres: 0.2 MB of arrays, allocated in steps of up to 2 MB."""
+    s = _lattice(100)
+    free = _free()
+    many = []
+    for _ in range(40):
+        many.append(Stepper([s], precision="fp64"))
+        many[-1].upload()
+    assert free - _free() <= 40 * (2 << 20) + (4 << 20)
+    for st in many:
+        st.step(1)
+        st.close()
