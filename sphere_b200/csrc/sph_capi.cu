@@ -84,7 +84,7 @@ struct SphHandle {
     char *chunk = nullptr;
     size_t chunk_left = 0, chunk_bytes = 0;
     char *scratch = nullptr;
-    size_t scratch_bytes = 0;
+    size_t scratch_bytes = 0, scratch_want = 0;
     unsigned long long *d_count = nullptr;
     uint32_t *vlist_mem = nullptr;   // neighbour-list storage (A.vlist is null when off)
     std::vector<double> rmax_box;    // largest radius per box (at upload)
@@ -148,6 +148,25 @@ static int fail(SphHandle *h, int code, const std::string &msg)
         }                                                                                   \
     } while (0)
 
+static void free_scratch(SphHandle *h)
+{
+    cudaFree(h->scratch);
+    h->scratch = nullptr;
+    h->scratch_bytes = 0;
+}
+
+// Device memory for the handle, at the scratch's cost where there is no other
+// (not while a call uses the scratch).
+static cudaError_t handle_alloc(SphHandle *h, void **p, size_t bytes)
+{
+    cudaError_t e = sph::dev_alloc(p, bytes);
+    if (e != cudaSuccess && h->scratch) {
+        free_scratch(h);
+        e = sph::dev_alloc(p, bytes);
+    }
+    return e;
+}
+
 // A device array of the handle, freed with it.  Arrays up to half a chunk are
 // cut from chunks (256-byte aligned, as cudaMalloc's): a handle of 50,000
 // spheres makes some 70 arrays, and each allocation of its own costs about
@@ -171,7 +190,7 @@ static int dalloc(SphHandle *h, T **p, uint64_t count)
     const bool own = bytes > h->chunk_bytes / 2;
     if (own || bytes > h->chunk_left) {
         void *q = nullptr;
-        cudaError_t e = sph::dev_alloc(&q, own ? bytes : h->chunk_bytes);
+        cudaError_t e = handle_alloc(h, &q, own ? bytes : h->chunk_bytes);
         if (e != cudaSuccess)
             return fail(h, SPH_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         h->allocs.push_back(q);
@@ -208,14 +227,20 @@ static void alloc_rewind(SphHandle *h, const AllocMark &m)
 
 // At least `bytes` of device scratch for one call (256-byte aligned), kept for
 // the next; its contents are the caller's only until the call returns.  Null
-// when the device has no room.
+// when the device has no room.  A call that could have used more says so in
+// scratch_want, and the next one takes that much if it is to be had.
 static char *scratch_mem(SphHandle *h, size_t bytes)
 {
+    void *q = nullptr;
+    if (h->scratch_want > h->scratch_bytes && h->scratch_want >= bytes &&
+        sph::dev_alloc(&q, h->scratch_want) == cudaSuccess) {
+        free_scratch(h);
+        h->scratch = static_cast<char *>(q);
+        h->scratch_bytes = h->scratch_want;
+    }
+    h->scratch_want = 0;
     if (bytes > h->scratch_bytes) {
-        cudaFree(h->scratch);
-        h->scratch = nullptr;
-        h->scratch_bytes = 0;
-        void *q = nullptr;
+        free_scratch(h);
         if (sph::dev_alloc(&q, bytes) != cudaSuccess) return nullptr;
         h->scratch = static_cast<char *>(q);
         h->scratch_bytes = bytes;
@@ -2125,7 +2150,7 @@ int sph_adjoint_forward(SphHandle *h, uint64_t nsteps, uint32_t ckpt, double *fo
     const uint64_t nseg = (nsteps + ckpt - 1) / ckpt;
     const size_t sb = state_bytes(h);
     void *q = nullptr;
-    if (sph::dev_alloc(&q, sb * (nseg + 1)) != cudaSuccess)
+    if (handle_alloc(h, &q, sb * (nseg + 1)) != cudaSuccess)
         return fail(h, SPH_ERR_NOMEM, "adjoint checkpoints do not fit in device memory");
     h->adj_snaps = (char *)q;
     DevBox box0;
@@ -2174,7 +2199,7 @@ int sph_adjoint_backward(SphHandle *h, const double *dx_final, double *grad_para
     std::vector<void *> mine;
     auto get = [&](size_t bytes) -> void * {
         void *q = nullptr;
-        if (sph::dev_alloc(&q, bytes) != cudaSuccess) return nullptr;
+        if (handle_alloc(h, &q, bytes) != cudaSuccess) return nullptr;
         mine.push_back(q);
         return q;
     };
@@ -2478,7 +2503,7 @@ int sph_autotune(SphHandle *h, uint32_t steps, double *ms_per_step, int *chosen)
     }
     const size_t sb = state_bytes(h);
     char *snap = nullptr;
-    if (sph::dev_alloc((void **)&snap, sb) != cudaSuccess)
+    if (handle_alloc(h, (void **)&snap, sb) != cudaSuccess)
         return fail(h, SPH_ERR_NOMEM, "no device memory for the autotune snapshot");
     const std::vector<double> t_saved = h->t_host;
     const uint64_t launches_saved = h->launches;
@@ -2682,9 +2707,8 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
     }
     if (list) {
         // room for as many pairs in the next call
-        const size_t want = used + 2 * ((8 * (size_t)total + 255) & ~(size_t)255);
+        h->scratch_want = used + 2 * ((8 * (size_t)total + 255) & ~(size_t)255);
         cudaFree(list);
-        (void)scratch_mem(h, want);
     }
     if (st != SPH_OK) return fail(h, st, "overlap-search launch failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
@@ -2727,7 +2751,7 @@ int sph_render(SphHandle *h, uint32_t box, int method, float maxval, float lower
     if (st == SPH_OK) e = cudaMemcpy(rgb, img, bytes, cudaMemcpyDeviceToHost);
     // room for as many tile-list entries in the next call
     const size_t want = img_bytes + rt_bytes + 256 + sizeof(uint32_t) * (size_t)rs.entries;
-    if (st == SPH_OK && e == cudaSuccess && want > h->scratch_bytes) (void)scratch_mem(h, want);
+    if (st == SPH_OK && e == cudaSuccess && want > h->scratch_bytes) h->scratch_want = want;
     if (st != SPH_OK) return fail(h, st, "ray-tracing kernels failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     return SPH_OK;

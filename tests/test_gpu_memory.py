@@ -110,3 +110,18 @@ def test_small_handles_take_little_memory():
     for st in many:
         st.step(1)
         st.close()
+
+
+def test_scratch_of_an_analysis_call_gives_way():
+    """The image buffer kept from a large image (27 MB) is given back when
+    the tuner's state snapshot, 15 MB, finds no other room."""
+    s = _lattice(10000)
+    st = Stepper([s], precision="fp64")
+    st.upload()
+    img = st.render(width=3000, height=3000)
+    pad = _fill()
+    st.autotune(steps=1)
+    del pad
+    _give_back()
+    assert numpy.array_equal(st.render(width=3000, height=3000), img)
+    st.close()
