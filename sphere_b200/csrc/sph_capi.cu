@@ -1690,7 +1690,26 @@ static int download_from(SphHandle *h, const StepArgs &S, cudaStream_t cs, SphPa
         // repacked on the device, then copied to the caller's arrays
         const cudaStream_t s = cs ? cs : h->stream;
         double *buf = (double *)scratch_mem(h, 8 * sizeof(double) * nb);
-        if (!buf) return fail(h, SPH_ERR_NOMEM, "bond staging");
+        if (!buf) {
+            // no room for that: repacked here
+            std::vector<double4> dl(nb), om(nb);
+            if (b->pairs) CUDA_TRY(h, d2h(b->pairs, S.bonds, sizeof(uint2) * nb));
+            CUDA_TRY(h, d2h(dl.data(), S.bdelta, sizeof(double4) * nb));
+            CUDA_TRY(h, d2h(om.data(), S.bomega, sizeof(double4) * nb));
+            auto split = [nb](const std::vector<double4> &v, double *xyz, double *w) {
+                for (uint64_t q = 0; q < nb; ++q) {
+                    if (xyz) {
+                        xyz[3 * q] = v[q].x;
+                        xyz[3 * q + 1] = v[q].y;
+                        xyz[3 * q + 2] = v[q].z;
+                    }
+                    if (w) w[q] = v[q].w;
+                }
+            };
+            split(dl, b->delta_t, b->delta_n);
+            split(om, b->omega_t, b->omega_n);
+            return SPH_OK;
+        }
         double *dt = buf, *ot = dt + 3 * nb, *dn = ot + 3 * nb, *on = dn + nb;
         k_pack_bonds<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(S.bdelta, S.bomega, nb, dt, dn, ot, on);
         CUDA_TRY(h, cudaGetLastError());

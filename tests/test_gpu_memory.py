@@ -125,3 +125,20 @@ def test_scratch_of_an_analysis_call_gives_way():
     _give_back()
     assert numpy.array_equal(st.render(width=3000, height=3000), img)
     st.close()
+
+
+def test_bonds_come_back_from_a_full_device():
+    s = scenes.bonded_pack(200000, nbonds=300000, seed=0, device=0)
+    out = []
+    for full in (False, True):
+        st = Stepper([s], precision="fp64")
+        st.upload()
+        st.step(3)
+        pad = _fill() if full else None
+        out.append(st.download()[1])     # 19 MB of staging on the device
+        del pad
+        _give_back()
+        st.close()
+    a, b = out
+    for name in ("pairs", "delta_n", "delta_t", "omega_n", "omega_t"):
+        assert getattr(a, name).any() and numpy.array_equal(getattr(a, name), getattr(b, name)), name
