@@ -2010,19 +2010,17 @@ int sph_get_sort(SphHandle *h, uint32_t *cell_id, uint32_t *perm, uint32_t *cell
     // the lazily sorted split step keeps each step's cell ids; the order
     // that follows from them is made here
     // (of the last rebuild after list steps, from that step's numbering)
-    uint32_t *ids = nullptr;
     if (n && (h->list_use == SphHandle::LISTS_LAZY || h->list_use == SphHandle::LISTS_PAIR)) {
         StepArgs T = h->A;
         int st = SPH_OK;
         if (h->list_use == SphHandle::LISTS_PAIR) {
-            CUDA_TRY(h, sph::dev_alloc((void **)&ids, 4 * n));
-            st = sph::pair_public_ids(h->A, h->P, ids, h->stream);
-            T.cell_id = ids;
+            // (the packed cells are the rebuild's own: free between two)
+            T.cell_id = reinterpret_cast<uint32_t *>(h->A.cellc);
+            st = sph::pair_public_ids(h->A, h->P, T.cell_id, h->stream);
         }
         if (st == SPH_OK) st = sph::sort_from_ids(T, h->stream);
         cudaError_t e = cudaStreamSynchronize(h->stream);
         if (e == cudaSuccess && cell_id) e = cudaMemcpy(cell_id, T.cell_id, 4 * n, cudaMemcpyDeviceToHost);
-        cudaFree(ids);
         if (st != SPH_OK) return fail(h, st, "cell sort failed");
         CUDA_TRY(h, e);
     } else if (cell_id && n) {

@@ -142,3 +142,21 @@ def test_bonds_come_back_from_a_full_device():
     a, b = out
     for name in ("pairs", "delta_n", "delta_t", "omega_n", "omega_t"):
         assert getattr(a, name).any() and numpy.array_equal(getattr(a, name), getattr(b, name)), name
+
+
+def test_sort_products_of_the_list_step_from_a_full_device():
+    s = _lattice(1300000)
+    st = Stepper([s], precision="mixed")
+    st.set_variant(4)
+    st.upload()
+    st.step(2)
+    a = st.sort_products()
+    pad = _fill()
+    b = st.sort_products()
+    del pad
+    _give_back()
+    st.step(2)
+    for u, v in zip(a, b):
+        assert numpy.array_equal(u, v)
+    assert (numpy.diff(a[0][a[1]].astype(numpy.int64)) >= 0).all()
+    st.close()
