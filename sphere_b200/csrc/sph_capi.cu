@@ -2800,7 +2800,7 @@ int sph_relax(SphHandle *h, uint32_t sweeps, double alpha, double z_top, double 
         int st0 = sync_public(h);
         if (st0 != SPH_OK) return st0;
         invalidate_pair(h);   // the sweeps move the spheres in the FP64 arrays
-        h->list_use = SphHandle::LISTS_NONE;   // the sweeps' sort is the last one
+        if (sweeps) h->list_use = SphHandle::LISTS_NONE;   // the sweeps' sort is the last one
     }
     uint64_t nl = 0;
     {

@@ -193,3 +193,23 @@ def test_graphs_captured_before_the_first_upload(precision, variant):
         st.close()
     for u, v in zip(*out):
         assert numpy.array_equal(u, v)
+
+
+@pytest.mark.parametrize("sweeps", [0, 1])
+def test_sort_products_after_packing_sweeps(sweeps):
+    """Those of the last sweep, or with no sweep of the last step, as from the
+    kernel that sorts at every step."""
+    s = scenes.gravity_settling(3000, seed=3)
+    s.vel[:] = numpy.random.default_rng(0).normal(0.0, 1.0, s.vel.shape)
+    out = []
+    for variant in (1, 3):
+        st = _stepper(s, variant)
+        st.step(60)
+        if sweeps:
+            st.relax(sweeps, alpha=0.5, z_top=float(s.L[2]))
+        else:
+            st._check(st.lib.sph_relax(st.h, 0, 0.5, float(s.L[2]), None), "sph_relax")
+        out.append(st.sort_products())
+        st.close()
+    for u, v in zip(*out):
+        assert numpy.array_equal(u, v)
