@@ -1933,6 +1933,12 @@ int sph_set_contacts(SphHandle *h, const uint32_t *contacts, const double *delta
     if (!h->uploaded) return fail(h, SPH_ERR_STATE, "sph_set_contacts before sph_upload");
     cudaSetDevice(h->device);
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    {
+        // the spheres keep their state: the list step's compact one is dropped
+        // below, and the rows' image codes follow the positions
+        int st = sync_public(h);
+        if (st != SPH_OK) return st;
+    }
     const uint64_t n = h->ntot, ns = n * sph::NC;
     if (n == 0) return SPH_OK;
     std::vector<uint32_t> w(ns, sph::EMPTY);

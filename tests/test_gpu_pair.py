@@ -189,6 +189,32 @@ def test_tuner_keeps_the_list_step_where_the_split_step_is_as_fast(n):
         assert numpy.array_equal(o.x, out[0].x) and numpy.array_equal(o.force, out[0].force)
 
 
+def test_set_contacts_after_list_steps_keeps_the_spheres():
+    """The rows of an earlier state handed over right after list steps, with no
+    other call in between that reads the state: the spheres stay where the
+    steps left them."""
+    s = cases.make("periodic_xy_wall_stress")[0]
+    out = []
+    for read in (True, False):
+        st = Stepper([copy.deepcopy(s)], precision="mixed")
+        st.set_variant(PAIR)
+        st.upload()
+        st.step(5)
+        c, h, _ = st.contacts()
+        st.step(20)
+        if read:
+            st.download()
+        st.set_contacts(c, h)
+        hp = [st.download()[0]]
+        st.step(5)
+        hp.append(st.download()[0])
+        out.append(hp)
+        st.close()
+    for u, v in zip(*out):
+        for name in ("x", "vel", "angvel", "force"):
+            assert numpy.array_equal(getattr(u, name), getattr(v, name)), name
+
+
 def test_pair_ensemble_box_by_box():
     sims = scenes.shear_ensemble(nboxes=6, seed=2, device=0, counts=(300, 3000), sweeps=400)
     a = Stepper(sims, precision="fp64")
