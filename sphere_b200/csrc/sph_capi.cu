@@ -291,6 +291,9 @@ static int ensure_pair(SphHandle *h)
     }
     if (nkeys > sph::SCAN_MAX) nkeys = 0;
     uint32_t *chunk_box = nullptr, *box_chunk0 = nullptr, *words = nullptr, *key_base = nullptr;
+    std::vector<char> consts(sph::pair_consts_bytes(h->nbox));
+    char *dev_consts = nullptr;
+    const AllocMark mark = alloc_mark(h);
     int st;
     if ((st = dalloc(h, &P.xr[0], n)) || (st = dalloc(h, &P.xr[1], n)) ||
         (st = dalloc(h, &P.vw[0], 2 * n)) || (st = dalloc(h, &P.vw[1], 2 * n)) ||
@@ -309,15 +312,13 @@ static int ensure_pair(SphHandle *h)
         (st = dalloc(h, &box_chunk0, h->nbox)) || (st = dalloc(h, &key_base, h->nbox)) ||
         (st = dalloc(h, &P.box_done, h->nbox)) || (st = dalloc(h, &P.src, n)) || (st = dalloc(h, &P.dst, n)) ||
         (st = dalloc(h, &P.key_count, nkeys)) || (st = dalloc(h, &P.key_off, nkeys + 1)) ||
-        (st = dalloc(h, &P.key_scan, nkeys / 4096 + 2)))
+        (st = dalloc(h, &P.key_scan, nkeys / 4096 + 2)) || (st = dalloc(h, &dev_consts, consts.size()))) {
+        alloc_rewind(h, mark);
+        P = sph::PairArgs{};
         return st;
-    {
-        std::vector<char> host(sph::pair_consts_bytes(h->nbox));
-        char *dev = nullptr;
-        if ((st = dalloc(h, &dev, host.size()))) return st;
-        sph::pair_consts(h->dbox.data(), h->nbox, P, host.data(), dev);
-        CUDA_TRY(h, cudaMemcpy(dev, host.data(), host.size(), cudaMemcpyHostToDevice));
     }
+    sph::pair_consts(h->dbox.data(), h->nbox, P, consts.data(), dev_consts);
+    CUDA_TRY(h, cudaMemcpy(dev_consts, consts.data(), consts.size(), cudaMemcpyHostToDevice));
     P.key_base = key_base;
     CUDA_TRY(h, cudaMemset(P.box_done, 0, sizeof(uint32_t) * h->nbox));
     P.nkeys = (uint32_t)nkeys;

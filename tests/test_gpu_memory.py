@@ -160,3 +160,24 @@ def test_sort_products_of_the_list_step_from_a_full_device():
         assert numpy.array_equal(u, v)
     assert (numpy.diff(a[0][a[1]].astype(numpy.int64)) >= 0).all()
     st.close()
+
+
+def test_list_step_that_does_not_fit_gives_back_what_it_got():
+    """2.7 kB a sphere of 300,000 with room for a third of it."""
+    s = _lattice(300000)
+    st = Stepper([s], precision="mixed")
+    st.upload()
+    pad = torch.empty(((_free() - (300 << 20)) // (2 << 20)) * (2 << 20), dtype=torch.uint8,
+                      device="cuda")
+    before = _free()
+    for _ in range(3):
+        with pytest.raises(SphereError) as e:
+            st.set_variant(4)
+        assert e.value.status == NOMEM and _free() == before
+    st.step(2)
+    del pad
+    _give_back()
+    st.set_variant(4)
+    st.step(2)
+    assert st.tuning()[0] == 4
+    st.close()
