@@ -108,9 +108,6 @@ struct SphHandle {
     // compact arrays hold the current state; pair_ahead: the FP64 arrays
     // of A are behind them (brought up to date by sync_public)
     sph::PairArgs P{};
-    // free slots may hold a history (sph_set_contacts): the next flush of the
-    // list step clears all of them
-    bool free_hist = false;
     bool pair_alloc = false, pair_valid = false, pair_ahead = false;
     // which steps the neighbour lists (and the cells of the lazily sorted
     // split step) belong to: prepare_steps asks for a rebuild when that
@@ -349,8 +346,7 @@ static int ensure_pair(SphHandle *h)
 static int sync_public(SphHandle *h)
 {
     if (!h->pair_ahead) return SPH_OK;
-    int st = sph::pair_flush(h->A, h->P, h->free_hist, h->stream);
-    h->free_hist = false;
+    int st = sph::pair_flush(h->A, h->P, h->stream);
     if (st != SPH_OK) return fail(h, st, "list-step state flush failed");
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     h->pair_ahead = false;
@@ -1824,8 +1820,7 @@ int sph_snapshot(SphHandle *h)
     }
     if (h->pair_ahead) {
         // the compact state into the FP64 arrays, on the stream, before the copies
-        int st = sph::pair_flush(h->A, h->P, h->free_hist, h->stream);
-        h->free_hist = false;
+        int st = sph::pair_flush(h->A, h->P, h->stream);
         if (st != SPH_OK) return fail(h, st, "list-step state flush failed");
         h->pair_ahead = false;
     }
@@ -1970,7 +1965,6 @@ int sph_set_contacts(SphHandle *h, const uint32_t *contacts, const double *delta
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     CUDA_TRY(h, cudaMemset(h->A.vflag, 1, 1));   // k_touch's record of the rows is stale
-    h->free_hist = true;
     invalidate_pair(h);
     return SPH_OK;
 }

@@ -347,8 +347,7 @@ int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg
 size_t pair_consts_bytes(uint32_t nbox);
 void pair_consts(const DevBox *boxes, uint32_t nbox, PairArgs &P, char *host, char *dev);
 int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st);
-// (all: clear the history of every free slot)
-int pair_flush(const StepArgs &A, const PairArgs &P, bool all, cudaStream_t st);
+int pair_flush(const StepArgs &A, const PairArgs &P, cudaStream_t st);
 int pair_count_live(const StepArgs &A, const PairArgs &P, cudaStream_t st,
                     unsigned long long *d_count);
 // The cell ids of the list step's last rebuild in the original numbering.

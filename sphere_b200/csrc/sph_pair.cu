@@ -1061,10 +1061,10 @@ __global__ void k_pair_load(StepArgs A, PairArgs P)
 // The compact state -> the FP64 arrays, and the touching entries of each
 // list -> the sphere's contact row (by ascending partner, slots 0, 1, ...)
 // with their histories and image codes.  A free slot's history is zero by
-// construction (upload, ended contacts), so only the slots that the row
-// held and no longer holds are cleared (all: every free slot): 1 KB per sphere less to write (885
-// -> 436 us at 1e6 spheres).
-__global__ void k_pair_flush(StepArgs A, PairArgs P, bool all)
+// construction (upload, ended contacts, sph_set_contacts), so only the slots
+// that the row held and no longer holds are cleared: 1 KB per sphere less to
+// write (885 -> 436 us at 1e6 spheres).
+__global__ void k_pair_flush(StepArgs A, PairArgs P)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= A.ntot) return;
@@ -1118,7 +1118,7 @@ __global__ void k_pair_flush(StepArgs A, PairArgs P, bool all)
         ++s;
     }
     for (; s < NC; ++s) {
-        if (row[s] == EMPTY && !all) continue;
+        if (row[s] == EMPTY) continue;
         row[s] = EMPTY;
         hist[s] = make_double4(0.0, 0.0, 0.0, 0.0);
     }
@@ -1365,9 +1365,9 @@ int pair_load(const StepArgs &A, const PairArgs &P, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 
-int pair_flush(const StepArgs &A, const PairArgs &P, bool all, cudaStream_t st)
+int pair_flush(const StepArgs &A, const PairArgs &P, cudaStream_t st)
 {
-    if (A.ntot) k_pair_flush<<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P, all);
+    if (A.ntot) k_pair_flush<<<blocks_for(A.ntot, 128), 128, 0, st>>>(A, P);
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 

@@ -215,6 +215,28 @@ def test_set_contacts_after_list_steps_keeps_the_spheres():
             assert numpy.array_equal(getattr(u, name), getattr(v, name)), name
 
 
+def test_free_slots_hold_no_history():
+    """Histories given for free slots are not taken over; the list step's flush
+    relies on that and on ended contacts leaving zeros."""
+    s = cases.make("fast_spheres")[0]
+    n = int(s.np[0])
+    st = Stepper([copy.deepcopy(s)], precision="mixed")
+    st.set_variant(PAIR)
+    st.upload()
+    st.step(5)
+    c, h, _ = st.contacts()
+    h = numpy.asarray(h).reshape(n, 32, 4).copy()
+    free = numpy.asarray(c).reshape(n, 32) == n
+    h[free] = 1.0
+    st.set_contacts(c, h.reshape(-1, 4))
+    for k in (1, 40):
+        st.step(k)
+        c, h, _ = st.contacts()
+        free = numpy.asarray(c).reshape(n, 32) == n
+        assert (~free).any() and not numpy.asarray(h).reshape(n, 32, 4)[free].any()
+    st.close()
+
+
 def test_pair_ensemble_box_by_box():
     sims = scenes.shear_ensemble(nboxes=6, seed=2, device=0, counts=(300, 3000), sweeps=400)
     a = Stepper(sims, precision="fp64")
