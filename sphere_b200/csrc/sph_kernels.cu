@@ -958,7 +958,7 @@ int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t s
     if (A.ntot > 0) {
         const bool split = split_active(A, cfg);
         if (A.lazy_sort) {
-            launch_resort(k_resort, A.ntot, st, A, resort_sync(A));
+            launch_resort<k_resort>(A.ntot, st, A, resort_sync(A));
             mark(prof, st, "k_resort");
             nl += 1;
         } else {

@@ -1274,7 +1274,7 @@ int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg
         prof->n = 0;
         record(prof->ev[0], st);
     }
-    launch_resort(k_pair_resort, A.ntot, st, A, P, resort_sync(A));
+    launch_resort<k_pair_resort>(A.ntot, st, A, P, resort_sync(A));
     mark(prof, st, "k_pair_resort");
     launch_pair_kernel(A, P, cfg, st);
     if (pair_shape_persistent(cfg.pair_shape)) {

@@ -261,19 +261,20 @@ __device__ __forceinline__ bool sort_all(const StepArgs &A, const GridSync &G, u
 
 // Launch a RESORT_THREADS-thread cooperative kernel over n spheres with the
 // list scratch in dynamic shared memory: as many blocks as can be resident,
-// at most one per RESORT_THREADS spheres.
-template <class... Par, class... Arg>
-inline void launch_resort(void (*kern)(Par...), uint64_t n, cudaStream_t st, Arg... args)
+// at most one per RESORT_THREADS spheres.  (The kernel is a template argument,
+// so that what is asked once of the device is asked once per kernel.)
+template <auto KERN, class... Arg>
+inline void launch_resort(uint64_t n, cudaStream_t st, Arg... args)
 {
     const size_t sm = sizeof(uint32_t) * ((size_t)VL_MAX * RESORT_THREADS + 64);
-    // (per thread and kernel: the device's answers, asked for once)
+    // (per thread: the device's answers, asked for once)
     static thread_local int for_dev = -1, sms = 0, per_sm = 0;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != for_dev) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RESORT_THREADS, sm);
+        cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, RESORT_THREADS, sm);
         for_dev = dev;
     }
     const uint64_t need = (n + RESORT_THREADS - 1) / RESORT_THREADS;
@@ -288,7 +289,7 @@ inline void launch_resort(void (*kern)(Par...), uint64_t n, cudaStream_t st, Arg
     at[0].val.cooperative = 1;
     c.attrs = at;
     c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kern, args...);
+    cudaLaunchKernelEx(&c, KERN, args...);
 }
 
 inline GridSync resort_sync(const StepArgs &A)
