@@ -462,10 +462,10 @@ __device__ __forceinline__ DpCoef load_coef(const DarcyArgs &D, uint32_t c, uint
 // a / b correctly rounded for a divisor b that stays fixed (the cell
 // sizes), from rb = RN(1 / b), by Markstein's correction (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34(1), 1990): q0 = RN(a rb) lies within one
-// ulp of a / b, the remainder r = a - b q0 is exact (one FMA), and
-// RN(q0 + r rb) is the correctly rounded quotient while q0 is a normal
-// number away from the ends of the range.  A zero a gives q0 = +-0, the
+// processor", IBM J. Res. Dev. 34(1), 1990): q0 = RN(a rb), the remainder
+// r = a - b q0 (one FMA), and RN(q0 + r rb) is the correctly rounded quotient
+// (sph_divisor.cuh says why) while q0 is a normal number away from the ends of
+// the range.  A zero a gives q0 = +-0, the
 // quotient with its sign (rb has the sign of b); tiny, huge, infinite and
 // NaN q0 take the division itself.  One multiply and two FMAs instead of a
 // division sequence -- and no division at all for the zero differences of

@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sph_divisor.cuh"
 #include "sphere_b200.h"
 
 namespace sph {
@@ -114,37 +115,6 @@ __device__ __forceinline__ d3 vadds(d3 a, double b) { return mk(a.x + b, a.y + b
 __device__ __forceinline__ d3 smul(double s, d3 a) { return mk(s * a.x, s * a.y, s * a.z); }
 __device__ __forceinline__ d3 muls(d3 a, double s) { return mk(a.x * s, a.y * s, a.z * s); }
 
-// Several correctly rounded quotients by one divisor b, by Markstein's
-// correction (P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990) from
-// r = RN(1 / b): q0 = RN(a r) lies within one ulp of a / b, the remainder
-// a - b q0 is exact (one FMA), and RN(q0 + r * remainder) is the quotient,
-// while a, r and q0 lie away from the ends of the range.  A zero a with a
-// finite r gives q0 = +-0, the quotient with its sign; every other operand
-// takes the division itself.  A multiply and two FMAs for each quotient
-// after the first division, instead of a division sequence (about ten FP64
-// instructions and a branch).  The rare division is a call: inlined, it was
-// computed beside each quotient (k_finish executed 1,900 instructions a warp).
-static __device__ __noinline__ double plain_quotient(double a, double b) { return a / b; }
-
-struct Divisor {
-    double b, r;
-    bool ok;
-    __device__ __forceinline__ explicit Divisor(double b_) : Divisor(b_, 1.0 / b_) {}
-    __device__ __forceinline__ Divisor(double b_, double r_) : b(b_), r(r_)
-    {
-        ok = fabs(r) > 0x1p-1000 && fabs(r) < 0x1p+1000;
-    }
-    __device__ __forceinline__ double div(double a) const
-    {
-        const double q0 = __dmul_rn(a, r);
-        const double aq = fabs(q0);
-        if (ok && aq > 0x1p-900 && aq < 0x1p+1000 && fabs(a) > 0x1p-900)
-            return __fma_rn(__fma_rn(-q0, b, a), r, q0);
-        if (ok && a == 0.0) return q0;
-        return plain_quotient(a, b);
-    }
-};
 __device__ __forceinline__ Divisor divisor_dt(const DevBox &B) { return Divisor(B.dt); }
 __device__ __forceinline__ Divisor divisor_dt(const BoxConst &C) { return Divisor(C.dt, C.inv_dt); }
 __device__ __forceinline__ d3 divs(d3 a, double s)
