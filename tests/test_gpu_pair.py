@@ -320,3 +320,34 @@ def test_pair_shapes_give_the_same_bits(name):
             assert numpy.array_equal(getattr(a, f), getattr(b, f)), (shape, f)
         assert ba.t_current == bb.t_current
         assert list(ba.walls.nx[0]) == list(bb.walls.nx[0])
+
+
+@pytest.mark.parametrize("walls", [True, False])
+def test_pair_shapes_give_the_same_bits_in_an_ensemble(walls):
+    """Several boxes, whose constants the kernels take from tables instead of
+    their arguments: packs of different sizes and parameters, pressed by their
+    walls or without any."""
+    if walls:
+        sims = scenes.shear_ensemble(nboxes=4, seed=5, device=0, counts=(300, 1500), sweeps=300)
+    else:
+        sims = [scenes.lattice_pack(n, seed=n, periodic=1, nw=0, gamma_n=20.0 * k + 10.0)
+                for k, n in enumerate((65, 500, 1200))]
+    sims[1].mu_s[0] = 0.2
+    out = {}
+    for shape in range(_abi.PAIR_SHAPES):
+        st = Stepper(copy.deepcopy(sims), precision="mixed")
+        st.set_variant(PAIR)
+        st.set_launch_shape(shape)
+        st.upload()
+        st.step(30)
+        hp, _ = st.download()
+        out[shape] = (hp, st.boxes())
+        st.close()
+    a, ba = out[0]
+    assert a.force.any()
+    for shape, (b, bb) in out.items():
+        for f in ("x", "vel", "angvel", "force", "torque", "es", "ev", "p"):
+            assert numpy.array_equal(getattr(a, f), getattr(b, f)), (shape, f)
+        for u, v in zip(ba, bb):
+            assert u.t_current == v.t_current and list(u.walls.nx[0]) == list(v.walls.nx[0])
+            assert list(u.walls.mvfd[0]) == list(v.walls.mvfd[0])
