@@ -121,6 +121,20 @@ def interact_bytes(n, c, precision):
     return 352 * n + 52 * c
 
 
+def interact_stage(kernels):
+    """The kernels of the interact stage among the profiled ones: the fused
+    kernel, those of the split step (search and contacts in one kernel, or in
+    two where a cell is no wider than the largest diameter) or the list
+    step's kernel (same work, same algorithmic bytes)."""
+    if "k_pair_step" in kernels:
+        return ["k_pair_step"]
+    if "k_interact" in kernels:
+        return ["k_interact"]
+    if "k_touch" in kernels:
+        return ["k_touch", "k_finish"]
+    return ["k_search", "k_contacts", "k_finish"]
+
+
 def step_bytes(n, c, precision):
     """Whole-step algorithmic bytes: interact bytes + the cell sort
     (16 B x 3 radix-equivalent passes per sphere)."""
@@ -679,15 +693,7 @@ def main():
         st.profile(False)
         contacts = st.count_contacts()
         nstats = st.neighbor_stats()
-        # the interact stage: the fused kernel, the three kernels of the
-        # split step or the list step's kernel (same work, same algorithmic
-        # bytes)
-        if "k_pair_step" in kernels:
-            stage = ["k_pair_step"]
-        elif "k_interact" in kernels:
-            stage = ["k_interact"]
-        else:
-            stage = ["k_search", "k_contacts", "k_finish"]
+        stage = interact_stage(kernels)
         parts = [kernels.get(k) for k in stage]
         t_int = sum(parts) if all(isinstance(v, float) for v in parts) else None
         b_int = interact_bytes(n, contacts, precision)
