@@ -513,6 +513,11 @@ def main():
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import oracle as O
         from sphere_b200 import scenes
+        if not O.available("ref"):
+            print(json.dumps({"impl": "reference", "unavailable":
+                              "the reference's kernels are not built (oracle/_ref): no checkout "
+                              "of the reference is at hand"}))
+            return 0
         nref = min(args.ref_n, args.n)
         threads = os.cpu_count() or 1
         t0 = time.perf_counter()

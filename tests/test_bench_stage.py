@@ -1,5 +1,11 @@
 """The kernels that bench.py counts as the interact stage, as sph_profile names
-them in each kind of step."""
+them in each kind of step, and its reference arm where the reference's kernels
+are not built: a line that says so, not a measurement of something else."""
+import json
+import os
+import subprocess
+import sys
+
 import pytest
 
 import bench
@@ -30,3 +36,14 @@ def test_interact_stage_names_are_the_profiled_ones():
         kernels = st.profile_read()
         assert all(k in kernels for k in bench.interact_stage(kernels)), sorted(kernels)
         st.close()
+
+
+def test_reference_arm_without_the_reference():
+    import oracle
+    if oracle.available("ref"):
+        pytest.skip("the reference's kernels are built here")
+    out = subprocess.run([sys.executable, os.path.abspath(bench.__file__), "--impl", "reference", "--steps",
+                          "1", "--warmup", "1"], capture_output=True, text=True, timeout=300)
+    line = json.loads(out.stdout.strip().splitlines()[-1])
+    assert out.returncode == 0 and line["impl"] == "reference"
+    assert line["unavailable"] and "value" not in line
