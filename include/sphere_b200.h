@@ -340,9 +340,9 @@ int sph_set_variant(SphHandle *h, int variant);
  * 128 x 4, 11: 64 x 10 with each list entry loaded at its turn instead of
  * one entry ahead (fewer registers, more resident warps), 12: 128 x 4 with
  * four lanes per sphere, for handles whose spheres do not fill the device
- * (SPH_PAIR_SHAPES).  The results do not depend on the shape.  sph_autotune tries every shape of variant 4
- * and reports the best in ms_per_step[4]; sph_get_tuning returns the
- * variant and shape in use. */
+ * (SPH_PAIR_SHAPES).  The results do not depend on the shape.
+ * sph_autotune tries every shape of variant 4 and reports the best in
+ * ms_per_step[4]; sph_get_tuning returns the variant and shape in use. */
 #define SPH_PAIR_SHAPES 13
 int sph_set_launch_shape(SphHandle *h, int shape);
 int sph_get_tuning(const SphHandle *h, int *variant, int *shape);

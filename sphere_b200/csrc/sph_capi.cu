@@ -115,9 +115,7 @@ struct SphHandle {
     enum ListUse { LISTS_NONE, LISTS_CHAIN, LISTS_LAZY, LISTS_PAIR };
     ListUse list_use = LISTS_NONE;
     // steps launched kernel by kernel instead of as captured graphs
-    // (SPHERE_B200_EAGER=1 at sph_create): for profilers that cannot see
-    // into graphs with conditional nodes; the list step then reads its
-    // rebuild request on the host each step
+    // (SPHERE_B200_EAGER=1 at sph_create), for profilers
     bool eager = false;
     // the Darcy coupling (sph_darcy_set): its device fields and state
     // (D.st null until set), the host mirror of the device's step count
@@ -1118,12 +1116,6 @@ static int capture_step(SphHandle *h, sph::Prof *prof, cudaGraph_t *g, cudaGraph
     StepConfig cfg = step_config(h);
     cfg.phase = phase;
     const bool pair = pair_active(h);
-    if (h->darcy_on && !h->side) {
-        // the Darcy coupling captures its Jacobi loop's body on the side stream
-        CUDA_TRY(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        CUDA_TRY(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-        CUDA_TRY(h, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
-    }
     cfg.side = h->side;
     cfg.fork = h->ev_fork;
     cfg.join = h->ev_join;
@@ -2009,8 +2001,8 @@ int sph_get_sort(SphHandle *h, uint32_t *cell_id, uint32_t *perm, uint32_t *cell
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     const uint64_t n = h->ntot, nc = h->ncells;
     // the lazily sorted split step keeps each step's cell ids; the order
-    // that follows from them is made here
-    // (of the last rebuild after list steps, from that step's numbering)
+    // that follows from them is made here (after list steps: of the last
+    // rebuild, whose ids are in that step's numbering)
     if (n && (h->list_use == SphHandle::LISTS_LAZY || h->list_use == SphHandle::LISTS_PAIR)) {
         StepArgs T = h->A;
         int st = SPH_OK;

@@ -24,17 +24,17 @@
 //    step's start and the new state is written to the other half of a
 //    ping-pong pair, so no second pass is needed; the wall stage sums the
 //    wall force in fixed-order chunks (deterministic, FP64) and advances
-//    the walls and time (k_pair_chunks, k_pair_box);
+//    the walls and time (k_pair_walls; k_pair_box without walls);
 //  * storage: FP64 where the precision contract keeps FP64 (positions,
 //    velocities, the history, xyzsum, es/ev, the wall force), FP32 for the
 //    rest (angular velocity, angpos, acc, angacc, force, torque, energy
 //    rates) -- the per-sphere bytes of the mixed budget.
 //
-// The lists are rebuilt inside the step graph only when a sphere has moved
-// more than half the skin since the last build: a conditional graph node
-// whose body is the cell sort, the list build and the history carry-over
-// (launch_step_pair), set by k_pair_cond from the flag the integration
-// raises.  Every launch shape gives the same bits: the code generator may
+// The lists are rebuilt only when a sphere has moved more than half the skin
+// since the last build: a cooperative launch in every step (k_pair_resort:
+// the cell sort, the list build, the history carry-over and the threads'
+// order) that ends at once unless the integration has raised its flag.
+// Every launch shape gives the same bits: the code generator may
 // fuse a multiply and an add, or lay out an approximate division,
 // differently in one shape than in another (it decides under each shape's
 // register budget), so the file is compiled without FMA contraction, the
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(PBOX_THREADS) k_pair_box(StepArgs A, PairArgs 
 // spheres in turn (slots t = block + k * grid), then, after a grid barrier,
 // the chunks' wall-force sums, and after another the boxes (walls, time)
 // and the hand-over of the ping-pong state.  The same arithmetic and order
-// of sums as k_pair_step + k_pair_chunks + k_pair_box.
+// of sums as k_pair_step + k_pair_walls.
 template <int LM, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_pair_persist(StepArgs A, PairArgs P, GridSync G)
 {

@@ -3,8 +3,8 @@ the Darcy oracle (oracle/sphere_oracle.c, itself pinned to the reference's
 own Darcy kernels by tests/test_darcy_oracle.py), bit for bit: every fluid
 field, the pressure force on each sphere, the sphere state after the
 coupled steps and the Jacobi record of every fluid step, on the scenes of
-tests/darcy_cases.py.  The Jacobi loop runs on the device (a conditional
-node of the step graph), so splitting the steps into calls must not change
+tests/darcy_cases.py.  The Jacobi loop runs on the device (a cooperative
+launch in the step graph), so splitting the steps into calls must not change
 a bit either; run() writes the reference's conv.log and output files."""
 import copy
 import os
