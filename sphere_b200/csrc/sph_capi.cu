@@ -84,7 +84,8 @@ struct SphHandle {
     char *chunk = nullptr;
     size_t chunk_left = 0, chunk_bytes = 0;
     char *scratch = nullptr;
-    size_t scratch_bytes = 0, scratch_want = 0;
+    size_t scratch_bytes = 0;
+    size_t pair_room = 0, tile_room = 0;   // what the last overlap and tile lists took
     unsigned long long *d_count = nullptr;
     uint32_t *vlist_mem = nullptr;   // neighbour-list storage (A.vlist is null when off)
     std::vector<double> rmax_box;    // largest radius per box (at upload)
@@ -142,6 +143,8 @@ static int fail(SphHandle *h, int code, const std::string &msg)
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
         }                                                                                   \
     } while (0)
+
+constexpr size_t SCRATCH_MIN = 4u << 20, SCRATCH_SPARE = 64u << 20;
 
 static void free_scratch(SphHandle *h)
 {
@@ -220,26 +223,29 @@ static void alloc_rewind(SphHandle *h, const AllocMark &m)
     h->chunk_left = m.left;
 }
 
-// At least `bytes` of device scratch for one call (256-byte aligned), kept for
-// the next; its contents are the caller's only until the call returns.  Null
-// when the device has no room.  A call that could have used more says so in
-// scratch_want, and the next one takes that much if it is to be had.
-static char *scratch_mem(SphHandle *h, size_t bytes)
+// At least `bytes` of device scratch for one call (256-byte aligned), and
+// `wish` more where that is to be had, kept for the next; its contents are the
+// caller's only until the call returns.  Null when the device has no room.
+// Allocated with room to spare (up to 64 MB): the calls that read one output
+// (image, porosity, overlaps) need different amounts, and mapping a block and
+// unmapping the last at each of them took half of a new handle's first pass
+// (image, profile and overlaps of 7,000 spheres 2.65 ms, 1.33 with one block;
+// of 50,000 4.9 and 3.5).
+static char *scratch_mem(SphHandle *h, size_t bytes, size_t wish = 0)
 {
+    if (bytes + wish <= h->scratch_bytes) return h->scratch;
+    if (bytes > h->scratch_bytes) free_scratch(h);
+    const size_t ample = std::max(bytes + std::max(std::min(bytes, SCRATCH_SPARE), wish), SCRATCH_MIN);
     void *q = nullptr;
-    if (h->scratch_want > h->scratch_bytes && h->scratch_want >= bytes &&
-        sph::dev_alloc(&q, h->scratch_want) == cudaSuccess) {
-        free_scratch(h);
-        h->scratch = static_cast<char *>(q);
-        h->scratch_bytes = h->scratch_want;
-    }
-    h->scratch_want = 0;
-    if (bytes > h->scratch_bytes) {
-        free_scratch(h);
+    size_t got = ample;
+    if (sph::dev_alloc(&q, ample) != cudaSuccess) {
+        if (h->scratch) return h->scratch;
+        got = bytes;
         if (sph::dev_alloc(&q, bytes) != cudaSuccess) return nullptr;
-        h->scratch = static_cast<char *>(q);
-        h->scratch_bytes = bytes;
     }
+    free_scratch(h);
+    h->scratch = static_cast<char *>(q);
+    h->scratch_bytes = got;
     return h->scratch;
 }
 
@@ -2677,7 +2683,7 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
                  o_coff = place(4 * (ncells + 1)), o_items = place(4 * n), o_xs = place(sizeof(double4) * n),
                  o_npair = place(4 * (n + 1)), o_poff = place(4 * (n + 1)),
                  o_scan = place(4 * (ncells / 4096 + n / 4096 + 2));
-    char *mem = scratch_mem(h, used);
+    char *mem = scratch_mem(h, used, max_pairs > 0 && (pairs || delta_n) ? h->pair_room : 0);
     if (!mem) return fail(h, SPH_ERR_NOMEM, "overlap-search buffers");
     O.cell_of = (uint32_t *)(mem + o_cell);
     O.slot = (uint32_t *)(mem + o_slot);
@@ -2715,11 +2721,8 @@ int sph_overlaps(SphHandle *h, uint32_t box, uint64_t max_pairs, uint32_t *pairs
             e = cudaMemcpyAsync(delta_n, O.delta, 8 * m, cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
-    if (list) {
-        // room for as many pairs in the next call
-        h->scratch_want = used + 2 * ((8 * (size_t)total + 255) & ~(size_t)255);
-        cudaFree(list);
-    }
+    h->pair_room = 2 * ((8 * (size_t)total + 255) & ~(size_t)255);   // for the next call
+    cudaFree(list);
     if (st != SPH_OK) return fail(h, st, "overlap-search launch failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     *npairs = total;
@@ -2750,7 +2753,7 @@ int sph_render(SphHandle *h, uint32_t box, int method, float maxval, float lower
     const size_t bytes = (size_t)width * height * 3;
     const size_t img_bytes = (bytes + 255) & ~(size_t)255;
     const size_t rt_bytes = sph::render_scratch(d.np, width, height);
-    uint8_t *img = (uint8_t *)scratch_mem(h, img_bytes + rt_bytes);
+    uint8_t *img = (uint8_t *)scratch_mem(h, img_bytes + rt_bytes, h->tile_room);
     if (!img) return fail(h, SPH_ERR_NOMEM, "image buffer");
     sph::RenderStats rs;
     int st = sph::render_image(h->A, d.p_base, d.np, d_L, method, maxval, lower_cutoff, width,
@@ -2759,9 +2762,7 @@ int sph_render(SphHandle *h, uint32_t box, int method, float maxval, float lower
     h->launches += (uint64_t)rs.launches;
     cudaError_t e = cudaSuccess;
     if (st == SPH_OK) e = cudaMemcpy(rgb, img, bytes, cudaMemcpyDeviceToHost);
-    // room for as many tile-list entries in the next call
-    const size_t want = img_bytes + rt_bytes + 256 + sizeof(uint32_t) * (size_t)rs.entries;
-    if (st == SPH_OK && e == cudaSuccess && want > h->scratch_bytes) h->scratch_want = want;
+    h->tile_room = 256 + sizeof(uint32_t) * (size_t)rs.entries;   // for the next call
     if (st != SPH_OK) return fail(h, st, "ray-tracing kernels failed");
     if (e != cudaSuccess) return fail(h, SPH_ERR_CUDA, cudaGetErrorString(e));
     return SPH_OK;
