@@ -705,7 +705,6 @@ int sph_create(const SphBox *boxes, uint32_t nboxes, int precision, int length_m
         return bail(st);
     }
     A.vcap = sph::VL_MAX;
-    A.sort_limit_ns = sph::BARRIER_LIMIT_NS;
     h->vlist_mem = A.vlist;
     A.box_of = box_of;
     A.part_owner = part_owner;
@@ -1993,7 +1992,7 @@ int sph_set_rebuild_limit(SphHandle *h, double seconds)
     if (!(seconds >= 0.0) || seconds > 10.0) return fail(h, SPH_ERR_INPUT, "limit outside 0 .. 10 s");
     cudaSetDevice(h->device);
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    h->A.sort_limit_ns = (unsigned long long)(seconds * 1e9);
+    h->cfg.rebuild_limit_ns = (unsigned long long)(seconds * 1e9);
     return drop_graphs(h);
 }
 

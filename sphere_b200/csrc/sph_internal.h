@@ -60,7 +60,6 @@ struct StepArgs {
     // that of the step before may run beside the rebuild
     uint32_t *vlist, *vcount, *vflag;
     uint32_t *sort_bar;        // grid-barrier words of the one-launch rebuilds
-    unsigned long long sort_limit_ns;   // ... and how long their blocks wait
     float4 *xref;
     uint64_t *cellc;
     uint32_t vcap;             // list capacity in use (<= VL_MAX)
@@ -252,6 +251,7 @@ struct StepConfig {
     // than the largest diameter
     bool touch = false;
     int phase = STEP_WHOLE;
+    unsigned long long rebuild_limit_ns = BARRIER_LIMIT_NS;   // how long a rebuild's blocks wait
     cudaStream_t side = nullptr;                       // STEP_OVERLAP only
     cudaEvent_t fork = nullptr, join = nullptr;        // STEP_OVERLAP only
     const DarcyArgs *darcy = nullptr;                  // the Darcy coupling, null: off

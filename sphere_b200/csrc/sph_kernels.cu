@@ -205,7 +205,7 @@ __global__ void k_bonds(StepArgs A)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= A.nbonds) return;
-    if (A.lazy_sort && A.vflag[3] != 0u) return;
+    const uint32_t stop = A.lazy_sort ? A.vflag[3] : 0u;   // a rebuild gave up
     const DevBox &B = A.boxes[A.bond_box[k]];
     const SphParams &P = B.P;
     const double dt = B.dt;
@@ -253,6 +253,7 @@ __global__ void k_bonds(StepArgs A)
     const d3 t_j = vadd(t_n, t_t);
     const double sigma_max = vlen<LM>(f_n) / Ar + vlen<LM>(t_t) * R_bar / I;
     const double tau_max = vlen<LM>(f_t) / Ar + vlen<LM>(t_n) * R_bar / J;
+    if (stop) return;   // the bond keeps its state
     if (sigma_max >= P.sigma_b || tau_max >= P.tau_b) {
         A.bonds[k].x = B.nb0;
         A.bbroken[k] = 1;
@@ -958,7 +959,7 @@ int launch_step_with(const StepArgs &args, const StepConfig &cfg, cudaStream_t s
     if (A.ntot > 0) {
         const bool split = split_active(A, cfg);
         if (A.lazy_sort) {
-            launch_resort<k_resort>(A.ntot, st, A, resort_sync(A));
+            launch_resort<k_resort>(A.ntot, st, A, resort_sync(A, cfg));
             mark(prof, st, "k_resort");
             nl += 1;
         } else {

@@ -802,13 +802,13 @@ __global__ void __launch_bounds__(PBOX_THREADS) k_pair_walls(StepArgs A, PairArg
     stage_box(B, A.boxes[bx]);
     grid_dependency_wait();
     const uint32_t stop = A.vflag[3];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !stop) *P.pp ^= 1u;
+    if (chunk) chunk_sum(A, P, blockIdx.x, s_w);
+    if (stop) return;   // (not ahead of the sums, which would wait for the word)
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicXor(P.pp, 1u);
     if (!chunk) {
-        if (B.np == 0 && !stop) box_sum_advance(A, P, bx, B, s_w);
+        if (B.np == 0) box_sum_advance(A, P, bx, B, s_w);
         return;
     }
-    chunk_sum(A, P, blockIdx.x, s_w);
-    if (stop) return;
     if (threadIdx.x == 0) {
         const uint32_t nch = (B.np + (1u << P.chunk_log2) - 1) >> P.chunk_log2;
         __threadfence();
@@ -1274,7 +1274,7 @@ int launch_step_pair(const StepArgs &A, const PairArgs &P, const StepConfig &cfg
         prof->n = 0;
         record(prof->ev[0], st);
     }
-    launch_resort<k_pair_resort>(A.ntot, st, A, P, resort_sync(A));
+    launch_resort<k_pair_resort>(A.ntot, st, A, P, resort_sync(A, cfg));
     mark(prof, st, "k_pair_resort");
     launch_pair_kernel(A, P, cfg, st);
     if (pair_shape_persistent(cfg.pair_shape)) {

@@ -292,12 +292,12 @@ inline void launch_resort(uint64_t n, cudaStream_t st, Arg... args)
     cudaLaunchKernelEx(&c, KERN, args...);
 }
 
-inline GridSync resort_sync(const StepArgs &A)
+inline GridSync resort_sync(const StepArgs &A, const StepConfig &cfg)
 {
     GridSync G;
     G.count = A.sort_bar;
     G.gen = A.sort_bar + 1;
-    G.limit_ns = A.sort_limit_ns;
+    G.limit_ns = cfg.rebuild_limit_ns;
     return G;
 }
 

@@ -1273,21 +1273,19 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
     const unsigned long long m = A.lmask[i];
     const uint32_t vc = A.vcount[i];
     uint32_t occ = A.occ[i];
+    const uint32_t stop = A.vflag[3];   // a rebuild gave up
     const uint32_t *lst = A.vlist + (size_t)i * VL_MAX;
     const double4 xa = A.x[i];
-    // after a rebuild that gave up: no contacts and no row is written (as a
-    // value in what follows, not as a branch ahead of the loads)
-    const bool go = A.vflag[3] == 0u;
     position_check(A, B, i, xa);
     if (A.tape_state) {
         A.tape_state[i] = xa;
         A.tape_state[A.ntot + i] = A.vel[i];
         A.tape_state[2 * (size_t)A.ntot + i] = A.angvel[i];
     }
-    if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return go ? touch_row<LM>(A, i) : 0u;
+    if (vc > (uint32_t)VL_MAX || !(m & LMASK_VALID)) return stop ? 0u : touch_row<LM>(A, i);
     // the first entry that is not in the row and touches, and its slot word
     uint32_t found = 0, kf = 0, wf = 0;
-    for (unsigned long long todo = go ? ((1ull << vc) - 1ull) & ~m : 0ull; todo;) {
+    for (unsigned long long todo = ((1ull << vc) - 1ull) & ~m; todo;) {
         // the next KB entries' gathers in flight together
         uint32_t bo[KB], ke[KB];
         double4 xb[KB];
@@ -1320,6 +1318,10 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
             }
         }
     }
+    // Stopped: no contacts, and no row is written.  (Here and not ahead of the
+    // loads, where every thread waited for the word first, 1 to 5 % of the
+    // kernel; what the search read is there, each list with its own length.)
+    if (stop) return 0u;
     // several new contacts take their slots in the cells' visit order
     if (found > 1u || (found == 1u && occ == 0xffffffffu)) return touch_row<LM>(A, i);
     uint32_t *row = A.slots + (size_t)i * NC;
@@ -1346,7 +1348,7 @@ __device__ __forceinline__ uint32_t touch_search(const StepArgs &A, const BX &B,
             A.tape_hist[q] = A.hist[q];
         }
     }
-    return go ? occ : 0u;
+    return occ;
 }
 
 // SPW: spheres of a warp (see launch_contacts_lm).

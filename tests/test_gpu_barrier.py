@@ -113,3 +113,24 @@ def test_a_rebuild_that_gives_up_leaves_the_state(precision, variant, shape, rad
         assert numpy.array_equal(u, v)
     st.close()
     ref.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_rebuild_that_gives_up_leaves_the_bonds(precision):
+    s = scenes.bonded_pack(3000, nbonds=4500, seed=1, device=0)
+    st = Stepper([s], precision=precision)
+    st.set_variant(3)
+    st.upload()
+    st.step(7)
+    before = st.download()
+    st.set_rebuild_limit(0.0)
+    st.set_neighbor_lists(48)
+    with pytest.raises(SphereError) as e:
+        st.step(4)
+    assert e.value.status == TIMEOUT
+    after = st.download()
+    for name in ("pairs", "delta_n", "delta_t", "omega_n", "omega_t"):
+        assert getattr(before[1], name).any()
+        assert numpy.array_equal(getattr(before[1], name), getattr(after[1], name)), name
+    assert numpy.array_equal(before[0].x, after[0].x) and numpy.array_equal(before[0].force, after[0].force)
+    st.close()
