@@ -2595,7 +2595,11 @@ int sph_autotune(SphHandle *h, uint32_t steps, double *ms_per_step, int *chosen)
     cudaFree(snap);
     h->t_host = t_saved;
     h->launches = launches_saved;
+    // what the timed steps raised is theirs, except that they did not run
+    uint32_t bits = 0;
+    cudaMemcpy(&bits, h->A.err, sizeof bits, cudaMemcpyDeviceToHost);
     cudaMemset(h->A.err, 0, sizeof(uint32_t));
+    if (st == SPH_OK && (bits & (1u << SPH_ERR_TIMEOUT))) st = SPH_ERR_TIMEOUT;
     h->cfg.variant = best;
     h->variant_set = true;
     h->cfg.pair_shape = best_shape;

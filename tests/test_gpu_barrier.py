@@ -134,3 +134,24 @@ def test_a_rebuild_that_gives_up_leaves_the_bonds(precision):
         assert numpy.array_equal(getattr(before[1], name), getattr(after[1], name)), name
     assert numpy.array_equal(before[0].x, after[0].x) and numpy.array_equal(before[0].force, after[0].force)
     st.close()
+
+
+def test_tuning_reports_a_rebuild_that_gave_up():
+    """Steps that return at once are the fastest of all: the tuner does not take
+    their times for a choice."""
+    s = scenes.lattice_pack(3000, seed=2, periodic=1, nw=1, wmode=1)
+    st = Stepper([s], precision="fp64")
+    st.upload()
+    st.step(3)
+    x = st.download()[0].x
+    st.set_rebuild_limit(0.0)
+    with pytest.raises(SphereError) as e:
+        st.autotune(steps=3)
+    assert e.value.status == TIMEOUT
+    assert numpy.array_equal(st.download()[0].x, x)
+    st.set_rebuild_limit(1.0)
+    st.upload()
+    st.autotune(steps=3)
+    st.step(3)
+    assert numpy.array_equal(st.download()[0].x, x)
+    st.close()
