@@ -1090,9 +1090,9 @@ int sph_upload(SphHandle *h, const SphParticles *p, const SphBonds *b)
     // Unless a variant was chosen: in the FP64 form the split step wherever it
     // can run.  It gives the fused kernel's bits at every size and is faster at
     // every size measured, since no thread walks a sphere's contacts one after
-    // the other (us a step, fused / split, shear pack, FP64: 500 spheres 66 /
-    // 45, 10,000 125 / 56, 60,000 181 / 80, 200,000 361 / 167; without
-    // contacts, 10,000 settling: 33 / 22).  The mixed form stays with the fused
+    // the other (us a step, fused / split, shear pack, FP64: 500 spheres 77 /
+    // 20, 10,000 122 / 26, 60,000 177 / 46, 200,000 369 / 118; without
+    // contacts, 10,000 settling: 29 / 17).  The mixed form stays with the fused
     // kernel: its file is compiled with FMA contraction, which the two kernels
     // need not fuse alike, and with lengths rounded to 32 bits a last bit moves
     // a force by a tenth (100 steps: forces differ by 2e-4 at 5,000 spheres, by
